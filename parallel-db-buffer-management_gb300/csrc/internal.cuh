@@ -23,11 +23,22 @@ bool device_writable(const void* p);
 
 constexpr uint32_t kDefaultMaxSteps = 4096;
 
+// Sum of v over the warp (every lane calls converged; every lane gets it).  Sums
+// that fit take one 32-bit reduction; a shuffle tree of 64-bit values is ten
+// shuffles and ten adds.
+__device__ __forceinline__ unsigned long long warp_total(unsigned long long v) {
+    if (!__any_sync(0xffffffffu, (v >> 27) != 0ull)) return __reduce_add_sync(0xffffffffu, (unsigned int)v);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    return v;
+}
+
 // Adds every thread's N counters to dst[0..N) with one global atomic per
-// counter per block: warp shuffles, then one shared atomic per warp.  Every
-// thread of the block calls it (after its loop, converged); blocks whose size
-// is not a multiple of 32 (one-thread replays) add directly.  Per-thread
-// atomics on a shared counter would serialise on one L2 address (~1.5 G/s).
+// counter per block: each warp leaves its sums in shared memory and, after the
+// block's one barrier, thread k adds up counter k.  Every thread of the block
+// calls it once (after its loop, converged); blocks whose size is not a
+// multiple of 32 (one-thread replays) add directly.  Per-thread atomics on a
+// shared counter would serialise on one L2 address (~1.5 G/s).
 template <int N>
 __device__ __forceinline__ void block_add_counters(const unsigned long long (&v)[N],
                                                    unsigned long long* const (&dst)[N]) {
@@ -36,19 +47,18 @@ __device__ __forceinline__ void block_add_counters(const unsigned long long (&v)
             if (v[k]) atomicAdd(dst[k], v[k]);
         return;
     }
-    __shared__ unsigned long long sh[N];
-    __syncthreads();   // an earlier call in the same kernel may still read sh
-    if (threadIdx.x < (unsigned)N) sh[threadIdx.x] = 0ull;
-    __syncthreads();
+    __shared__ unsigned long long sh[32][N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        unsigned long long x = v[k];
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(0xffffffffu, x, d);
-        if ((threadIdx.x & 31u) == 0u && x) atomicAdd(&sh[k], x);
+        const unsigned long long x = warp_total(v[k]);
+        if ((threadIdx.x & 31u) == 0u) sh[threadIdx.x >> 5][k] = x;
     }
     __syncthreads();
-    if (threadIdx.x < (unsigned)N && sh[threadIdx.x]) atomicAdd(dst[threadIdx.x], sh[threadIdx.x]);
+    if (threadIdx.x < (unsigned)N) {
+        unsigned long long x = 0ull;
+        for (uint32_t w = 0; w < blockDim.x >> 5; ++w) x += sh[w][threadIdx.x];
+        if (x) atomicAdd(dst[threadIdx.x], x);
+    }
 }
 // Makes a device current for the rest of the calling scope and restores the
 // caller's device when the scope ends.  Every entry point that takes a pool
