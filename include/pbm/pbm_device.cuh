@@ -203,6 +203,126 @@ __device__ __forceinline__ int32_t walk_page(const PoolView& v, int32_t seed0,
     return -1;
 }
 
+// Affine jump-ahead of the LCG by n steps: lcg31 applied n times to x is
+// (an * x + cn) mod 2^31.  The maps of 1, 2, 4, ... steps, each the square of the
+// one before, are composed by the bits of n (n < 2^BITS).
+template <int BITS>
+__device__ __forceinline__ void lcg_jump(uint32_t n, uint32_t& an, uint32_t& cn) {
+    uint32_t a = 1103515245u, c = 12345u;
+    an = 1u;
+    cn = 0u;
+#pragma unroll
+    for (int k = 0; k < BITS; ++k) {
+        if ((n >> k) & 1u) {
+            cn = a * cn + c;
+            an *= a;
+        }
+        c = a * c + c;
+        a *= a;
+    }
+}
+
+// The page-probe walks of a whole warp (lanes with `need`, each on its own LCG
+// sequence from its seed0); the warp calls converged.  A lane's walk alone is a
+// chain of dependent round trips, and the warp, and with it the launch, lasts as
+// long as its longest chain while the served lanes idle (250,007 requests on 5 M
+// pages at 90%: 8 of 32 lanes worked on average, the longest walk was some 240
+// probes).  Here each lane makes its first kOwnProbes probes itself, and then the
+// served lanes look ahead for the others: with m lanes unserved, each walk gets
+// 2^floor(log2(32 / m)) lanes, and each of these reads the pages of
+// kPageAhead consecutive probes (the LCG's state advanced to the first of them at
+// once) with all its loads in flight; the first page of a walk that reads as free
+// is claimed with the atomicOr.  Every walk tries the same pages in the
+// same order and counts the same probes as walk_page; a page read as free but
+// lost to another claim counts as held, and the walk goes on just past it.  The
+// lanes per walk double from one round to the next at most: reading far ahead
+// after a few misses would read pages that a walk in a half-empty pool rarely
+// needs.  Measured on GB300 (alloc + free of that launch, us): 114 -> 45; 16,384
+// requests at 95%: 88 -> 24; at 2% nothing is left after the own probes (10.4
+// both).  Two probes read ahead per lane: 52 and 39; eight: 50 and 21, but 20%
+// slower for a million requests at 50%, where the extra loads cost more.
+constexpr uint32_t kOwnProbes = 3;
+constexpr uint32_t kPageAhead = 4;
+
+__device__ __forceinline__ int32_t walk_page_warp(const PoolView& v, bool need, int32_t seed0,
+                                                  uint32_t max_steps, int32_t* steps_out) {
+    int32_t x = seed0 & 0x7fffffff;   // walks run on 31-bit states
+    uint32_t s = 0;
+    int32_t id = -1;
+#pragma unroll 1
+    for (uint32_t k = 0; k < kOwnProbes; ++k) {
+        if (!(need && id < 0 && s < max_steps)) break;
+        ++s;
+        x = lcg31(x);
+        const uint32_t p = idx_hi(x, v.n_pages);
+        const uint32_t bit = 1u << (p & 31u);
+        if (!(atomicOr(v.words + (p >> 5), bit) & bit)) id = (int32_t)p;
+    }
+    uint32_t pend = __ballot_sync(kFull32, need && id < 0 && s < max_steps);
+    if (pend) {
+        const uint32_t lane = threadIdx.x & 31u;
+        const uint32_t lt = (1u << lane) - 1u;
+        uint32_t aj, cj;                  // jump of lane * kPageAhead steps
+        lcg_jump<7>(lane * kPageAhead, aj, cj);
+        uint32_t max_sh = 0u;             // log2 of the most lanes one walk may get
+        do {
+            const uint32_t m = (uint32_t)__popc(pend);
+            uint32_t sh = (uint32_t)__clz((int)(m - 1u)) - 27u;   // floor(log2(32 / m)): clz(0) is 32
+            if (sh > max_sh) sh = max_sh;
+            if (max_sh < 5u) ++max_sh;
+            // this lane's place: lane j of the walk of the pending lane of that rank
+            const uint32_t j = lane & ((1u << sh) - 1u);
+            const uint32_t rank = lane >> sh;
+            const uint32_t owner = rank < m ? nth_set_bit(pend, (int)rank) : 0u;
+            const uint32_t x0 = (uint32_t)__shfl_sync(kFull32, x, (int)owner);
+            const uint32_t s0 = __shfl_sync(kFull32, s, (int)owner) + j * kPageAhead;
+            const uint32_t a = __shfl_sync(kFull32, aj, (int)j), c = __shfl_sync(kFull32, cj, (int)j);
+            int32_t xj = (int32_t)((a * x0 + c) & 0x7fffffffu);
+            uint32_t p[kPageAhead], val[kPageAhead];
+#pragma unroll
+            for (uint32_t u = 0; u < kPageAhead; ++u) {
+                xj = lcg31(xj);
+                p[u] = idx_hi(xj, v.n_pages);
+                val[u] = (rank < m && s0 < max_steps && u < max_steps - s0) ? load_word(v.words + (p[u] >> 5)) : kFull32;
+            }
+            uint32_t pc = 0u, k = kPageAhead;   // the first page read as free, the probes up to it
+            bool fre = false;
+#pragma unroll
+            for (int u = (int)kPageAhead - 1; u >= 0; --u) {
+                if (!((val[u] >> (p[u] & 31u)) & 1u)) {
+                    pc = p[u];
+                    k = (uint32_t)u + 1u;
+                    fre = true;
+                }
+            }
+            const uint32_t fm = __ballot_sync(kFull32, fre);
+            const bool first = fre && !(fm & lt & ~((1u << (lane - j)) - 1u));   // of its walk's lanes
+            const uint32_t bit = 1u << (pc & 31u);
+            const bool won = first && !(atomicOr(v.words + (pc >> 5), bit) & bit);
+            const uint32_t wm = __ballot_sync(kFull32, won);
+            // the walk's own lane takes up the result: the first page read as free, else the last one read
+            const uint32_t base = ((uint32_t)__popc(pend & lt) << sh) & 31u;   // its walk's first lane
+            const uint32_t last = base + (1u << sh) - 1u;
+            const uint32_t seen = (fm >> base) << base;
+            const uint32_t low = seen ? (uint32_t)__ffs((int)seen) - 1u : 32u;
+            const uint32_t src = low <= last ? low : last;
+            const uint32_t past = (src - base) * kPageAhead + __shfl_sync(kFull32, k, (int)src);
+            const uint32_t ps = __shfl_sync(kFull32, pc, (int)src);
+            if ((pend >> lane) & 1u) {
+                const uint32_t d = min(past, max_steps - s);   // probes made: 1 .. 32 * kPageAhead
+                if ((wm >> src) & 1u) id = (int32_t)ps;
+                uint32_t an, cn;
+                lcg_jump<8>(d, an, cn);
+                x = (int32_t)((an * (uint32_t)x + cn) & 0x7fffffffu);
+                s += d;
+            }
+            pend = __ballot_sync(kFull32, need && id < 0 && s < max_steps);
+        } while (pend);
+    }
+    if (steps_out) *steps_out = (int32_t)s;
+    return id;
+}
+
 // ---------------------------------------------------------------------------
 // Per-thread word-probe walk (RandomWalkBasic_BM semantics): jump to a random
 // word, claim its lowest clear bit; on a lost race retry in the same word;
@@ -787,18 +907,6 @@ __device__ __forceinline__ int32_t walk_span(const PoolView& v, uint32_t n, int3
     return -1;
 }
 
-// Affine jump-ahead of the LCG by lane + 1 steps: lcg31 applied lane + 1
-// times to x is (aj * x + cj) mod 2^31.  The same table serves every walk of
-// the warp, so it is computed once per call.
-__device__ __forceinline__ void lcg_jump_for_lane(uint32_t lane, uint32_t& aj, uint32_t& cj) {
-    aj = 1103515245u;
-    cj = 12345u;
-    for (uint32_t k = 0; k < lane; ++k) {
-        cj = 1103515245u * cj + 12345u;
-        aj *= 1103515245u;
-    }
-}
-
 // Runs of need_n <= 32 pages (0 = none) for the lanes of a whole warp, each
 // lane on its own LCG sequence from seed0; steps = jumps.  Every needing
 // lane first takes one jump of its own (all in parallel).  Each lane still
@@ -826,7 +934,7 @@ __device__ __forceinline__ int32_t walk_span_warp(const PoolView& v, uint32_t ne
     }
     uint32_t pend = __ballot_sync(kFull32, need_n > 0u && id < 0 && s < max_steps);
     uint32_t aj = 0u, cj = 0u;                             // jump ahead by lane + 1 steps
-    if (pend) lcg_jump_for_lane(lane, aj, cj);
+    if (pend) lcg_jump<6>(lane + 1u, aj, cj);
     while (pend) {
         const int l0 = __ffs((int)pend) - 1;
         const uint32_t x0 = (uint32_t)__shfl_sync(kFull32, x, l0);

@@ -59,7 +59,14 @@ __global__ void __launch_bounds__(256, 8) k_alloc_thread(AllocArgs a) {
             id = take_listed(a.v, a.free_list, (long long)r);   // request r takes the r-th free page
             s = 1;
         }
-        if (r >= a.n || id >= 0) {
+        if (K == Walk::Page && blockDim.x >= 32u) {
+            int32_t ws = 0;
+            const int32_t wid = walk_page_warp(a.v, go && id < 0, request_seed(a.seed, (uint32_t)r), a.max_steps, &ws);
+            if (go && id < 0) {
+                id = wid;
+                s = ws;
+            }
+        } else if (r >= a.n || id >= 0) {
             // past the last request, or served from the list
         } else if (!go) {
             // past the launch budget: no free page is left for this request
@@ -266,9 +273,12 @@ __global__ void __launch_bounds__(256) k_free_runs(PoolView v, uint32_t n, const
 __global__ void __launch_bounds__(256) k_claim_write_free(AllocArgs a, uint32_t payload_words, int hold) {
     Acc acc;
     unsigned long long frees = 0;
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < a.n; r += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t n_round = ((uint64_t)a.n + 31u) & ~31ull;   // whole warps walk together
+    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_round;
+         r += (uint64_t)gridDim.x * blockDim.x) {
         int32_t s = 0;
-        int32_t id = walk_page(a.v, request_seed(a.seed, r), a.max_steps, &s);
+        const int32_t id = walk_page_warp(a.v, r < a.n, request_seed(a.seed, (uint32_t)r), a.max_steps, &s);
+        if (r >= a.n) continue;
         a.ids[r] = id;
         if (a.steps) a.steps[r] = s;
         if (id >= 0) {

@@ -165,10 +165,11 @@ __device__ __forceinline__ void batch_round(const BatchArgs& a, uint32_t seed, b
         const uint32_t gl = threadIdx.x & (uint32_t)(W - 1);
         id = walk_collab<W, Word>(a.v, need, request_seed(seed, (uint32_t)(q - gl)), lane_off,
                                   a.dedupe != 0, a.max_steps, gslots, &s);
+    } else if constexpr (K == BWalk::Page) {
+        id = walk_page_warp(a.v, need, request_seed(seed, (uint32_t)q), a.max_steps, &s);
     } else if (need) {
         const int32_t seed0 = request_seed(seed, (uint32_t)q);
-        if constexpr (K == BWalk::Page) id = walk_page(a.v, seed0, a.max_steps, &s);
-        else if constexpr (K == BWalk::Word32) id = walk_word<uint32_t>(a.v, seed0, a.max_steps, &s);
+        if constexpr (K == BWalk::Word32) id = walk_word<uint32_t>(a.v, seed0, a.max_steps, &s);
         else id = walk_word<uint64_t>(a.v, seed0, a.max_steps, &s);
     }
     batch_finish(a, active, op, q, slot, held, need, id, s, acc);

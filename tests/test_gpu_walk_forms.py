@@ -6,6 +6,70 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+A, C, M31 = 1103515245, 12345, 0x7FFFFFFF
+
+
+def _probe_pages(orc, S, reqs, steps, n_pages):
+    """The page of probe `steps[i]` of request reqs[i]'s walk."""
+    x = np.array([orc.seed(S, int(r)) for r in reqs], dtype=np.int64)
+    out = np.zeros(len(reqs), dtype=np.int64)
+    for k in range(1, int(steps.max()) + 1):
+        x = (A * x + C) & M31
+        out = np.where(steps == k, (x * n_pages) >> 31, out)
+    return out
+
+
+@pytest.mark.parametrize("max_steps", [1, 3, 4, 7, 8, 35, 36, 131, 132, 133, 4096])
+@pytest.mark.parametrize("T,occ", [(8192, 0.5), (65536 + 17, 0.97), (1 << 20, 0.999)])
+def test_page_walk_of_one_request_is_the_sequential_walk(cuda, pbm_mod, orc, T, occ, max_steps):
+    """Alone in its launch a walk meets no race: id, steps and bitmap equal the replay's,
+    also where the bound cuts the look-ahead short."""
+    torch, pbm = cuda, pbm_mod
+    pool = pbm.Pool(T, 64)
+    cfg = pbm.walk_config(pbm.RANDOM_WALK, max_steps=max_steps)
+    ids = torch.empty(1, dtype=torch.int32, device="cuda")
+    steps = torch.empty(1, dtype=torch.int32, device="cuda")
+    for S in range(8):
+        pool.prefill(occ, 5)
+        words = orc.bernoulli_bitmap(T, occ, 5)
+        pool.alloc(cfg, 1, S, ids, steps)
+        e_ids, e_steps = orc.replay_alloc(words, T, pbm.RANDOM_WALK, 1, S, max_steps=max_steps)
+        assert (ids.item(), steps.item()) == (int(e_ids[0]), int(e_steps[0]))
+        assert np.array_equal(pool.read_bitmap(), words)
+    pool.close()
+
+
+@pytest.mark.parametrize("form", ["alloc", "claim", "batch"])
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 257, 3001])
+@pytest.mark.parametrize("occ", [0.05, 0.9, 0.985])
+def test_page_walks_end_at_their_own_probe(cuda, pbm_mod, orc, form, n, occ):
+    """Whole warps walking together: every request holds a page of its own, taken at the
+    probe of its own sequence that its step count names."""
+    torch, pbm = cuda, pbm_mod
+    T, S = 400000 + 7, 77
+    pool = pbm.Pool(T, 64, materialize=form == "claim")
+    pool.prefill(occ, 9)
+    before = pool.read_bitmap()
+    ids = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    steps = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+    cfg = pbm.walk_config(pbm.RANDOM_WALK)
+    if form == "alloc":
+        pool.alloc(cfg, n, S, ids, steps)
+    elif form == "claim":
+        pool.claim_write_free(n, S, ids, steps, hold=True)
+    else:
+        pool.batch(cfg, None, pbm.groups_array([(pbm.OP_ALLOC, n, 0)]), 1, ids, n, S, pbm.LAUNCH_PERSISTENT,
+                   steps=steps)
+    got, st = ids.cpu().numpy(), steps.cpu().numpy()
+    chk = pool.check(ids, n)
+    assert (chk.n_ok, chk.n_failed, chk.n_duplicates, chk.n_not_marked, chk.n_out_of_range) == (n, 0, 0, 0, 0)
+    assert chk.used_pages == orc.used_pages(before, T) + n
+    assert np.array_equal(got, _probe_pages(orc, S, range(n), st, T))
+    stats = pool.stats()
+    assert (stats.successes, stats.failures, stats.steps) == (n, 0, int(st.sum()))
+    pool.close()
+
+
 @pytest.mark.parametrize("n", [0, 1, 3, 4, 5, 1023, 1024, 4099, 700001])
 @pytest.mark.parametrize("shift,merge", [(0, 0), (1, 0), (0, 1)])
 def test_free_clears_exactly_the_listed_pages(cuda, pbm_mod, n, shift, merge):
