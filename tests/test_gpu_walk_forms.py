@@ -93,3 +93,44 @@ def test_free_clears_exactly_the_listed_pages(cuda, pbm_mod, n, shift, merge):
     assert np.array_equal(pool.read_bitmap(), np.packbits(bits, bitorder="little").view(np.uint32))
     assert pool.stats().frees == len(valid)
     pool.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 256, 257, 5000, 160000])
+@pytest.mark.parametrize("block_size", [64, 256])
+def test_free_list_serves_blocks_in_release_order(cuda, pbm_mod, n, block_size):
+    """Gets come out in list order, call by call, across the ring's wrap; a call that asks for more
+    than the list holds gets exactly the rest; ids that name no page are skipped by a put."""
+    torch, pbm = cuda, pbm_mod
+    T = max(64, 2 * n + n // 2 + 1)
+    pool = pbm.Pool(T, 64)
+    cfg = pbm.walk_config(pbm.LINKED_LIST, block_size=block_size)
+    queue = [np.arange(T)]                              # what each put brought, oldest first
+    out = []
+    for k in range(6):
+        ids = torch.empty(n, dtype=torch.int32, device="cuda")
+        pool.alloc(cfg, n, 0, ids)
+        got = ids.cpu().numpy()
+        flat = np.concatenate(queue)
+        want, rest = flat[:n], flat[n:]
+        assert np.array_equal(np.sort(got[got >= 0]), np.sort(want)) and (got < 0).sum() == n - len(want)
+        out.append(got[got >= 0])
+        queue = [rest]
+        if k >= 1:                                      # give the older of the two held batches back
+            back = out.pop(0)
+            # puts of one call have no order among themselves: keep the next gets to whole batches
+            padded = np.full(2 * len(back) + 1, -1, dtype=np.int32)
+            padded[1::2] = back
+            padded[0] = T + 3
+            pool.free(cfg, len(padded), torch.from_numpy(padded).cuda())
+            queue.append(back)
+            if len(np.concatenate(queue[:1])) < n:      # the next call would split a batch
+                break
+    st = pool.stats()
+    assert st.frees == st.successes - sum(len(x) for x in out)
+    more = torch.empty(T, dtype=torch.int32, device="cuda")
+    pool.alloc(cfg, T, 0, more)
+    left = T - sum(len(x) for x in out)
+    assert int((more >= 0).sum()) == left
+    chk = pool.check(more, T)
+    assert (chk.n_duplicates, chk.n_not_marked, chk.used_pages) == (0, 0, T)
+    pool.close()
