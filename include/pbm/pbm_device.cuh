@@ -102,6 +102,11 @@ __host__ __device__ __forceinline__ uint64_t hash64(uint64_t seed, uint64_t ctr)
     return z ^ (z >> 31);
 }
 
+// bits lo..hi (inclusive) of a 32-bit word
+__host__ __device__ __forceinline__ uint32_t bit_range(uint32_t lo, uint32_t hi) {
+    return (hi >= 31u ? kFull32 : ((1u << (hi + 1u)) - 1u)) & ~((1u << lo) - 1u);
+}
+
 #ifdef __CUDACC__
 
 // ---------------------------------------------------------------------------
@@ -693,6 +698,101 @@ __device__ __forceinline__ int32_t sweep_single(const PoolView& v, unsigned long
     return -1;
 }
 
+// The single clock's sweep for a warp's requests (lanes with `need`); the warp calls
+// converged.  The shared arm is one address, and one atomic per position examined
+// (and warp) queued there: 300,007 requests at 75% moved it some 190,000 times.
+// Here a warp moves the arm once over a window of positions, long enough to hold the
+// free pages it needs at the density seen last (at first: in 32 words drawn at
+// random), each lane reads one word of the window, and the first free pages in
+// sweep order are claimed, one atomicOr per word, and go to the needing lanes in lane
+// order.  Pages of the window beyond the need are passed until the arm comes round
+// again.  `alone`: no other warp of the launch moves the arm much, so the
+// unused end of the last window is given back (when the arm is still where this
+// warp left it): a launch of one block leaves the arm just past its last page and
+// passes no free page, as the one-thread sweep does.  A request's steps are the
+// positions from the page before its own; requests that find no page end after
+// max_steps positions each, taken together.
+constexpr uint32_t kClockWindow = 896;   // positions: at most 30 words, wrapped windows included
+
+__device__ __forceinline__ uint32_t clock_window(uint32_t m, uint32_t free_pages, uint32_t positions) {
+    // m / density, an eighth and 8 positions to spare
+    const uint32_t f = free_pages ? free_pages : 1u;
+    const uint32_t w = (uint32_t)(((unsigned long long)m * positions) / f);
+    const uint32_t p = w + (w >> 3) + 8u;
+    return p < kClockWindow ? p : kClockWindow;
+}
+
+__device__ __forceinline__ int32_t sweep_single_warp(const PoolView& v, unsigned long long* arm, bool need, int32_t seed,
+                                                     uint32_t max_steps, bool alone, int32_t* steps_out) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t T = v.n_pages;
+    int32_t id = -1, steps = need ? (int32_t)max_steps : 0;
+    uint32_t needm = __ballot_sync(kFull32, need);
+    if (!needm) {
+        if (steps_out) *steps_out = 0;
+        return -1;
+    }
+    unsigned long long left = (unsigned long long)__popc(needm) * max_steps;   // positions the requests may examine
+    uint32_t fr_seen = __reduce_add_sync(kFull32, (uint32_t)__popc(~load_word(v.words + idx_hi(seed, v.n_words32))));
+    uint32_t p_seen = 1024u;
+    unsigned long long passed = 0;                                 // positions since the last page claimed
+    while (needm && left) {
+        const uint32_t m = (uint32_t)__popc(needm);
+        uint32_t P = clock_window(m, fr_seen, p_seen);
+        if (P > T) P = T;
+        if (P > left) P = (uint32_t)left;
+        left -= P;
+        unsigned long long a0 = 0;
+        if (lane == 0u) a0 = atomicAdd(arm, (unsigned long long)P);
+        a0 = __shfl_sync(kFull32, a0, 0);
+        const uint32_t p0 = (uint32_t)(a0 % T);
+        // lane i: word i of the pages p0 .. p0 + P - 1, wrapping past the last page
+        const uint32_t w0 = p0 >> 5;
+        const uint32_t end_a = min(T, p0 + P);                     // first stretch [p0, end_a)
+        const uint32_t n_a = ((end_a + 31u) >> 5) - w0;
+        const uint32_t end_b = P - (end_a - p0);                   // second stretch [0, end_b)
+        const uint32_t w = lane < n_a ? w0 + lane : lane - n_a;
+        const uint32_t lo = lane < n_a ? max(p0, w << 5) : w << 5, hi = lane < n_a ? end_a : end_b;
+        uint32_t fr = 0u;
+        if ((w << 5) < hi) fr = ~load_word(v.words + w) & bit_range(lo & 31u, min(31u, hi - 1u - (w << 5)));
+        int cnt = __popc(fr);
+        int incl = group_incl_scan<32>(cnt, lane, kFull32);
+        fr_seen = (uint32_t)__shfl_sync(kFull32, incl, 31);
+        p_seen = P;
+        uint32_t got = low_bits(fr, (int)m - (incl - cnt));
+        if (got) got &= ~atomicOr(v.words + w, got);               // less what another claim took first
+        const int g = __popc(got);
+        const int gincl = group_incl_scan<32>(g, lane, kFull32);
+        const int G = __shfl_sync(kFull32, gincl, 31);
+        // needing lane of rank r takes page r of those claimed
+        const bool mine = (needm >> lane) & 1u;
+        const int r = mine ? __popc(needm & lt) : 0;
+        int src = 0;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1)
+            if (__shfl_sync(kFull32, gincl, src + step - 1) <= r) src += step;
+        const int src_excl = __shfl_sync(kFull32, gincl - g, src);
+        const uint32_t src_w = __shfl_sync(kFull32, w, src), src_got = __shfl_sync(kFull32, got, src);
+        const bool served = mine && r < G;
+        uint32_t at = 0u;                                          // position past the lane's page, from p0
+        if (served) {
+            id = (int32_t)((src_w << 5) + nth_set_bit(src_got, r - src_excl));
+            at = (uint32_t)id >= p0 ? (uint32_t)id - p0 + 1u : (uint32_t)id + (T - p0) + 1u;
+        }
+        const uint32_t before = needm & lt;
+        const uint32_t prev = __shfl_sync(kFull32, at, before ? 31 - __clz((int)before) : 0);
+        if (served) steps = (int32_t)min((unsigned long long)max_steps, before ? at - prev : passed + at);
+        const uint32_t at_last = __reduce_max_sync(kFull32, at);
+        passed = at_last ? P - at_last : passed + P;
+        if (alone && G >= (int)m && lane == 31u - (uint32_t)__clz((int)needm) && at < P)
+            atomicCAS(arm, a0 + P, a0 + at);                       // the end of the window was not needed
+        needm = __ballot_sync(kFull32, mine && !served);
+    }
+    if (steps_out) *steps_out = steps;
+    return id;
+}
+
 __device__ __forceinline__ int32_t sweep_dist(const PoolView& v, uint32_t* arm,
                                               uint32_t max_steps, int32_t* steps_out) {
     uint32_t s = 0, a = *arm;
@@ -766,11 +866,6 @@ __device__ __forceinline__ int32_t walk_run(const PoolView& v, uint32_t n, int32
 // set is released again and the walk jumps anew.  steps = jumps.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kMaxSpanPages = 1u << 16;
-
-// bits lo..hi (inclusive) of a 32-bit word
-__host__ __device__ __forceinline__ uint32_t bit_range(uint32_t lo, uint32_t hi) {
-    return (hi >= 31u ? kFull32 : ((1u << (hi + 1u)) - 1u)) & ~((1u << lo) - 1u);
-}
 
 // mask of the pages of run [p0, p0+n) that lie in word ww
 __host__ __device__ __forceinline__ uint32_t span_mask(uint32_t p0, uint32_t n, uint32_t ww) {

@@ -44,7 +44,7 @@ enum class Walk { Page, Word32, Word64, Crw, SingleClock, DistClock };
 // Per-thread strategies.  The loop runs whole warps (uniform trip count) so
 // the block-level flush can use full-warp shuffles.
 template <Walk K>
-__global__ void __launch_bounds__(256, 8) k_alloc_thread(AllocArgs a) {
+__global__ void __launch_bounds__(256, K == Walk::SingleClock ? 6 : 8) k_alloc_thread(AllocArgs a) {
     Acc acc;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nthr = (uint64_t)gridDim.x * blockDim.x;
@@ -62,6 +62,14 @@ __global__ void __launch_bounds__(256, 8) k_alloc_thread(AllocArgs a) {
         if (K == Walk::Page && blockDim.x >= 32u) {
             int32_t ws = 0;
             const int32_t wid = walk_page_warp(a.v, go && id < 0, request_seed(a.seed, (uint32_t)r), a.max_steps, &ws);
+            if (go && id < 0) {
+                id = wid;
+                s = ws;
+            }
+        } else if (K == Walk::SingleClock && blockDim.x >= 32u) {
+            int32_t ws = 0;
+            const int32_t wid = sweep_single_warp(a.v, a.arm, go && id < 0, request_seed(a.seed, (uint32_t)r),
+                                                  a.max_steps, gridDim.x == 1u, &ws);
             if (go && id < 0) {
                 id = wid;
                 s = ws;

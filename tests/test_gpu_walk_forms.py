@@ -134,3 +134,69 @@ def test_free_list_serves_blocks_in_release_order(cuda, pbm_mod, n, block_size):
     chk = pool.check(more, T)
     assert (chk.n_duplicates, chk.n_not_marked, chk.used_pages) == (0, 0, T)
     pool.close()
+
+
+@pytest.mark.parametrize("T,occ", [(40, 0.2), (96, 0.5), (1000, 0.9), (8192 + 5, 0.5), (1 << 16, 0.99), (1 << 18, 0.02)])
+@pytest.mark.parametrize("n", [1, 2, 31, 32])
+def test_clock_sweep_of_one_warp_takes_the_next_free_pages(cuda, pbm_mod, orc, T, occ, n):
+    """Launches of one warp, one after the other and round the pool: together they take the free pages
+    in sweep order and pass none, as the one-thread sweep does; steps add up to the positions passed."""
+    torch, pbm = cuda, pbm_mod
+    words = orc.bernoulli_bitmap(T, occ, 4)
+    bits = np.unpackbits(words.view(np.uint8), bitorder="little")[:T]
+    order = np.nonzero(bits == 0)[0]
+    pool = pbm.Pool(T, 64)
+    pool.prefill(occ, 4)
+    cfg = pbm.walk_config(pbm.SINGLE_CLOCK, max_steps=1 << 20)
+    ids = torch.empty(n, dtype=torch.int32, device="cuda")
+    steps = torch.empty(n, dtype=torch.int32, device="cuda")
+    taken = 0
+    for S in range(min(6, len(order) // n)):
+        pool.alloc(cfg, n, S, ids, steps)
+        want = order[taken:taken + n]
+        assert np.array_equal(ids.cpu().numpy(), want)
+        first = order[taken - 1] + 1 if taken else 0
+        assert int(steps.sum()) == want[-1] + 1 - first
+        taken += n
+    # free what was taken: the arm, past it, reaches those pages again after the rest of the pool
+    if taken:
+        back = torch.from_numpy(order[:taken].astype(np.int32)).cuda()
+        pool.free(cfg, taken, back)
+        rest = len(order) - taken + taken
+        got = []
+        for S in range(rest // n):
+            pool.alloc(cfg, n, 50 + S, ids)
+            got.append(ids.cpu().numpy())
+            if S >= 40:
+                break
+        got = np.concatenate(got)
+        assert np.array_equal(got, np.concatenate([order[taken:], order[:taken]])[:len(got)])
+    pool.close()
+
+
+@pytest.mark.parametrize("T,occ,n", [(1 << 16, 0.97, 1900), (1 << 20, 0.9, 50000), (1 << 20, 0.0, 300000), (3000, 0.0, 2999),
+                                     (100000, 0.5, 60000)])
+@pytest.mark.parametrize("max_steps", [1, 5, 4096])
+def test_clock_sweep_of_many_warps(cuda, pbm_mod, orc, T, occ, n, max_steps):
+    """Pages are distinct and were free; no request reports more than max_steps positions; with room and a
+    generous bound all are served, and a launch never examines more than its bound allows."""
+    torch, pbm = cuda, pbm_mod
+    pool = pbm.Pool(T, 64)
+    pool.prefill(occ, 3)
+    before = pool.read_bitmap()
+    free = T - orc.used_pages(before, T)
+    ids = torch.empty(n, dtype=torch.int32, device="cuda")
+    steps = torch.empty(n, dtype=torch.int32, device="cuda")
+    pool.alloc(pbm.walk_config(pbm.SINGLE_CLOCK, max_steps=max_steps), n, 1, ids, steps)
+    got, st = ids.cpu().numpy(), steps.cpu().numpy()
+    chk = pool.check(ids, n)
+    assert (chk.n_duplicates, chk.n_not_marked, chk.n_out_of_range) == (0, 0, 0)
+    assert chk.used_pages == T - free + chk.n_ok
+    h = got[got >= 0]
+    assert not ((before[h >> 5] >> (h & 31).astype(np.uint32)) & 1).any()
+    assert st.max() <= max_steps and st.min() >= 1 and (st[got < 0] == max_steps).all()
+    if max_steps == 4096:
+        assert chk.n_ok == min(n, free)
+    pool.free(pbm.walk_config(pbm.SINGLE_CLOCK), n, ids)
+    assert np.array_equal(pool.read_bitmap(), before)
+    pool.close()
