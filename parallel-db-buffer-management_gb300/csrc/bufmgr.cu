@@ -365,43 +365,94 @@ __device__ __forceinline__ int32_t sweep_warp(const BmView& b, uint32_t loaders,
     return out;
 }
 
-// The loaders' side of a cooperative miss: copy the new pages from the
-// backing store with the whole warp, then publish the entries.  The warp's
-// copies are one flat run of 16-byte pieces (loader by loader, piece by
-// piece); each lane has kCopyInFlight of its pieces loading at once before
-// it stores them, so a warp keeps 32 x kCopyInFlight loads in flight across
-// its loaders' pages.  The whole warp calls converged.
-constexpr uint32_t kCopyInFlight = 4;
+// Bulk copies between global and shared memory (the TMA's untiled form: 16-byte
+// aligned addresses, sizes a multiple of 16).
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar) {
+    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    for (uint32_t i = 0; i < kFetchSpinLimit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_stores_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_stores_done() {
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async;" ::: "memory");
+}
+
+// The loaders' side of a cooperative miss: copy the new pages from the backing
+// store with the whole warp, then publish the entries.  The warp's copies are a run
+// of pieces (loader by loader) of at most kCopyPiece bytes; a lane brings one
+// piece at a time into its own slot of the warp's staging buffer with one bulk load and
+// sends it to the frame with one bulk store, so a warp has kCopyStage bytes
+// in flight with two instructions per piece.  Copying through registers, four 16-byte
+// loads per lane, kept 2 KiB per warp in flight: a round of 16,384 fetches (30%
+// misses) of 4 KiB pages took 41 us, of which COPY_NOTE.  The whole warp
+// calls converged.
+constexpr uint32_t kCopyPiece = 4096;
+constexpr uint32_t kCopyStage = 32768;   // per warp
+
+__host__ __device__ __forceinline__ uint32_t copy_piece(uint32_t frame_size) {
+    return frame_size < kCopyPiece ? frame_size : kCopyPiece;
+}
+// Pieces a warp has in flight: one slot per lane at most.
+__host__ __device__ __forceinline__ uint32_t copy_slots(uint32_t frame_size) {
+    const uint32_t s = kCopyStage / copy_piece(frame_size);
+    return s < 32u ? s : 32u;
+}
+
+struct CopyStage {
+    uint32_t buf;      // this lane's slot (shared address)
+    uint32_t bar;      // its barrier
+    uint32_t parity;   // of the barrier's next completion
+};
 
 template <bool COPY>
-__device__ __forceinline__ void finish_loads_warp(const BmView& b, bool loader, uint32_t page, int32_t h,
+__device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs, bool loader, uint32_t page, int32_t h,
                                                   uint32_t old_page, uint32_t k, BmAcc& acc) {
     if (COPY) {
         const uint32_t lane = threadIdx.x & 31u;
-        const uint32_t n16 = b.frame_size / 16u;
         const uint32_t todo = __ballot_sync(0xffffffffu, loader && h >= 0);
-        const uint32_t total = (uint32_t)__popc(todo) * n16;
-        for (uint32_t base = 0; base < total; base += 32u * kCopyInFlight) {
-            int4 v[kCopyInFlight];
-            int4* dst[kCopyInFlight];
-#pragma unroll
-            for (uint32_t u = 0; u < kCopyInFlight; ++u) {
-                const uint32_t c = base + u * 32u + lane;
-                const uint32_t li = (c < total ? c : 0u) / n16;
-                const int l = (int)nth_set_bit(todo, (int)li);   // every lane shuffles
-                const uint32_t pg = __shfl_sync(0xffffffffu, page, l);
-                const int32_t fr = __shfl_sync(0xffffffffu, h, l);
-                const uint32_t j = c - li * n16;
-                dst[u] = nullptr;
-                if (c < total) {
-                    v[u] = reinterpret_cast<const int4*>(b.backing + (size_t)pg * b.frame_size)[j];
-                    dst[u] = reinterpret_cast<int4*>(b.frames + (size_t)(uint32_t)fr * b.frame_size) + j;
-                }
+        const uint32_t slots = copy_slots(b.frame_size), piece = copy_piece(b.frame_size);
+        const uint32_t per = (b.frame_size + piece - 1u) / piece;          // pieces per page
+        const uint32_t total = (uint32_t)__popc(todo) * per;
+        for (uint32_t base = 0; base < total; base += slots) {
+            const uint32_t c = base + lane;
+            const bool mine = lane < slots && c < total;
+            const uint32_t li = (mine ? c : 0u) / per;
+            const int l = (int)nth_set_bit(todo, (int)li);                 // every lane shuffles
+            const uint32_t pg = __shfl_sync(0xffffffffu, page, l);
+            const int32_t fr = __shfl_sync(0xffffffffu, h, l);
+            if (mine) {
+                const uint32_t off = (c - li * per) * piece;
+                const uint32_t bytes = b.frame_size - off < piece ? b.frame_size - off : piece;
+                bulk_stores_read();                                        // the slot's last piece has left it
+                bulk_load(cs.buf, b.backing + (size_t)pg * b.frame_size + off, bytes, cs.bar);
+                if (!mbar_wait(cs.bar, cs.parity)) ++acc.timeouts;         // reported: the page's bytes are late
+                cs.parity ^= 1u;
+                bulk_store(b.frames + (size_t)(uint32_t)fr * b.frame_size + off, cs.buf, bytes);
             }
-#pragma unroll
-            for (uint32_t u = 0; u < kCopyInFlight; ++u)
-                if (dst[u]) *dst[u] = v[u];
         }
+        if (total) bulk_stores_done();
         __syncwarp();
     }
     if (loader) publish(b, page, h, old_page, k, acc);
@@ -456,28 +507,30 @@ __device__ __forceinline__ bool release_target(const BmView& b, int32_t v, uint3
 // queue on one page's entry by the block's warps.  Releases by page share
 // the fetches' table: a block that releases and fetches one page moves its
 // pins with one atomic.
-constexpr uint32_t kMergeSlots = 1024;           // >= 2 x the keys of one block (256 fetches + 256 releases)
+// A table has twice as many slots as the block can have keys (KEYS: a power of two).
 constexpr uint32_t kMergeEmpty = 0xffffffffu;   // no page or frame id reaches it
 constexpr uint32_t kMergeFirst = 1u << 31;
 
+template <uint32_t KEYS, bool FRAMES>
 struct MergeTables {
-    uint32_t fkey[kMergeSlots];   // pages (and, releasing by page, released pages)
-    uint32_t fcnt[kMergeSlots];   // fetches of the page
-    uint32_t frel[kMergeSlots];   // releases of the page (releasing by page)
-    int32_t fres[kMergeSlots];    // the fetch's frame
-    uint32_t rkey[kMergeSlots];   // released frames (releasing by frame)
-    uint32_t rcnt[kMergeSlots];
+    uint32_t fkey[2 * KEYS];   // pages (and, releasing by page, released pages)
+    uint32_t fcnt[2 * KEYS];   // fetches of the page
+    uint32_t frel[2 * KEYS];   // releases of the page (releasing by page)
+    int32_t fres[2 * KEYS];    // the fetch's frame
+    uint32_t rkey[FRAMES ? 2 * KEYS : 1];   // released frames (releasing by frame)
+    uint32_t rcnt[FRAMES ? 2 * KEYS : 1];
 };
 
 // Adds c to cnt[slot of key]; returns the slot, with kMergeFirst set for the
 // lane whose add came first (the slot's leader for that count).  A table
 // never holds more keys than half its slots, so a slot is found.
+template <uint32_t KEYS>
 __device__ __forceinline__ uint32_t merge_insert(uint32_t* keys, uint32_t* cnt, uint32_t key, uint32_t c) {
-    uint32_t h = (key * 2654435761u) >> 22;   // 10 bits: kMergeSlots
-    for (uint32_t probe = 0; probe < kMergeSlots; ++probe) {
+    uint32_t h = (uint32_t)(((unsigned long long)(key * 2654435761u) * (2u * KEYS)) >> 32);
+    for (uint32_t probe = 0; probe < 2u * KEYS; ++probe) {
         const uint32_t prev = atomicCAS(keys + h, kMergeEmpty, key);
         if (prev == kMergeEmpty || prev == key) return atomicAdd(cnt + h, c) == 0u ? (h | kMergeFirst) : h;
-        h = (h + 1u) & (kMergeSlots - 1u);
+        h = (h + 1u) & (2u * KEYS - 1u);
     }
     return kMergeEmpty;   // not reached
 }
@@ -495,13 +548,24 @@ __device__ __forceinline__ uint32_t merge_insert(uint32_t* keys, uint32_t* cnt, 
 // round may land after other blocks' fetches of the same round; a sweep
 // that meets a page whose release has not landed yet passes it as pinned,
 // as it would any pinned page.
-template <bool DIST, bool BYPAGE, bool COPY>
+template <bool DIST, bool BYPAGE, bool COPY, int BLOCK>
 __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* release_of, const int32_t* release_idx,
                                              uint32_t n_release, const int32_t* pages, uint32_t n, uint32_t slot0,
                                              int32_t* frames_out, int32_t* held_out, unsigned long long& ok,
                                              unsigned long long& bad, BmAcc& acc) {
-    __shared__ MergeTables t;
+    constexpr uint32_t KEYS = 2u * BLOCK;   // BLOCK fetches and BLOCK releases
+    __shared__ MergeTables<KEYS, !BYPAGE> t;
     const uint32_t lane = threadIdx.x & 31u;
+    CopyStage cs{};
+    if constexpr (COPY) {
+        extern __shared__ __align__(128) unsigned char stage[];
+        __shared__ unsigned long long bars[BLOCK];
+        const uint32_t piece = copy_piece(b.frame_size), slots = copy_slots(b.frame_size);
+        cs.buf = smem_addr(stage) + ((threadIdx.x >> 5) * slots + (lane < slots ? lane : 0u)) * piece;
+        cs.bar = smem_addr(bars + threadIdx.x);
+        mbar_init(cs.bar);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the barriers before the copies that use them
+    }
     const uint64_t work = n > n_release ? n : n_release;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     // block-uniform trip count
@@ -511,7 +575,7 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
         if (!DIST && lane == 0u) hbase = atomicAdd(b.single_hand, 32ull);   // the first sweep window
         const int32_t ri = i < n_release ? __ldg(release_idx + i) : -1;
         const int32_t p = i < n ? __ldg(pages + i) : -1;
-        for (uint32_t s = threadIdx.x; s < kMergeSlots; s += blockDim.x) {
+        for (uint32_t s = threadIdx.x; s < 2u * KEYS; s += BLOCK) {
             t.fkey[s] = kMergeEmpty;
             t.fcnt[s] = 0u;
             t.frel[s] = 0u;
@@ -536,10 +600,10 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
         if (BYPAGE && rv >= 0 && !rin && (uint32_t)(__ffs((int)rpeers) - 1) == lane) bad += (uint32_t)__popc(rpeers);
         __syncthreads();   // tables clear
         uint32_t fslot = kMergeEmpty, rslot = kMergeEmpty;
-        if (valid && lane == leader) fslot = merge_insert(t.fkey, t.fcnt, (uint32_t)p, (uint32_t)__popc(peers));
+        if (valid && lane == leader) fslot = merge_insert<KEYS>(t.fkey, t.fcnt, (uint32_t)p, (uint32_t)__popc(peers));
         if (rin && (uint32_t)(__ffs((int)rpeers) - 1) == lane)
-            rslot = BYPAGE ? merge_insert(t.fkey, t.frel, (uint32_t)rv, (uint32_t)__popc(rpeers))
-                           : merge_insert(t.rkey, t.rcnt, (uint32_t)rv, (uint32_t)__popc(rpeers));
+            rslot = BYPAGE ? merge_insert<KEYS>(t.fkey, t.frel, (uint32_t)rv, (uint32_t)__popc(rpeers))
+                           : merge_insert<KEYS>(t.rkey, t.rcnt, (uint32_t)rv, (uint32_t)__popc(rpeers));
         __syncthreads();   // counts complete
         if (!DIST) w0.e = w0.q < b.n_logical ? __ldcg(b.pt + w0.q) : 0ull;
         // the page's fetch leader moves the block's pins of it with one atomic
@@ -585,14 +649,14 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
             const uint32_t lm = __ballot_sync(0xffffffffu, st == kStLoad);
             uint32_t old_page = kEmptyPage;
             const int32_t h = sweep_warp(b, lm, (uint32_t)p, &old_page, &w0);
-            if (lm) finish_loads_warp<COPY>(b, st == kStLoad, (uint32_t)p, h, old_page, k, acc);
+            if (lm) finish_loads_warp<COPY>(b, cs, st == kStLoad, (uint32_t)p, h, old_page, k, acc);
             if (st == kStLoad) f = h;
-        } else if (st == kStLoad) {
+        } else if (__any_sync(0xffffffffu, st == kStLoad)) {
             uint32_t old_page = kEmptyPage;
-            const int32_t h = sweep_private(b, (uint32_t)p, slot, &old_page);
-            if (COPY && h >= 0) copy_frame(b, (uint32_t)p, h);
-            publish(b, (uint32_t)p, h, old_page, k, acc);
-            f = h;
+            int32_t h = -1;
+            if (st == kStLoad) h = sweep_private(b, (uint32_t)p, slot, &old_page);
+            finish_loads_warp<COPY>(b, cs, st == kStLoad, (uint32_t)p, h, old_page, k, acc);
+            if (st == kStLoad) f = h;
         }
         if (st == kStWait) {
             f = wait_loaded(b, (uint32_t)p);
@@ -620,24 +684,52 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
     }
 }
 
-// A round of releases only (no fetch): the lanes of a warp that release
-// one name merge into one atomic, and no sweep runs, so the hand stays where
-// it is.  BYPAGE as for k_round.
+// A round of releases only (no fetch): the block's releases of one name meet
+// in a shared-memory table and go as one atomic, and no sweep runs, so the hand
+// stays where it is.  BYPAGE as for k_round.  Merged within the warp only, the
+// hottest page's entry took an atomic from nearly every warp: 471,000 releases of a
+// Zipf(0.99) stream took REL_NOTE us.
+constexpr int kReleaseItems = 2;   // per thread, their reads in flight together
+
 template <bool BYPAGE>
-__global__ void __launch_bounds__(256, 4) k_release(BmView b, const int32_t* release_of, const int32_t* release_idx,
+__global__ void __launch_bounds__(256) k_release(BmView b, const int32_t* release_of, const int32_t* release_idx,
                                                  uint32_t n_release) {
+    constexpr uint32_t KEYS = 256u * kReleaseItems;
+    __shared__ uint32_t keys[2 * KEYS], cnt[2 * KEYS];
     unsigned long long ok = 0, bad = 0;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    // warp-uniform trip count (blockDim is a multiple of 32)
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < n_release; base += stride) {
-        const uint64_t j = base + lane;
-        const int32_t rv = j < n_release ? __ldcg(release_of + __ldg(release_idx + j)) : -1;
-        const uint32_t peers = __match_any_sync(0xffffffffu, rv >= 0 ? (uint32_t)rv : 0x80000000u + lane);
+    const uint64_t base = (uint64_t)blockIdx.x * (256u * kReleaseItems) + threadIdx.x;
+    int32_t rv[kReleaseItems];
+#pragma unroll
+    for (int u = 0; u < kReleaseItems; ++u) {
+        const uint64_t j = base + (uint64_t)u * 256u;
+        rv[u] = j < n_release ? __ldg(release_idx + j) : -1;
+    }
+    for (uint32_t s = threadIdx.x; s < 2u * KEYS; s += 256u) {
+        keys[s] = kMergeEmpty;
+        cnt[s] = 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < kReleaseItems; ++u)
+        if (base + (uint64_t)u * 256u < n_release) rv[u] = __ldcg(release_of + rv[u]);
+    __syncthreads();   // table clear
+    uint32_t slot[kReleaseItems];
+#pragma unroll
+    for (int u = 0; u < kReleaseItems; ++u) {
+        const bool have = base + (uint64_t)u * 256u < n_release && rv[u] >= 0;
+        const uint32_t peers = __match_any_sync(0xffffffffu, have ? (uint32_t)rv[u] : 0x80000000u + lane);
+        slot[u] = kMergeEmpty;
+        if (have && (uint32_t)(__ffs((int)peers) - 1) == lane)
+            slot[u] = merge_insert<KEYS>(keys, cnt, (uint32_t)rv[u], (uint32_t)__popc(peers));
+    }
+    __syncthreads();   // counts complete
+#pragma unroll
+    for (int u = 0; u < kReleaseItems; ++u) {
+        if (slot[u] == kMergeEmpty || !(slot[u] & kMergeFirst)) continue;
         uint32_t q = 0;
         int32_t f = -1;
-        const uint32_t k = (uint32_t)__popc(peers);
-        if (rv >= 0 && (uint32_t)(__ffs((int)peers) - 1) == lane && release_target<BYPAGE>(b, rv, k, &q, &f, bad))
+        const uint32_t k = cnt[slot[u] & ~kMergeFirst];
+        if (release_target<BYPAGE>(b, rv[u], k, &q, &f, bad))
             release_check(b, q, f, k, release_issue(b, q, k), ok, bad);
     }
     block_add_counters<2>({ok, bad}, {&b.stats->unpins, &b.stats->bad_unpins});
@@ -649,8 +741,8 @@ __global__ void __launch_bounds__(256, 4) k_release(BmView b, const int32_t* rel
 // release_of names pages, else frames.  COPY: misses copy their page from
 // the backing store (b.backing and b.frames set).  held_out (may be null)
 // receives each fetch's page, or -1 where the fetch got no frame.
-template <bool DIST, bool BYPAGE, bool COPY>
-__global__ void __launch_bounds__(256) k_round(BmView b, const int32_t* release_of, const int32_t* release_idx,
+template <bool DIST, bool BYPAGE, bool COPY, int BLOCK>
+__global__ void __launch_bounds__(BLOCK) k_round(BmView b, const int32_t* release_of, const int32_t* release_idx,
                                                uint32_t n_release, const int32_t* pages, uint32_t n, uint32_t slot0,
                                                int32_t* frames_out, int32_t* held_out) {
     unsigned long long ok = 0, bad = 0;
@@ -671,7 +763,7 @@ __global__ void __launch_bounds__(256) k_round(BmView b, const int32_t* release_
             if (held_out) held_out[i] = f >= 0 ? p : -1;
         }
     } else {
-        round_blocks<DIST, BYPAGE, COPY>(b, release_of, release_idx, n_release, pages, n, slot0, frames_out, held_out, ok,
+        round_blocks<DIST, BYPAGE, COPY, BLOCK>(b, release_of, release_idx, n_release, pages, n, slot0, frames_out, held_out, ok,
                                    bad, acc);
     }
     block_add_counters<7>({ok, bad, acc.hits, acc.misses, acc.evictions, acc.failures, acc.timeouts},
@@ -826,11 +918,9 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     pbm::DeviceScope scope(m->device);
     if (n == 0 && n_release == 0) return PBM_OK;
     const uint32_t work = n > n_release ? n : n_release;
-    const int block = serial ? 1 : 256;
-    const int grid = serial ? 1 : (int)((work + 255u) / 256u);
     cudaStream_t s = (cudaStream_t)stream;
     if (n == 0 && !serial) {   // releases only: no fetch, no sweep
-        const int rgrid = (int)((n_release + 255u) / 256u);
+        const int rgrid = (int)(((uint64_t)n_release + 256u * kReleaseItems - 1u) / (256u * kReleaseItems));
         if (by_page)
             k_release<true><<<rgrid, 256, 0, s>>>(m->v, d_release_of, d_release_idx, n_release);
         else
@@ -838,22 +928,39 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
         PBM_LAUNCH_CHECK();
         return PBM_OK;
     }
-    auto go = [&](auto kernel) {
-        kernel<<<grid, block, 0, s>>>(m->v, d_release_of, d_release_idx, n_release, d_pages, n, slot0, d_frames_out,
-                                      d_held_out);
-    };
+    // Blocks of 64 threads for rounds that would not give every SM two blocks of 256 (a
+    // round of 16,384 fetches is 64 such blocks), and for rounds that copy, whose
+    // staging buffers (32 KiB a warp) are then shared out in small blocks.  A larger round
+    // that copies nothing merges its requests over 256 threads.
     const bool copy = m->v.backing && m->v.frames;
+    const bool small = copy || work < (uint32_t)sm_count() * 512u;
+    const int block = serial ? 1 : small ? 64 : 256;
+    const int grid = serial ? 1 : (int)(((uint64_t)work + (uint32_t)block - 1u) / (uint32_t)block);
+    const size_t stage = copy && !serial ? 2u * (size_t)copy_slots(m->v.frame_size) * copy_piece(m->v.frame_size) : 0u;
+    cudaError_t attr = cudaSuccess;
+    auto go = [&](auto kernel) {
+        if (stage) attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)kCopyStage);
+        if (attr == cudaSuccess)
+            kernel<<<grid, block, stage, s>>>(m->v, d_release_of, d_release_idx, n_release, d_pages, n, slot0, d_frames_out,
+                                              d_held_out);
+    };
     if (copy) {
         if (m->v.dist)
-            by_page ? go(k_round<true, true, true>) : go(k_round<true, false, true>);
+            by_page ? go(k_round<true, true, true, 64>) : go(k_round<true, false, true, 64>);
         else
-            by_page ? go(k_round<false, true, true>) : go(k_round<false, false, true>);
+            by_page ? go(k_round<false, true, true, 64>) : go(k_round<false, false, true, 64>);
+    } else if (small) {
+        if (m->v.dist)
+            by_page ? go(k_round<true, true, false, 64>) : go(k_round<true, false, false, 64>);
+        else
+            by_page ? go(k_round<false, true, false, 64>) : go(k_round<false, false, false, 64>);
     } else {
         if (m->v.dist)
-            by_page ? go(k_round<true, true, false>) : go(k_round<true, false, false>);
+            by_page ? go(k_round<true, true, false, 256>) : go(k_round<true, false, false, 256>);
         else
-            by_page ? go(k_round<false, true, false>) : go(k_round<false, false, false>);
+            by_page ? go(k_round<false, true, false, 256>) : go(k_round<false, false, false, 256>);
     }
+    PBM_CUDA_TRY(attr);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }

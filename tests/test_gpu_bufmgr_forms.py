@@ -1,0 +1,87 @@
+"""Buffer-manager rounds at the sizes where the launch changes form: blocks of 64 and 256
+threads, frames copied in one or several pieces, releases merged over a block.  Whole
+numbers and bytes, compared exactly."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("frame_size", [16, 48, 1040, 4096, 4112, 12304])
+@pytest.mark.parametrize("policy", [0, 1])
+@pytest.mark.parametrize("by_page", [True, False])
+def test_every_copied_frame_holds_its_page(cuda, pbm_mod, frame_size, policy, by_page):
+    torch, pbm = cuda, pbm_mod
+    n_logical, n_frames, R, rounds = 6000, 1500, 333, 12
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(frame_size)
+    words = frame_size // 4
+    backing = torch.randint(-2**31, 2**31 - 1, (n_logical, words), generator=gen, device="cuda", dtype=torch.int32)
+    bm = pbm.BufferManager(n_logical, n_frames, frame_size=frame_size, policy=policy, n_arms=R if policy else 1,
+                           backing=backing)
+    rng = np.random.default_rng(1)
+    prev = idx = None
+    for r in range(rounds):
+        # some pages asked for by many requests of the round, and some ids that name no page
+        pages = np.where(rng.random(R) < 0.3, rng.integers(0, 5, R), rng.integers(0, n_logical, R)).astype(np.int32)
+        pages[rng.random(R) < 0.02] = -1
+        d = torch.from_numpy(pages).cuda()
+        frames = torch.empty(R, dtype=torch.int32, device="cuda")
+        held = torch.empty(R, dtype=torch.int32, device="cuda")
+        k = 0 if prev is None else R
+        if by_page:
+            bm.round_pages(prev, idx, k, d, R, r * R, frames, held)
+            assert np.array_equal(held.cpu().numpy(), np.where(pages >= 0, pages, -1))
+        else:
+            bm.round(prev, idx, k, d, R, r * R, frames)
+        out = torch.empty(R, words, dtype=torch.int32, device="cuda")
+        bm.gather(frames, R, frame_size, out)
+        ok = d >= 0
+        assert torch.equal(frames >= 0, ok)
+        assert torch.equal(out[ok], backing[d[ok].long()])
+        prev, idx = (held if by_page else frames), torch.randperm(R, device="cuda").to(torch.int32)
+    if by_page:
+        bm.round_pages(prev, idx, R, None, 0, 0, None)
+    else:
+        bm.round(prev, idx, R, None, 0, 0, None)
+    c, chk = bm.counters(), bm.check()
+    assert (c.bad_unpins, c.timeouts, c.failures, chk.mismatches, chk.loading, chk.pins) == (0, 0, 0, 0, 0, 0)
+    assert c.hits + c.misses == c.unpins and c.evictions > 0
+    bm.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 511, 513, 5000, 80001])
+@pytest.mark.parametrize("by_page", [True, False])
+def test_release_rounds_move_exactly_the_listed_pins(cuda, pbm_mod, n, by_page):
+    """Each page is fetched several times and released in parts: after every part the pins of every page
+    are what the host counts; releases of pins that are not held are refused and counted."""
+    torch, pbm = cuda, pbm_mod
+    n_logical, n_frames = 4096, 4096
+    rng = np.random.default_rng(n)
+    pages = np.minimum(rng.zipf(1.3, n) - 1, n_logical - 1).astype(np.int32)
+    bm = pbm.BufferManager(n_logical, n_frames)
+    d = torch.from_numpy(pages).cuda()
+    frames = torch.empty(n, dtype=torch.int32, device="cuda")
+    held = torch.empty(n, dtype=torch.int32, device="cuda")
+    bm.round_pages(None, None, 0, d, n, 0, frames, held)
+    order = torch.from_numpy(rng.permutation(n).astype(np.int32)).cuda()
+    pins = np.bincount(pages, minlength=n_logical)
+    for lo, hi in ((0, n // 3), (n // 3, n)):
+        if hi == lo:
+            continue
+        if by_page:
+            bm.round_pages(held, order[lo:], hi - lo, None, 0, 0, None)
+        else:
+            bm.round(frames, order[lo:], hi - lo, None, 0, 0, None)
+        pins = pins - np.bincount(pages[order[lo:hi].cpu().numpy()], minlength=n_logical)
+        assert np.array_equal(bm.read_tables()[1], pins)
+    c = bm.counters()
+    assert (c.unpins, c.bad_unpins) == (n, 0) and not pins.any()
+    extra = torch.tensor([0], dtype=torch.int32, device="cuda")
+    if by_page:
+        bm.round_pages(held, extra, 1, None, 0, 0, None)
+    else:
+        bm.round(frames, extra, 1, None, 0, 0, None)
+    c = bm.counters()
+    assert (c.unpins, c.bad_unpins) == (n, 1) and not bm.read_tables()[1].any()
+    bm.close()
