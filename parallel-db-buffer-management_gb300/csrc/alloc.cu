@@ -45,6 +45,7 @@ enum class Walk { Page, Word32, Word64, Crw, SingleClock, DistClock };
 // the block-level flush can use full-warp shuffles.
 template <Walk K>
 __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 6 : 8) k_alloc_thread(AllocArgs a) {
+    stream_wait();
     Acc acc;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nthr = (uint64_t)gridDim.x * blockDim.x;
@@ -116,6 +117,7 @@ __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 6 : 8) k_alloc_t
 // (blockDim == W, one block) replays the groups in request order.
 template <int W, typename Word>
 __global__ void __launch_bounds__(256) k_alloc_collab(AllocArgs a) {
+    stream_wait();
     __shared__ int32_t slots[256];
     Acc acc;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -164,6 +166,7 @@ constexpr int kFifoItems = 4;
 
 template <int ITEMS>
 __global__ void __launch_bounds__(256) k_fifo_alloc(AllocArgs a, FifoState* st, int32_t* ring) {
+    stream_wait();
     Acc acc;
     if (blockDim.x & 31u) {
         for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < a.n; r += (uint64_t)gridDim.x * blockDim.x) {
@@ -228,6 +231,7 @@ __global__ void __launch_bounds__(256) k_fifo_alloc(AllocArgs a, FifoState* st, 
 template <int ITEMS>
 __global__ void __launch_bounds__(256) k_fifo_free(PoolView v, uint32_t n, const int32_t* ids,
                                                    FifoState* st, int32_t* ring, DevStats* stats) {
+    stream_wait();
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_slot;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -305,6 +309,7 @@ __global__ void __launch_bounds__(256) k_fifo_free(PoolView v, uint32_t n, const
 // (the configuration's free_merge).
 template <bool MERGE>
 __global__ void __launch_bounds__(256) k_free_pages(PoolView v, uint32_t n, const int32_t* ids, DevStats* stats) {
+    stream_wait();
     unsigned long long f = 0;
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nthr = (uint64_t)gridDim.x * blockDim.x;
@@ -358,6 +363,7 @@ __global__ void __launch_bounds__(256) k_free_pages(PoolView v, uint32_t n, cons
 // word holds the run (1 <= k <= 32, the reference's getXPage semantics).
 template <bool SPAN>
 __global__ void __launch_bounds__(256) k_alloc_runs(AllocArgs a, const int32_t* npages) {
+    stream_wait();
     Acc acc;
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < a.n; r += (uint64_t)gridDim.x * blockDim.x) {
         int32_t k = npages[r];
@@ -379,6 +385,7 @@ __global__ void __launch_bounds__(256) k_alloc_runs(AllocArgs a, const int32_t* 
 
 __global__ void __launch_bounds__(256) k_free_runs(PoolView v, uint32_t n, const int32_t* ids,
                                                    const int32_t* npages, DevStats* stats) {
+    stream_wait();
     unsigned long long f = 0;
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (uint64_t)gridDim.x * blockDim.x) {
         int32_t id = ids[r], k = npages[r];
@@ -396,6 +403,7 @@ __global__ void __launch_bounds__(256) k_free_runs(PoolView v, uint32_t n, const
 // and frees the page unless `hold` (unitTest1.5.cu:138-150 get/free kernels
 // plus the payload write of the page-pool workload).
 __global__ void __launch_bounds__(256) k_claim_write_free(AllocArgs a, uint32_t payload_words, int hold) {
+    stream_wait();
     Acc acc;
     unsigned long long frees = 0;
     const uint64_t n_round = ((uint64_t)a.n + 31u) & ~31ull;   // whole warps walk together
@@ -426,6 +434,7 @@ __global__ void __launch_bounds__(256) k_claim_write_free(AllocArgs a, uint32_t 
 
 __global__ void k_gather_pages(PoolView v, const int32_t* ids, uint32_t n, uint32_t words_per_page,
                                int32_t* out) {
+    stream_wait();
     const unsigned long long total = (unsigned long long)n * words_per_page;
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (unsigned long long)gridDim.x * blockDim.x) {
@@ -491,7 +500,7 @@ AllocArgs make_args(pbm_pool* p, const pbm_walk_config* c, uint32_t n, uint32_t 
 
 template <int W, typename Word>
 int launch_collab_w(const AllocArgs& a, int grid, int block, cudaStream_t s) {
-    k_alloc_collab<W, Word><<<grid, block, 0, s>>>(a);
+    launch_next(k_alloc_collab<W, Word>, grid, block, 0, s, a);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }
@@ -505,20 +514,20 @@ int launch_alloc(pbm_pool* p, const pbm_walk_config* c, const AllocArgs& a, bool
     const int grid = serial ? 1 : (int)((a.n + (uint32_t)block - 1u) / (uint32_t)block);
     switch (c->strategy) {
     case PBM_RANDOM_WALK:
-        k_alloc_thread<Walk::Page><<<grid, block, 0, s>>>(a);
+        launch_next(k_alloc_thread<Walk::Page>, grid, block, 0, s, a);
         break;
     case PBM_RANDOM_WALK_BM:
-        if (w64) k_alloc_thread<Walk::Word64><<<grid, block, 0, s>>>(a);
-        else k_alloc_thread<Walk::Word32><<<grid, block, 0, s>>>(a);
+        if (w64) launch_next(k_alloc_thread<Walk::Word64>, grid, block, 0, s, a);
+        else launch_next(k_alloc_thread<Walk::Word32>, grid, block, 0, s, a);
         break;
     case PBM_CLUSTERED_RW_BM:
-        k_alloc_thread<Walk::Crw><<<grid, block, 0, s>>>(a);
+        launch_next(k_alloc_thread<Walk::Crw>, grid, block, 0, s, a);
         break;
     case PBM_SINGLE_CLOCK:
-        k_alloc_thread<Walk::SingleClock><<<grid, block, 0, s>>>(a);
+        launch_next(k_alloc_thread<Walk::SingleClock>, grid, block, 0, s, a);
         break;
     case PBM_DIST_CLOCK:
-        k_alloc_thread<Walk::DistClock><<<grid, block, 0, s>>>(a);
+        launch_next(k_alloc_thread<Walk::DistClock>, grid, block, 0, s, a);
         break;
     case PBM_COLLAB_RW_BM: {
         int cb = serial ? W : block_cfg;
@@ -533,9 +542,9 @@ int launch_alloc(pbm_pool* p, const pbm_walk_config* c, const AllocArgs& a, bool
             if (rc) return rc;
         }
         if (serial || a.n < (uint32_t)(sm_count() * block * kFifoItems))
-            k_fifo_alloc<1><<<grid, block, 0, s>>>(a, p->d_fifo, p->d_ring);
+            launch_next(k_fifo_alloc<1>, grid, block, 0, s, a, p->d_fifo, p->d_ring);
         else
-            k_fifo_alloc<kFifoItems><<<(grid + kFifoItems - 1) / kFifoItems, block, 0, s>>>(a, p->d_fifo, p->d_ring);
+            launch_next(k_fifo_alloc<kFifoItems>, (grid + kFifoItems - 1) / kFifoItems, block, 0, s, a, p->d_fifo, p->d_ring);
         break;
     }
     default:
@@ -594,17 +603,15 @@ int pbm_free(pbm_pool* pool, const pbm_walk_config* cfg, uint32_t n, const int32
             if (rc) return rc;
         }
         if (n < (uint32_t)(sm_count() * block * kFifoItems))
-            k_fifo_free<1><<<grid, block, 0, s>>>(pool->view, n, d_ids, pool->d_fifo, pool->d_ring, pool->d_stats);
+            launch_next(k_fifo_free<1>, grid, block, 0, s, pool->view, n, d_ids, pool->d_fifo, pool->d_ring, pool->d_stats);
         else
-            k_fifo_free<kFifoItems><<<(grid + kFifoItems - 1) / kFifoItems, block, 0, s>>>(
-                pool->view, n, d_ids, pool->d_fifo, pool->d_ring, pool->d_stats);
+            launch_next(k_fifo_free<kFifoItems>, (grid + kFifoItems - 1) / kFifoItems, block, 0, s, pool->view, n, d_ids, pool->d_fifo, pool->d_ring, pool->d_stats);
     } else {
         pool->fifo_valid = false;
         if (cfg->free_merge && block >= 32) {
-            k_free_pages<true><<<grid, block, 0, s>>>(pool->view, n, d_ids, pool->d_stats);
+            launch_next(k_free_pages<true>, grid, block, 0, s, pool->view, n, d_ids, pool->d_stats);
         } else {
-            k_free_pages<false><<<capped_grid(((uint64_t)n + 3u) / 4u, block), block, 0, s>>>(pool->view, n, d_ids,
-                                                                                    pool->d_stats);
+            launch_next(k_free_pages<false>, capped_grid(((uint64_t)n + 3u) / 4u, block), block, 0, s, pool->view, n, d_ids, pool->d_stats);
         }
     }
     PBM_LAUNCH_CHECK();
@@ -622,8 +629,8 @@ static int alloc_runs_impl(pbm_pool* pool, uint32_t n, const int32_t* d_npages, 
     AllocArgs a = make_args(pool, &c, n, seed, d_ids, d_steps);
     int block = serial ? 1 : kDefaultBlock;
     int grid = serial ? 1 : (int)((n + (uint32_t)block - 1u) / (uint32_t)block);
-    if (span) k_alloc_runs<true><<<grid, block, 0, (cudaStream_t)stream>>>(a, d_npages);
-    else k_alloc_runs<false><<<grid, block, 0, (cudaStream_t)stream>>>(a, d_npages);
+    if (span) launch_next(k_alloc_runs<true>, grid, block, 0, (cudaStream_t)stream, a, d_npages);
+    else launch_next(k_alloc_runs<false>, grid, block, 0, (cudaStream_t)stream, a, d_npages);
     PBM_LAUNCH_CHECK();
     pool->fifo_valid = false;
     return PBM_OK;
@@ -658,7 +665,7 @@ int pbm_free_runs(pbm_pool* pool, uint32_t n, const int32_t* d_ids, const int32_
     if (!pool || (n && (!d_ids || !d_npages))) return PBM_ERR_INVALID;
     if (n == 0) return PBM_OK;
     int grid = (int)((n + 255u) / 256u);
-    k_free_runs<<<grid, 256, 0, (cudaStream_t)stream>>>(pool->view, n, d_ids, d_npages, pool->d_stats);
+    launch_next(k_free_runs, grid, 256, 0, (cudaStream_t)stream, pool->view, n, d_ids, d_npages, pool->d_stats);
     PBM_LAUNCH_CHECK();
     pool->fifo_valid = false;
     return PBM_OK;
@@ -678,7 +685,7 @@ int pbm_claim_write_free(pbm_pool* pool, uint32_t n, uint32_t seed, uint32_t pay
     // 64-thread blocks, so its walks spread over every SM
     const int block = n < (uint32_t)sm_count() * 512u ? 64 : 256;
     int grid = (int)((n + (uint32_t)block - 1u) / (uint32_t)block);
-    k_claim_write_free<<<grid, block, 0, (cudaStream_t)stream>>>(a, payload_bytes / 4u, hold);
+    launch_next(k_claim_write_free, grid, block, 0, (cudaStream_t)stream, a, payload_bytes / 4u, hold);
     PBM_LAUNCH_CHECK();
     pool->fifo_valid = false;
     return PBM_OK;
@@ -691,8 +698,7 @@ int pbm_gather_pages(pbm_pool* pool, const int32_t* d_ids, uint32_t n, uint32_t 
         (bytes_per_page & 3u) || bytes_per_page == 0)
         return PBM_ERR_INVALID;
     if (n == 0) return PBM_OK;
-    k_gather_pages<<<sm_count() * 4, 256, 0, (cudaStream_t)stream>>>(pool->view, d_ids, n, bytes_per_page / 4u,
-                                                                     d_out);
+    launch_next(k_gather_pages, sm_count() * 4, 256, 0, (cudaStream_t)stream, pool->view, d_ids, n, bytes_per_page / 4u, d_out);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }

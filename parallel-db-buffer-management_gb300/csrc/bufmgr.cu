@@ -694,6 +694,7 @@ constexpr int kReleaseItems = 2;   // per thread, their reads in flight together
 template <bool BYPAGE>
 __global__ void __launch_bounds__(256) k_release(BmView b, const int32_t* release_of, const int32_t* release_idx,
                                                  uint32_t n_release) {
+    stream_wait();
     constexpr uint32_t KEYS = 256u * kReleaseItems;
     __shared__ uint32_t keys[2 * KEYS], cnt[2 * KEYS];
     unsigned long long ok = 0, bad = 0;
@@ -745,6 +746,7 @@ template <bool DIST, bool BYPAGE, bool COPY, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_round(BmView b, const int32_t* release_of, const int32_t* release_idx,
                                                uint32_t n_release, const int32_t* pages, uint32_t n, uint32_t slot0,
                                                int32_t* frames_out, int32_t* held_out) {
+    stream_wait();
     unsigned long long ok = 0, bad = 0;
     BmAcc acc;
     if ((uint64_t)gridDim.x * blockDim.x == 1u) {
@@ -817,6 +819,7 @@ __global__ void k_bm_check(BmView b, BmCheck* out) {
 }
 
 __global__ void k_bm_gather(BmView b, const int32_t* ids, uint32_t n, uint32_t words_per_frame, int32_t* out) {
+    stream_wait();
     const unsigned long long total = (unsigned long long)n * words_per_frame;
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (unsigned long long)gridDim.x * blockDim.x) {
@@ -922,9 +925,9 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     if (n == 0 && !serial) {   // releases only: no fetch, no sweep
         const int rgrid = (int)(((uint64_t)n_release + 256u * kReleaseItems - 1u) / (256u * kReleaseItems));
         if (by_page)
-            k_release<true><<<rgrid, 256, 0, s>>>(m->v, d_release_of, d_release_idx, n_release);
+            launch_next(k_release<true>, rgrid, 256, 0, s, m->v, d_release_of, d_release_idx, n_release);
         else
-            k_release<false><<<rgrid, 256, 0, s>>>(m->v, d_release_of, d_release_idx, n_release);
+            launch_next(k_release<false>, rgrid, 256, 0, s, m->v, d_release_of, d_release_idx, n_release);
         PBM_LAUNCH_CHECK();
         return PBM_OK;
     }
@@ -941,8 +944,7 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     auto go = [&](auto kernel) {
         if (stage) attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)kCopyStage);
         if (attr == cudaSuccess)
-            kernel<<<grid, block, stage, s>>>(m->v, d_release_of, d_release_idx, n_release, d_pages, n, slot0, d_frames_out,
-                                              d_held_out);
+            launch_next(kernel, grid, block, stage, s, m->v, d_release_of, d_release_idx, n_release, d_pages, n, slot0, d_frames_out, d_held_out);
     };
     if (copy) {
         if (m->v.dist)
@@ -1025,8 +1027,7 @@ int pbm_bufmgr_gather(pbm_bufmgr* m, const int32_t* d_frame_ids, uint32_t n, uin
         return PBM_ERR_INVALID;
     pbm::DeviceScope scope(m->device);
     if (n == 0) return PBM_OK;
-    k_bm_gather<<<sm_count() * 4, 256, 0, (cudaStream_t)stream>>>(m->v, d_frame_ids, n, bytes_per_frame / 4u,
-                                                                  d_out);
+    launch_next(k_bm_gather, sm_count() * 4, 256, 0, (cudaStream_t)stream, m->v, d_frame_ids, n, bytes_per_frame / 4u, d_out);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }

@@ -60,6 +60,36 @@ __device__ __forceinline__ void block_add_counters(const unsigned long long (&v)
         if (x) atomicAdd(dst[threadIdx.x], x);
     }
 }
+// Programmatic dependent launch.  A kernel launched with launch_next may be set up and
+// get its blocks onto the SMs while the kernel before it in the stream still runs;
+// it calls stream_wait() before its first access to global memory, which returns once
+// that kernel has ended and its writes are visible (at once after an ordinary
+// predecessor), and then lets the kernel after it do the same.  Most calls here are
+// kernels of 3-20 us launched one after another, and the start of a launch is 2-3 us of
+// each.  Measured on GB300, a call and the calls after it in a stream: 32 claims + frees
+// 8.2 -> 6.3 us; claim, read and free of 16,384 pages 18.5 -> 12.7; eight
+// buffer-manager rounds of 131,072 fetches 157 -> 136; with 4 KiB copies 205 -> 168.
+__device__ __forceinline__ void stream_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                               A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Makes a device current for the rest of the calling scope and restores the
 // caller's device when the scope ends.  Every entry point that takes a pool
 // (or an object built on one) opens one with the pool's device, so a process
