@@ -27,7 +27,6 @@ struct AllocArgs {
     uint32_t max_slots;
     int32_t dedupe;              // collaborative walk: W*stride may exceed L
     LaunchBudget* budget;        // fail-fast launch budget (null: every request walks)
-    const int32_t* free_list;    // the budget's list of free pages (list mode)
 };
 
 // Per-thread accumulators reduced once per block.
@@ -37,6 +36,29 @@ struct Acc {
 
 __device__ __forceinline__ void flush_acc(const Acc& a, DevStats* st) {
     block_add_counters<3>({a.ok, a.fail, a.steps}, {&st->successes, &st->failures, &st->steps});
+}
+
+// A launch whose budget pass served the requests in order (list mode) has only the
+// refused ones left: ids -1, no steps.  Returns true when that is all; false when some
+// requests lost their page meanwhile and walk (or the pass served none).
+__device__ __forceinline__ bool finish_listed(const AllocArgs& a, Acc& acc) {
+    if (!a.budget || !__ldcg(&a.budget->list_mode) || __ldcg(&a.budget->lost)) return false;
+    // the first kFinishBlocks blocks do it: each block that counts something ends in an atomic at one address
+    constexpr uint32_t kFinishBlocks = 1024;
+    const uint64_t nthr = (uint64_t)min(gridDim.x, kFinishBlocks) * blockDim.x;
+    if (blockIdx.x >= kFinishBlocks) return true;
+    for (uint64_t r = (uint64_t)__ldcg(&a.budget->free_at_start) + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < a.n;
+         r += nthr) {
+        a.ids[r] = -1;
+        if (a.steps) a.steps[r] = 0;
+        ++acc.fail;
+    }
+    return true;
+}
+
+// Whether request r walks: granted by the budget and not served by its pass.
+__device__ __forceinline__ bool must_walk(const AllocArgs& a, bool listed, uint64_t r) {
+    return r < a.n && budget_grants(a.budget, r) && (!listed || a.ids[r] == kLostPage);
 }
 
 enum class Walk { Page, Word32, Word64, Crw, SingleClock, DistClock };
@@ -52,33 +74,17 @@ __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 6 : 8) k_alloc_t
     const uint64_t n_round = ((uint64_t)a.n + 31u) & ~31ull;
     // whole warps iterate together (n_round and nthr are multiples of 32), or
     // one thread in the serial replay
+    const bool done = finish_listed(a, acc);
     const bool listed = a.budget && __ldcg(&a.budget->list_mode);
-    for (uint64_t r = tid; r < n_round; r += nthr) {
-        const bool go = r < a.n && budget_grants(a.budget, r);
+    for (uint64_t r = tid; r < n_round && !done; r += nthr) {
+        const bool go = must_walk(a, listed, r);
         int32_t s = 0, id = -1;
-        if (go && listed) {
-            id = take_listed(a.v, a.free_list, (long long)r);   // request r takes the r-th free page
-            s = 1;
-        }
         if (K == Walk::Page && blockDim.x >= 32u) {
-            int32_t ws = 0;
-            const int32_t wid = walk_page_warp(a.v, go && id < 0, request_seed(a.seed, (uint32_t)r), a.max_steps, &ws);
-            if (go && id < 0) {
-                id = wid;
-                s = ws;
-            }
+            id = walk_page_warp(a.v, go, request_seed(a.seed, (uint32_t)r), a.max_steps, &s);
         } else if (K == Walk::SingleClock && blockDim.x >= 32u) {
-            int32_t ws = 0;
-            const int32_t wid = sweep_single_warp(a.v, a.arm, go && id < 0, request_seed(a.seed, (uint32_t)r),
-                                                  a.max_steps, gridDim.x == 1u, &ws);
-            if (go && id < 0) {
-                id = wid;
-                s = ws;
-            }
-        } else if (r >= a.n || id >= 0) {
-            // past the last request, or served from the list
+            id = sweep_single_warp(a.v, a.arm, go, request_seed(a.seed, (uint32_t)r), a.max_steps, gridDim.x == 1u, &s);
         } else if (!go) {
-            // past the launch budget: no free page is left for this request
+            // past the last request, or past the launch budget: no free page is left for this request
         } else if constexpr (K == Walk::Page) {
             const int32_t seed0 = request_seed(a.seed, r);
             id = walk_page(a.v, seed0, a.max_steps, &s);
@@ -102,7 +108,7 @@ __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 6 : 8) k_alloc_t
             id = sweep_dist(a.v, &ar, a.max_steps, &s);
             *arm = ar;
         }
-        if (r >= a.n) continue;
+        if (r >= a.n || (listed && !go && budget_grants(a.budget, r))) continue;   // served by the budget pass
         a.ids[r] = id;
         if (a.steps) a.steps[r] = s;
         acc.ok += id >= 0;
@@ -126,20 +132,16 @@ __global__ void __launch_bounds__(256) k_alloc_collab(AllocArgs a) {
     const uint32_t L = WordTraits<Word>::count(a.v);
     const uint32_t lane_off = (uint32_t)(((unsigned long long)gl * a.stride) % L);
     volatile int32_t* my_slots = slots + (threadIdx.x & ~(uint32_t)(W - 1));
+    const bool done = finish_listed(a, acc);
     const bool listed = a.budget && __ldcg(&a.budget->list_mode);
     // trip count uniform across each group of W lanes
-    for (uint64_t base = tid - gl; base < a.n; base += nthr) {
+    for (uint64_t base = tid - gl; base < a.n && !done; base += nthr) {
         const uint64_t r = base + gl;
-        const bool need = r < a.n && budget_grants(a.budget, r);
-        const int32_t from_list = (need && listed) ? take_listed(a.v, a.free_list, (long long)r) : -1;
+        const bool need = must_walk(a, listed, r);
         int32_t s = 0;
-        int32_t id = walk_collab<W, Word>(a.v, need && from_list < 0, request_seed(a.seed, base), lane_off,
-                                          a.dedupe != 0, a.max_steps, my_slots, &s);
-        if (from_list >= 0) {
-            id = from_list;
-            s = 1;
-        }
-        if (r < a.n) {
+        const int32_t id = walk_collab<W, Word>(a.v, need, request_seed(a.seed, base), lane_off, a.dedupe != 0, a.max_steps,
+                                                my_slots, &s);
+        if (r < a.n && (need || !listed || !budget_grants(a.budget, r))) {   // else served by the budget pass
             a.ids[r] = id;
             if (a.steps) a.steps[r] = need ? s : 0;   // refused by the budget: no walk
             acc.ok += id >= 0;
@@ -494,7 +496,6 @@ AllocArgs make_args(pbm_pool* p, const pbm_walk_config* c, uint32_t n, uint32_t 
     uint32_t L = c->word_bits == 64 ? p->view.n_words64 : p->view.n_words32;
     a.dedupe = ((unsigned long long)(W - 1) * a.stride >= L) ? 1 : 0;
     a.budget = nullptr;
-    a.free_list = nullptr;
     return a;
 }
 
@@ -568,10 +569,9 @@ int pbm_alloc(pbm_pool* pool, const pbm_walk_config* cfg, uint32_t n, uint32_t s
     AllocArgs a = make_args(pool, cfg, n, seed, d_ids, d_steps);
     if (cfg->strategy != PBM_LINKED_LIST) pool->fifo_valid = false;
     if (cfg->fail_fast && cfg->strategy != PBM_LINKED_LIST) {   // the free list counts its pages itself
-        rc = budget_prepare(pool, n, (cudaStream_t)stream);
+        rc = budget_prepare(pool, n, d_ids, d_steps, (cudaStream_t)stream);
         if (rc) return rc;
         a.budget = pool->d_budget;
-        a.free_list = pool->d_free_list;
     }
     return launch_alloc(pool, cfg, a, false, (cudaStream_t)stream);
 }

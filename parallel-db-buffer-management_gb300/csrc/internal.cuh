@@ -136,8 +136,7 @@ struct pbm_pool {
     unsigned long long* d_scan;     // scratch for prefix sums (per-block partials)
     unsigned long long* d_prefix;   // batch prefix (n_groups + 1)
     pbm::LaunchBudget* d_budget;    // fail-fast launch budget: free pages at launch start
-    int32_t* d_free_list;           // the budget pass's list of free pages (list mode)
-    uint64_t free_list_cap;
+    uint64_t list_cap;              // free pages up to which the budget pass may hand them out itself
     unsigned long long* d_budget_blocks;   // free pages per block slice of the budget pass
     uint32_t budget_blocks;
     uint32_t prefix_cap;
@@ -173,7 +172,7 @@ namespace pbm {
 int fifo_build(pbm_pool* pool, cudaStream_t s);
 int popcount_used(pbm_pool* pool, uint64_t* used, cudaStream_t s);
 // Counts the pool's free pages into pool->d_budget on stream s (no sync); a
-// launch of n_requests that asks for at least half of them also gets them
-// listed in order in pool->d_free_list (list mode, when they fit).
-int budget_prepare(pbm_pool* pool, uint64_t n_requests, cudaStream_t s);
+// launch of n_requests that asks for at least half of them is served in order by
+// the same pass (list mode).
+int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s);
 }  // namespace pbm

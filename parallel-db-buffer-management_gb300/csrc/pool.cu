@@ -247,9 +247,10 @@ int fifo_build(pbm_pool* pool, cudaStream_t s) {
 
 // ---- fail-fast launch budget ----
 // Pass 1: the free pages (clear bits; padding bits stay set) of each block's
-// contiguous slice of `per` 64-bit words, into counts[block] and the totals.
-__global__ void k_free_budget(const unsigned long long* words, uint32_t n_words64, uint32_t per,
-                              unsigned long long* counts, LaunchBudget* b) {
+// contiguous slice of `per` 64-bit words, into counts[block].
+__global__ void __launch_bounds__(256) k_free_budget(const unsigned long long* words, uint32_t n_words64, uint32_t per,
+                                                     unsigned long long* counts, LaunchBudget* b) {
+    stream_wait();
     const uint64_t w0 = (uint64_t)blockIdx.x * per;
     const uint64_t w1 = min((uint64_t)n_words64, w0 + per);
     unsigned long long c = 0;
@@ -258,72 +259,126 @@ __global__ void k_free_budget(const unsigned long long* words, uint32_t n_words6
     c = block_sum(c);
     if (threadIdx.x == 0) {
         counts[blockIdx.x] = c;
-        if (c) atomicAdd(reinterpret_cast<unsigned long long*>(&b->free_at_start), c);
+        if (blockIdx.x == 0) b->lost = 0u;
     }
 }
 
-// Pass 2: when the launch asks for at least half of the F free pages and the
-// list holds them, every block writes its slice's free pages in ascending
-// order at its offset (the counts of the blocks before it); list_mode says
-// whether the list is valid for this launch.
-__global__ void k_free_list(const unsigned long long* words, uint32_t n_words64, uint32_t per,
-                            const unsigned long long* counts, LaunchBudget* b, unsigned long long n_requests,
-                            int32_t* list, unsigned long long cap) {
-    __shared__ unsigned long long warp_tot[32];
-    __shared__ unsigned long long s_base;
-    const long long F = b->free_at_start;
-    const bool mode = F > 0 && 2ull * n_requests >= (unsigned long long)F && (unsigned long long)F <= cap;
-    if (blockIdx.x == 0 && threadIdx.x == 0) b->list_mode = mode ? 1 : 0;
-    if (!mode) return;
-    unsigned long long off = 0;
-    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) off += counts[k];
+// Pass 2: F, the sum of the counts, and, when the launch asks for at least half of
+// the F free pages (and F is at most `cap`), the pages themselves: request r takes
+// the r-th free page in ascending order.  Each block claims its slice's
+// pages word by word with one atomicOr and writes their ids to the requests that
+// start at its offset (the counts of the blocks before it); the ids of a warp's 32 words
+// go through shared memory so that they leave as whole lines.  A slice gives exactly
+// the pages counted in it: pages another stream took since then leave their
+// requests kLostPage, which the launch's kernel serves by walking.  Writing
+// a list of pages here and taking each page of it with an atomic of its own in that kernel
+// moved 8 more bytes per page and took an atomic per page instead of per
+// word.  Measured on GB300, 2^22 requests on 2^24 pages at 90% (1.68 M granted) and
+// their frees: 63 -> 37 us.
+__global__ void __launch_bounds__(256) k_take_free(unsigned long long* words, uint32_t n_words64, uint32_t per,
+                                                   const unsigned long long* counts, LaunchBudget* b, uint32_t n_requests,
+                                                   unsigned long long cap, int32_t* ids, int32_t* steps, DevStats* stats) {
+    __shared__ uint32_t warp_tot[8];
+    __shared__ unsigned long long s_sum[2];
+    __shared__ uint16_t stage[8][2048];        // per warp: page offsets within its 32 words
+    stream_wait();
+    unsigned long long off = 0, F = 0;
+    for (uint32_t k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
+        const unsigned long long c = __ldcg(counts + k);
+        F += c;
+        if (k < blockIdx.x) off += c;
+    }
+    F = block_sum(F);
     off = block_sum(off);
-    if (threadIdx.x == 0) s_base = off;
+    if (threadIdx.x == 0) {
+        s_sum[0] = F;
+        s_sum[1] = off;
+    }
     __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    F = s_sum[0];
+    off = s_sum[1];
+    const bool mode = F > 0ull && 2ull * n_requests >= F && F <= cap;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        b->free_at_start = (long long)F;
+        b->list_mode = mode ? 1 : 0;
+    }
+    if (!mode || off >= n_requests) return;
+    // this slice's requests: off .. off + quota - 1
+    const uint32_t quota = (uint32_t)min(__ldcg(counts + blockIdx.x), (unsigned long long)n_requests - off);
+    int32_t* out = ids + off;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint64_t w0 = (uint64_t)blockIdx.x * per;
     const uint64_t w1 = min((uint64_t)n_words64, w0 + per);
-    for (uint64_t base = w0; base < w1; base += blockDim.x) {
+    uint32_t done = 0, lost = 0;               // requests behind this chunk (block-uniform); lost: this thread's
+    for (uint64_t base = w0; base < w1 && done < quota; base += 256u) {
         const uint64_t w = base + threadIdx.x;
-        unsigned long long fr = w < w1 ? ~__ldcg(words + w) : 0ull;
+        const uint64_t fr = w < w1 ? ~(uint64_t)__ldcg(words + w) : 0ull;
         const int c = __popcll(fr);
         int incl = c;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += y;
+            const int y = __shfl_up_sync(kFull32, incl, d);
+            if ((int)lane >= d) incl += y;
         }
-        if (lane == 31) warp_tot[warp] = (unsigned long long)incl;
+        if (lane == 31u) warp_tot[warp] = (uint32_t)incl;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long acc = 0;
-            for (int i = 0; i < nwarps; ++i) { const unsigned long long t = warp_tot[i]; warp_tot[i] = acc; acc += t; }
-            warp_tot[31] = acc;   // (nwarps <= 8 here, so slot 31 is free) the chunk's total
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 8u; ++i) {
+            const uint32_t x = warp_tot[i];
+            if (i < warp) before += x;
+            total += x;
         }
-        __syncthreads();
-        unsigned long long pos = s_base + warp_tot[warp] + (unsigned long long)(incl - c);
-        while (fr) {
-            const int bit = __ffsll((long long)fr) - 1;
-            fr &= fr - 1ull;
-            list[pos++] = (int32_t)(w * 64u + (uint64_t)bit);
+        const uint32_t wpos = done + before;                       // the warp's first request
+        const uint32_t wlim = wpos < quota ? min(quota - wpos, warp_tot[warp]) : 0u;   // and how many it has
+        const uint32_t excl = (uint32_t)(incl - c);
+        uint64_t take = excl < wlim ? low_bits(fr, (int)(wlim - excl)) : 0ull;
+        uint64_t gone = 0ull;
+        if (take) gone = take & (uint64_t)atomicOr(words + w, (unsigned long long)take);
+        uint32_t pos = excl;
+        for (uint64_t m = take; m; m &= m - 1ull) {
+            const uint32_t bit = (uint32_t)__ffsll((long long)m) - 1u;
+            const bool missed = (gone >> bit) & 1ull;
+            stage[warp][pos++] = missed ? 0xffffu : (uint16_t)(lane * 64u + bit);
+            lost += missed;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) s_base += warp_tot[31];
-        __syncthreads();
+        __syncwarp();
+        const uint32_t page0 = (uint32_t)(base + warp * 32u) * 64u;
+        for (uint32_t i = lane; i < wlim; i += 32u) {
+            const uint32_t o = stage[warp][i];
+            out[wpos + i] = o == 0xffffu ? kLostPage : (int32_t)(page0 + o);
+            if (steps) steps[off + wpos + i] = 1;
+        }
+        done += total;
+        __syncthreads();   // warp_tot and the stage are used again
+    }
+    // pages counted here but gone before they were read
+    uint32_t missing = 0;
+    for (uint32_t i = done + threadIdx.x; i < quota; i += 256u) {
+        out[i] = kLostPage;
+        ++missing;
+    }
+    lost += missing;
+    const unsigned long long all_lost = block_sum(lost);
+    if (threadIdx.x == 0) {
+        if (all_lost) atomicAdd(&b->lost, (uint32_t)all_lost);
+        const unsigned long long got = quota - all_lost;
+        if (got) {
+            atomicAdd(&stats->successes, got);
+            atomicAdd(&stats->steps, got);
+        }
     }
 }
 
-int budget_prepare(pbm_pool* pool, uint64_t n_requests, cudaStream_t s) {
-    PBM_CUDA_TRY(cudaMemsetAsync(pool->d_budget, 0, sizeof(LaunchBudget), s));
+int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s) {
     const uint32_t nw64 = (uint32_t)(pool->bitmap_bytes / 8u);
     const uint32_t nb = pool->budget_blocks;
     const uint32_t per = (nw64 + nb - 1u) / nb;
-    k_free_budget<<<nb, 256, 0, s>>>(reinterpret_cast<const unsigned long long*>(pool->d_words), nw64, per,
-                                     pool->d_budget_blocks, pool->d_budget);
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(pool->d_words);
+    launch_next(k_free_budget, nb, 256, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget);
     PBM_LAUNCH_CHECK();
-    k_free_list<<<nb, 256, 0, s>>>(reinterpret_cast<const unsigned long long*>(pool->d_words), nw64, per,
-                                   pool->d_budget_blocks, pool->d_budget, (unsigned long long)n_requests,
-                                   pool->d_free_list, (unsigned long long)pool->free_list_cap);
+    launch_next(k_take_free, nb, 256, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget, n_requests,
+                pool->list_cap, d_ids, d_steps, pool->d_stats);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }
@@ -359,7 +414,6 @@ static void pool_free_all(pbm_pool* p) {
     cudaFree(p->d_seen);
     cudaFree(p->d_check);
     cudaFree(p->d_budget);
-    cudaFree(p->d_free_list);
     cudaFree(p->d_budget_blocks);
     cudaFree(p->d_scan);
     cudaFree(p->d_prefix);
@@ -417,10 +471,10 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
     p->view.page_size = cfg->page_size;
     const uint32_t nb_scan = (uint32_t)((p->view.n_words32 + 4095u) / 4096u) + 1u;
     p->prefix_cap = 0;
-    // the budget pass: one block per 256 64-bit words, at most 4 per SM; its
-    // free list covers launches into a pool at least half full
+    // the budget pass: one block per 256 64-bit words, at most 4 per SM; it hands
+    // pages out itself in a pool at least half full
     p->budget_blocks = (uint32_t)std::min<uint64_t>((uint64_t)sm_count() * 4u, std::max<uint64_t>(1u, (nw64 + 255u) / 256u));
-    p->free_list_cap = std::max<uint64_t>(1024u, cfg->n_pages / 2u);
+    p->list_cap = std::max<uint64_t>(1024u, cfg->n_pages / 2u);
     bool ok = cudaMalloc(&p->d_words, p->bitmap_bytes) == cudaSuccess &&
               cudaMalloc(&p->d_stats, sizeof(DevStats)) == cudaSuccess &&
               cudaMalloc(&p->d_cursors, sizeof(int32_t) * p->max_slots) == cudaSuccess &&
@@ -430,7 +484,6 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
               cudaMalloc(&p->d_seen, p->bitmap_bytes) == cudaSuccess &&
               cudaMalloc(&p->d_check, sizeof(CheckCounters)) == cudaSuccess &&
               cudaMalloc(&p->d_budget, sizeof(LaunchBudget)) == cudaSuccess &&
-              cudaMalloc(&p->d_free_list, sizeof(int32_t) * p->free_list_cap) == cudaSuccess &&
               cudaMalloc(&p->d_budget_blocks, sizeof(unsigned long long) * p->budget_blocks) == cudaSuccess &&
               cudaMalloc(&p->d_scan, sizeof(unsigned long long) * nb_scan) == cudaSuccess;
     if (ok && (cfg->flags & PBM_POOL_MATERIALIZE)) {

@@ -200,3 +200,65 @@ def test_clock_sweep_of_many_warps(cuda, pbm_mod, orc, T, occ, n, max_steps):
     pool.free(pbm.walk_config(pbm.SINGLE_CLOCK), n, ids)
     assert np.array_equal(pool.read_bitmap(), before)
     pool.close()
+
+
+@pytest.mark.parametrize("strategy", [0, 1, 2, 3, 5, 6])
+@pytest.mark.parametrize("T,occ", [(64, 0.5), (2000, 0.7), (65536 + 17, 0.9), (1 << 20, 0.6), (3000001, 0.95)])
+def test_budget_pass_hands_the_free_pages_out_in_order(cuda, pbm_mod, orc, strategy, T, occ):
+    """A launch that asks for at least half of the F free pages: request r gets the r-th free page, the
+    requests past F are refused, and the counters say so; one that asks for fewer walks as without a budget."""
+    torch, pbm = cuda, pbm_mod
+    words = orc.bernoulli_bitmap(T, occ, 6)
+    bits = np.unpackbits(words.view(np.uint8), bitorder="little")[:T]
+    free = np.nonzero(bits == 0)[0]
+    F = len(free)
+    pool = pbm.Pool(T, 64)
+    cfg = pbm.walk_config(strategy, fail_fast=1)
+    for n in sorted({(F + 1) // 2, F - 1, F, F + 1, F + 70, 3 * F}):
+        if n < 1:
+            continue
+        pool.reset()
+        pool.prefill(occ, 6)
+        ids = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        steps = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        pool.alloc(cfg, n, 3, ids, steps)
+        k = min(n, F)
+        got, st = ids.cpu().numpy(), steps.cpu().numpy()
+        assert np.array_equal(got[:k], free[:k]) and (got[k:] == -1).all()
+        assert (st[:k] == 1).all() and (st[k:] == 0).all()
+        after = bits.copy()
+        after[free[:k]] = 1
+        assert np.array_equal(np.unpackbits(pool.read_bitmap().view(np.uint8), bitorder="little")[:T], after)
+        s = pool.stats()
+        assert (s.successes, s.failures, s.steps) == (k, n - k, k)
+    pool.close()
+
+
+def test_budget_pass_beside_another_stream(cuda, pbm_mod, orc):
+    """While the pass hands pages out, another stream takes and frees pages of the same pool: no page goes
+    to two holders, and the bitmap holds exactly the prefill and what both hold."""
+    torch, pbm = cuda, pbm_mod
+    T = 1 << 22
+    pool = pbm.Pool(T, 64)
+    pool.prefill(0.9, 2)
+    base = pool.used()
+    n, m = 150000, 40000
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    a = torch.empty(T // 8, dtype=torch.int32, device="cuda")
+    b = torch.empty(m, dtype=torch.int32, device="cuda")
+    cfg, ff = pbm.walk_config(pbm.RANDOM_WALK_BM), pbm.walk_config(pbm.COLLAB_RW_BM, fail_fast=1, max_steps=256)
+    torch.cuda.synchronize()
+    for k in range(20):
+        for j in range(3):
+            pool.alloc(cfg, m, 100 * k + j, b, stream=s2.cuda_stream)
+            if j < 2:
+                pool.free(cfg, m, b, stream=s2.cuda_stream)
+        pool.alloc(ff, a.numel(), k, a, stream=s1.cuda_stream)
+        torch.cuda.synchronize()
+        both = torch.cat([a, b])
+        chk = pool.check(both, both.numel())
+        assert (chk.n_duplicates, chk.n_not_marked, chk.n_out_of_range) == (0, 0, 0)
+        assert chk.used_pages == base + chk.n_ok
+        pool.free(cfg, both.numel(), both)
+        assert pool.used() == base
+    pool.close()
