@@ -434,20 +434,6 @@ __global__ void __launch_bounds__(256) k_claim_write_free(AllocArgs a, uint32_t 
                           {&a.stats->successes, &a.stats->failures, &a.stats->steps, &a.stats->frees});
 }
 
-__global__ void k_gather_pages(PoolView v, const int32_t* ids, uint32_t n, uint32_t words_per_page,
-                               int32_t* out) {
-    stream_wait();
-    const unsigned long long total = (unsigned long long)n * words_per_page;
-    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
-        uint32_t r = (uint32_t)(i / words_per_page), k = (uint32_t)(i % words_per_page);
-        int32_t id = ids[r];
-        out[i] = (id >= 0 && (uint32_t)id < v.n_pages)
-                     ? reinterpret_cast<const int32_t*>(v.base + (size_t)(uint32_t)id * v.page_size)[k]
-                     : 0;
-    }
-}
-
 }  // namespace pbm
 
 using namespace pbm;
@@ -698,7 +684,7 @@ int pbm_gather_pages(pbm_pool* pool, const int32_t* d_ids, uint32_t n, uint32_t 
         (bytes_per_page & 3u) || bytes_per_page == 0)
         return PBM_ERR_INVALID;
     if (n == 0) return PBM_OK;
-    launch_next(k_gather_pages, sm_count() * 4, 256, 0, (cudaStream_t)stream, pool->view, d_ids, n, bytes_per_page / 4u, d_out);
+    gather_rows(pool->view.base, pool->page_size, pool->view.n_pages, d_ids, n, bytes_per_page, d_out, (cudaStream_t)stream);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }

@@ -555,6 +555,7 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
                                              unsigned long long& bad, BmAcc& acc) {
     constexpr uint32_t KEYS = 2u * BLOCK;   // BLOCK fetches and BLOCK releases
     __shared__ MergeTables<KEYS, !BYPAGE> t;
+    __shared__ uint32_t s_hand;   // the block's first sweep windows
     const uint32_t lane = threadIdx.x & 31u;
     CopyStage cs{};
     if constexpr (COPY) {
@@ -571,8 +572,7 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
     // block-uniform trip count
     for (uint64_t bbase = (uint64_t)blockIdx.x * blockDim.x; bbase < work; bbase += stride) {
         const uint64_t i = bbase + threadIdx.x;
-        unsigned long long hbase = 0;
-        if (!DIST && lane == 0u) hbase = atomicAdd(b.single_hand, 32ull);   // the first sweep window
+        if (!DIST && threadIdx.x == 0) s_hand = atomicAdd(b.single_hand, (unsigned long long)BLOCK) % b.n_frames;
         const int32_t ri = i < n_release ? __ldg(release_idx + i) : -1;
         const int32_t p = i < n ? __ldg(pages + i) : -1;
         for (uint32_t s = threadIdx.x; s < 2u * KEYS; s += BLOCK) {
@@ -584,12 +584,6 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
                 t.rcnt[s] = 0u;
             }
         }
-        SweepWin w0{};
-        if (!DIST) {
-            hbase = __shfl_sync(0xffffffffu, hbase, 0);
-            w0.f = (uint32_t)((hbase + lane) % b.n_frames);
-            w0.q = __ldcg(b.frame_page + w0.f);
-        }
         const bool valid = p >= 0 && (uint32_t)p < b.n_logical;
         const uint32_t peers = __match_any_sync(0xffffffffu, valid ? (uint32_t)p : 0x80000000u + lane);
         const uint32_t leader = (uint32_t)__ffs((int)peers) - 1u;
@@ -599,6 +593,12 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
         const bool rin = rv >= 0 && (!BYPAGE || (uint32_t)rv < b.n_logical);
         if (BYPAGE && rv >= 0 && !rin && (uint32_t)(__ffs((int)rpeers) - 1) == lane) bad += (uint32_t)__popc(rpeers);
         __syncthreads();   // tables clear
+        SweepWin w0{};
+        if (!DIST) {
+            w0.f = s_hand + threadIdx.x;
+            if (w0.f >= b.n_frames) w0.f = b.n_frames > BLOCK ? w0.f - b.n_frames : w0.f % b.n_frames;
+            w0.q = __ldcg(b.frame_page + w0.f);
+        }
         uint32_t fslot = kMergeEmpty, rslot = kMergeEmpty;
         if (valid && lane == leader) fslot = merge_insert<KEYS>(t.fkey, t.fcnt, (uint32_t)p, (uint32_t)__popc(peers));
         if (rin && (uint32_t)(__ffs((int)rpeers) - 1) == lane)
@@ -818,19 +818,6 @@ __global__ void k_bm_check(BmView b, BmCheck* out) {
     if (pins) atomicAdd(&out->pins, pins);
 }
 
-__global__ void k_bm_gather(BmView b, const int32_t* ids, uint32_t n, uint32_t words_per_frame, int32_t* out) {
-    stream_wait();
-    const unsigned long long total = (unsigned long long)n * words_per_frame;
-    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
-        uint32_t r = (uint32_t)(i / words_per_frame), k = (uint32_t)(i % words_per_frame);
-        int32_t f = ids[r];
-        out[i] = (f >= 0 && (uint32_t)f < b.n_frames)
-                     ? reinterpret_cast<const int32_t*>(b.frames + (size_t)(uint32_t)f * b.frame_size)[k]
-                     : 0;
-    }
-}
-
 }  // namespace
 }  // namespace pbm
 
@@ -1027,7 +1014,7 @@ int pbm_bufmgr_gather(pbm_bufmgr* m, const int32_t* d_frame_ids, uint32_t n, uin
         return PBM_ERR_INVALID;
     pbm::DeviceScope scope(m->device);
     if (n == 0) return PBM_OK;
-    launch_next(k_bm_gather, sm_count() * 4, 256, 0, (cudaStream_t)stream, m->v, d_frame_ids, n, bytes_per_frame / 4u, d_out);
+    gather_rows(m->v.frames, m->v.frame_size, m->v.n_frames, d_frame_ids, n, bytes_per_frame, d_out, (cudaStream_t)stream);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }

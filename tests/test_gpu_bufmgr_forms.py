@@ -85,3 +85,26 @@ def test_release_rounds_move_exactly_the_listed_pins(cuda, pbm_mod, n, by_page):
     c = bm.counters()
     assert (c.unpins, c.bad_unpins) == (n, 1) and not bm.read_tables()[1].any()
     bm.close()
+
+
+@pytest.mark.parametrize("page_size,nbytes", [(4, 4), (16, 16), (64, 60), (96, 96), (100, 96), (4096, 4096), (4096, 16)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gather_copies_rows(cuda, pbm_mod, page_size, nbytes, shift):
+    """Whole and partial rows, 16-byte pieces and 4-byte ones (odd page sizes, an output off a 16-byte
+    boundary), ids that name no page."""
+    torch, pbm = cuda, pbm_mod
+    T, n = 1000, 777
+    pool = pbm.Pool(T, page_size, materialize=True)
+    ids = torch.empty(n, dtype=torch.int32, device="cuda")
+    full = page_size // 4 * 4
+    pool.claim_write_free(n, 3, ids, payload_bytes=full, hold=True)
+    ask = ids.clone()
+    ask[5], ask[6] = -1, T
+    buf = torch.full((n * nbytes // 4 + 8,), -7, dtype=torch.int32, device="cuda")
+    out = buf[shift:shift + n * nbytes // 4]
+    pool.gather_pages(ask, n, nbytes, out)
+    want = torch.arange(n, dtype=torch.int32, device="cuda").repeat_interleave(nbytes // 4).view(n, -1)
+    want[5], want[6] = 0, 0
+    assert torch.equal(out.view(n, -1), want)
+    assert (buf[:shift] == -7).all() and (buf[shift + n * nbytes // 4:] == -7).all()
+    pool.close()
