@@ -18,10 +18,10 @@
 //               sits in pools that blocks which finish their own range early
 //               drain.
 #include <atomic>
-#include <new>
+#include <cstddef>
 #include <cstring>
+#include <new>
 #include <type_traits>
-#include <vector>
 
 #include "batch_common.cuh"
 
@@ -199,23 +199,6 @@ __device__ __forceinline__ S wrap_slot(S slot, S len) {
     return slot;
 }
 
-// Last g in [lo, n_groups) with prefix[g] <= q (prefix[lo] <= q), searched
-// by the whole warp: 32 evenly spaced probes and a ballot narrow the range
-// 32-fold per round (two rounds for 256 groups).
-__device__ __forceinline__ uint32_t find_group_warp(const unsigned long long* prefix, uint32_t n_groups,
-                                                    unsigned long long q, uint32_t lo) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t hi = n_groups;
-    while (hi - lo > 1u) {
-        const uint32_t stride = (hi - lo + 31u) >> 5;
-        const uint32_t idx = lo + lane * stride;
-        const uint32_t b = __ballot_sync(0xffffffffu, idx < hi && prefix[idx] <= q);
-        lo += (31u - (uint32_t)__clz((int)b)) * stride;
-        hi = min(hi, lo + stride);
-    }
-    return lo;
-}
-
 // The persistent batch kernel.  With a.fuse each block scans the step's
 // group counts into shared memory itself (no separate prefix kernel); the
 // graph form's step comes with the launch's parameters (no counter to read,
@@ -231,6 +214,7 @@ __device__ __forceinline__ uint32_t find_group_warp(const unsigned long long* pr
 // measured slower: the extra instructions cost more than the latency they hid.)
 template <BWalk K, int W, typename Word, int MINB, typename Tab, typename SlotT>
 __global__ void __launch_bounds__(256, MINB) k_batch_persistent(BatchArgs a, const __grid_constant__ Tab tab) {
+    stream_wait();
     extern __shared__ unsigned long long s_prefix[];
     __shared__ int32_t slots[256];
     __shared__ unsigned long long s_acc[4];
@@ -347,6 +331,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch_persistent(BatchArgs a, con
 
 template <BWalk K, int W, typename Word>
 __global__ void __launch_bounds__(256) k_batch_plain(BatchArgs a) {
+    stream_wait();
     __shared__ int32_t slots[256];
     BAcc acc;
     const uint32_t lane = threadIdx.x & 31u;
@@ -407,7 +392,7 @@ int persistent_blocks_per_sm(int block) {
 // and that needs fewer blocks than fill the GPU).
 template <BWalk K, int W, typename Word, typename Tab, typename SlotT>
 void launch_persistent_slots(const BatchArgs& a, const Tab& tab, int block, int blocks_per_sm, size_t smem,
-                             cudaStream_t s, unsigned grid_cap) {
+                             cudaStream_t s, unsigned grid_cap, bool captured) {
     auto grid_of = [&](int per_sm) {
         const unsigned g = (unsigned)(sm_count() * per_sm);
         return grid_cap && grid_cap < g ? grid_cap : g;
@@ -415,11 +400,13 @@ void launch_persistent_slots(const BatchArgs& a, const Tab& tab, int block, int 
     if (blocks_per_sm >= kCappedBlocks) {
         int fit = persistent_blocks_per_sm<K, W, Word, kCappedBlocks, Tab, SlotT>(block);
         int per_sm = blocks_per_sm < fit ? blocks_per_sm : fit;
-        k_batch_persistent<K, W, Word, kCappedBlocks, Tab, SlotT><<<grid_of(per_sm), block, smem, s>>>(a, tab);
+        launch_next_if(!captured, k_batch_persistent<K, W, Word, kCappedBlocks, Tab, SlotT>, grid_of(per_sm),
+                       (unsigned)block, smem, s, a, tab);
     } else {
         int fit = persistent_blocks_per_sm<K, W, Word, 1, Tab, SlotT>(block);
         int per_sm = (blocks_per_sm > 0 && blocks_per_sm < fit) ? blocks_per_sm : fit;
-        k_batch_persistent<K, W, Word, 1, Tab, SlotT><<<grid_of(per_sm), block, smem, s>>>(a, tab);
+        launch_next_if(!captured, k_batch_persistent<K, W, Word, 1, Tab, SlotT>, grid_of(per_sm), (unsigned)block, smem, s,
+                       a, tab);
     }
 }
 
@@ -431,56 +418,58 @@ template <BWalk K> constexpr bool kHasSlot32 = K == BWalk::Collab2;
 
 template <BWalk K, int W, typename Word, typename Tab>
 void launch_persistent(const BatchArgs& a, const Tab& tab, int block, int blocks_per_sm, size_t smem,
-                       cudaStream_t s, unsigned grid_cap) {
+                       cudaStream_t s, unsigned grid_cap, bool captured) {
     if constexpr (kHasSlot32<K>) {
         if (a.arena_len <= kSlot32Max) {
-            launch_persistent_slots<K, W, Word, Tab, uint32_t>(a, tab, block, blocks_per_sm, smem, s, grid_cap);
+            launch_persistent_slots<K, W, Word, Tab, uint32_t>(a, tab, block, blocks_per_sm, smem, s, grid_cap,
+                                                              captured);
             return;
         }
     }
-    launch_persistent_slots<K, W, Word, Tab, unsigned long long>(a, tab, block, blocks_per_sm, smem, s, grid_cap);
+    launch_persistent_slots<K, W, Word, Tab, unsigned long long>(a, tab, block, blocks_per_sm, smem, s, grid_cap, captured);
 }
 
 // tab: the inline descriptor table of a launch-form batch (null: a.groups).
+// captured: the launch becomes a graph's only batch node, with nothing to overlap.
 template <BWalk K, int W, typename Word>
 int launch_batch_kw(const BatchArgs& a, bool persistent, int block, int blocks_per_sm, cudaStream_t s,
-                    const GroupTable* tab, unsigned grid_cap) {
+                    const GroupTable* tab, unsigned grid_cap, bool captured) {
     if (persistent) {
         const size_t smem = a.fuse ? sizeof(unsigned long long) * (a.n_groups + 1u) : 0u;
-        if (tab) launch_persistent<K, W, Word>(a, *tab, block, blocks_per_sm, smem, s, grid_cap);
-        else launch_persistent<K, W, Word>(a, NoTable{}, block, blocks_per_sm, smem, s, grid_cap);
+        if (tab) launch_persistent<K, W, Word>(a, *tab, block, blocks_per_sm, smem, s, grid_cap, captured);
+        else launch_persistent<K, W, Word>(a, NoTable{}, block, blocks_per_sm, smem, s, grid_cap, captured);
     } else {
         const unsigned long long per_warp = 32ull * kReqPerLane<K>;
         unsigned long long warps = (a.count + per_warp - 1ull) / per_warp;
         unsigned long long grid = (warps * 32ull + (unsigned long long)block - 1ull) / (unsigned long long)block;
         if (grid < 1) grid = 1;
-        k_batch_plain<K, W, Word><<<(unsigned)grid, block, 0, s>>>(a);
+        launch_next(k_batch_plain<K, W, Word>, (unsigned)grid, (unsigned)block, 0, s, a);
     }
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }
 
 int launch_batch(const pbm_walk_config* c, const BatchArgs& a, bool persistent, cudaStream_t s,
-                 const GroupTable* tab = nullptr, unsigned grid_cap = 0) {
+                 const GroupTable* tab = nullptr, unsigned grid_cap = 0, bool captured = false) {
     const int block = c->block_size ? c->block_size : kDefaultBlock;
     const int bps = c->blocks_per_sm;
     const bool w64 = c->word_bits == 64;
     switch (c->strategy) {
     case PBM_RANDOM_WALK:
-        return launch_batch_kw<BWalk::Page, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap);
+        return launch_batch_kw<BWalk::Page, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap, captured);
     case PBM_RANDOM_WALK_BM:
-        return w64 ? launch_batch_kw<BWalk::Word64, 32, uint64_t>(a, persistent, block, bps, s, tab, grid_cap)
-                   : launch_batch_kw<BWalk::Word32, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap);
+        return w64 ? launch_batch_kw<BWalk::Word64, 32, uint64_t>(a, persistent, block, bps, s, tab, grid_cap, captured)
+                   : launch_batch_kw<BWalk::Word32, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap, captured);
     case PBM_COLLAB_RW_BM: {
         const int W = c->collab_width ? c->collab_width : 32;
-        if (W == 64) return w64 ? launch_batch_kw<BWalk::Collab2, 32, uint64_t>(a, persistent, block, bps, s, tab, grid_cap)
-                                : launch_batch_kw<BWalk::Collab2, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap);
-        if (W == 8) return w64 ? launch_batch_kw<BWalk::Collab, 8, uint64_t>(a, persistent, block, bps, s, tab, grid_cap)
-                               : launch_batch_kw<BWalk::Collab, 8, uint32_t>(a, persistent, block, bps, s, tab, grid_cap);
-        if (W == 16) return w64 ? launch_batch_kw<BWalk::Collab, 16, uint64_t>(a, persistent, block, bps, s, tab, grid_cap)
-                                : launch_batch_kw<BWalk::Collab, 16, uint32_t>(a, persistent, block, bps, s, tab, grid_cap);
-        return w64 ? launch_batch_kw<BWalk::Collab, 32, uint64_t>(a, persistent, block, bps, s, tab, grid_cap)
-                   : launch_batch_kw<BWalk::Collab, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap);
+        if (W == 64) return w64 ? launch_batch_kw<BWalk::Collab2, 32, uint64_t>(a, persistent, block, bps, s, tab, grid_cap, captured)
+                                : launch_batch_kw<BWalk::Collab2, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap, captured);
+        if (W == 8) return w64 ? launch_batch_kw<BWalk::Collab, 8, uint64_t>(a, persistent, block, bps, s, tab, grid_cap, captured)
+                               : launch_batch_kw<BWalk::Collab, 8, uint32_t>(a, persistent, block, bps, s, tab, grid_cap, captured);
+        if (W == 16) return w64 ? launch_batch_kw<BWalk::Collab, 16, uint64_t>(a, persistent, block, bps, s, tab, grid_cap, captured)
+                                : launch_batch_kw<BWalk::Collab, 16, uint32_t>(a, persistent, block, bps, s, tab, grid_cap, captured);
+        return w64 ? launch_batch_kw<BWalk::Collab, 32, uint64_t>(a, persistent, block, bps, s, tab, grid_cap, captured)
+                   : launch_batch_kw<BWalk::Collab, 32, uint32_t>(a, persistent, block, bps, s, tab, grid_cap, captured);
     }
     default:
         return PBM_ERR_UNSUPPORTED;
@@ -622,7 +611,7 @@ int pbm_batch_launch_results(pbm_pool* pool, const pbm_walk_config* cfg, const p
         }
         pool->prefix_cap = n_groups + 1u;
     }
-    k_batch_prefix<<<1, 1024, 0, s>>>(d_groups, n_groups, nullptr, 0u, 1u, pool->d_prefix);
+    k_batch_prefix<<<1, 1024, 0, s>>>(d_groups, n_groups, 0u, 1u, pool->d_prefix);
     PBM_LAUNCH_CHECK();
     a.groups = d_groups;
     a.n_groups = n_groups;
@@ -661,22 +650,17 @@ int pbm_batch_graph_create_results(pbm_pool* pool, const pbm_walk_config* cfg, c
     if (!g) return PBM_ERR_NOMEM;
     g->device = pool->device;
     const size_t pool_bytes = sizeof(unsigned long long) * 2u * kPools * 16u;
-    if (cudaMalloc(&g->d_pools, pool_bytes) != cudaSuccess ||
-        cudaMalloc(&g->d_prefix, sizeof(unsigned long long) * (n_groups + 1u)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(g->d_pools);
-        delete g;
-        return PBM_ERR_NOMEM;
-    }
     auto fail = [&](int code) {
-        if (g->exec) cudaGraphExecDestroy(g->exec);
-        if (g->graph) cudaGraphDestroy(g->graph);
         cudaFree(g->d_pools);
         cudaFree(g->d_prefix);
         delete g;
         cudaGetLastError();
         return code;
     };
+    const bool fuse = n_groups <= kFusedGroups;
+    if (cudaMalloc(&g->d_pools, pool_bytes) != cudaSuccess ||
+        (!fuse && cudaMalloc(&g->d_prefix, sizeof(unsigned long long) * (n_groups + 1u)) != cudaSuccess))
+        return fail(PBM_ERR_NOMEM);
     if (cudaMemsetAsync(g->d_pools, 0, pool_bytes, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
         return fail(PBM_ERR_CUDA);
     BatchArgs a = base_args(pool, cfg, d_arena, arena_len, seed0, nullptr);
@@ -687,61 +671,13 @@ int pbm_batch_graph_create_results(pbm_pool* pool, const pbm_walk_config* cfg, c
     a.step = 0u;                              // written before each replay
     a.n_steps = n_steps;
     a.pools = g->d_pools;
-    a.fuse = n_groups <= kFusedGroups ? 1 : 0;
-    static_assert(sizeof(BatchArgs) <= sizeof(g->batch_args), "graph keeps the kernel's arguments");
-    std::memcpy(g->batch_args, &a, sizeof(a));
-    g->prefix_groups = d_groups;
-    g->prefix_n_groups = n_groups;
-    g->prefix_n_steps = n_steps;
-    g->prefix_out = g->d_prefix;
-    // Capture on a private stream (the legacy default stream cannot be
-    // captured); the graph is replayed later on the caller's stream.  The
-    // occupancy query runs before capture.
-    pbm_walk_config c2 = *cfg;
+    a.fuse = fuse ? 1 : 0;
     resolve_blocks_per_sm(cfg, arena_len);   // fills the occupancy caches before the capture starts
-    cudaStream_t cap = nullptr;
-    if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess) return fail(PBM_ERR_CUDA);
     const unsigned long long before = g_launches.load();
-    cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) {
-        cudaStreamDestroy(cap);
-        return fail(PBM_ERR_CUDA);
-    }
-    if (!a.fuse) {
-        k_batch_prefix<<<1, 1024, 0, cap>>>(d_groups, n_groups, nullptr, 0u, n_steps, g->d_prefix);
-        count_launch();
-    }
-    rc = launch_batch(&c2, a, true, cap);
-    cudaGraph_t graph = nullptr;
-    e = cudaStreamEndCapture(cap, &graph);
-    cudaStreamDestroy(cap);
-    g->graph = graph;
-    if (rc || e != cudaSuccess) return fail(rc ? rc : PBM_ERR_CUDA);
-    // the kernel nodes whose parameters carry the step
-    size_t nn = 0;
-    if (cudaGraphGetNodes(graph, nullptr, &nn) != cudaSuccess) return fail(PBM_ERR_CUDA);
-    std::vector<cudaGraphNode_t> nodes(nn);
-    if (nn && cudaGraphGetNodes(graph, nodes.data(), &nn) != cudaSuccess) return fail(PBM_ERR_CUDA);
-    for (cudaGraphNode_t node : nodes) {
-        cudaGraphNodeType t;
-        cudaKernelNodeParams kp{};
-        if (cudaGraphNodeGetType(node, &t) != cudaSuccess || t != cudaGraphNodeTypeKernel) continue;
-        if (cudaGraphKernelNodeGetParams(node, &kp) != cudaSuccess) return fail(PBM_ERR_CUDA);
-        kp.kernelParams = nullptr;   // pointed into the graph; replays pass their own
-        kp.extra = nullptr;
-        if (kp.func == (void*)k_batch_prefix) {
-            g->prefix_node = node;
-            g->prefix_kp = kp;
-        } else {
-            g->batch_node = node;
-            g->batch_kp = kp;
-        }
-    }
-    if (!g->batch_node || (!a.fuse && !g->prefix_node)) return fail(PBM_ERR_CUDA);
-    if (cudaGraphInstantiate(&g->exec, graph, 0) != cudaSuccess) return fail(PBM_ERR_CUDA);
-    g->launches_per_replay = g_launches.load() - before;
-    // capture does not launch: take the counted launches back
-    g_launches.fetch_sub(g->launches_per_replay);
+    rc = graph_capture(g, a, offsetof(BatchArgs, step), d_groups, n_groups, n_steps, fuse,
+                       [&](cudaStream_t cap) { return launch_batch(cfg, a, true, cap, nullptr, 0, true); });
+    g_launches.fetch_sub(g_launches.load() - before);   // capture does not launch: take the counted launches back
+    if (rc != PBM_OK) return fail(rc);
     pool->fifo_valid = false;
     *out = g;
     return PBM_OK;
@@ -750,29 +686,26 @@ int pbm_batch_graph_create_results(pbm_pool* pool, const pbm_walk_config* cfg, c
 int pbm_graph_replay(pbm_graph* g, void* stream) {
     if (!g || !g->exec) return PBM_ERR_INVALID;
     pbm::DeviceScope scope(g->device);
-    if (g->batch_node) {
-        // this replay's step goes into the kernels' parameters (a host-side
-        // update of the instantiated graph; launches already queued keep theirs)
-        BatchArgs a;
-        std::memcpy(&a, g->batch_args, sizeof(a));
-        a.step = g->host_step;
-        NoTable tab{};
-        void* args[2] = {&a, &tab};
-        cudaKernelNodeParams kp = g->batch_kp;
-        kp.kernelParams = args;
-        PBM_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g->exec, g->batch_node, &kp));
-        if (g->prefix_node) {
-            const pbm_group* groups = g->prefix_groups;
-            uint32_t n_groups = g->prefix_n_groups, step = g->host_step, n_steps = g->prefix_n_steps;
-            const uint32_t* no_counter = nullptr;
-            unsigned long long* prefix = g->prefix_out;
-            void* pargs[6] = {&groups, &n_groups, &no_counter, &step, &n_steps, &prefix};
-            cudaKernelNodeParams pkp = g->prefix_kp;
-            pkp.kernelParams = pargs;
-            PBM_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g->exec, g->prefix_node, &pkp));
-        }
-        ++g->host_step;
+    // this replay's step goes into the kernels' parameters (a host-side
+    // update of the instantiated graph; launches already queued keep theirs)
+    alignas(16) unsigned char args[sizeof(g->main_args)];
+    std::memcpy(args, g->main_args, sizeof(args));
+    std::memcpy(args + g->step_offset, &g->host_step, sizeof(uint32_t));
+    NoTable tab{};
+    void* params[2] = {args, &tab};           // the malloc kernels take the first only
+    cudaKernelNodeParams kp = g->main_kp;
+    kp.kernelParams = params;
+    PBM_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g->exec, g->main_node, &kp));
+    if (g->prefix_node) {
+        const pbm_group* groups = g->prefix_groups;
+        uint32_t n_groups = g->prefix_n_groups, step = g->host_step, n_steps = g->prefix_n_steps;
+        unsigned long long* prefix = g->d_prefix;
+        void* pargs[5] = {&groups, &n_groups, &step, &n_steps, &prefix};
+        cudaKernelNodeParams pkp = g->prefix_kp;
+        pkp.kernelParams = pargs;
+        PBM_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g->exec, g->prefix_node, &pkp));
     }
+    ++g->host_step;
     PBM_CUDA_TRY(cudaGraphLaunch(g->exec, (cudaStream_t)stream));
     count_launch(g->launches_per_replay);
     return PBM_OK;
@@ -782,13 +715,9 @@ int pbm_graph_set_step(pbm_graph* g, uint32_t step, void* stream) {
     if (!g) return PBM_ERR_INVALID;
     pbm::DeviceScope scope(g->device);
     cudaStream_t s = (cudaStream_t)stream;
-    if (g->batch_node) {
-        g->host_step = step;
-        // both parities of the tail pools start empty again
-        PBM_CUDA_TRY(cudaMemsetAsync(g->d_pools, 0, sizeof(unsigned long long) * 2u * kPools * 16u, s));
-    } else {
-        PBM_CUDA_TRY(cudaMemcpyAsync(g->d_step, &step, sizeof(step), cudaMemcpyHostToDevice, s));
-    }
+    g->host_step = step;
+    // both parities of the batch kernel's tail pools start empty again
+    if (g->d_pools) PBM_CUDA_TRY(cudaMemsetAsync(g->d_pools, 0, sizeof(unsigned long long) * 2u * kPools * 16u, s));
     PBM_CUDA_TRY(cudaStreamSynchronize(s));
     return PBM_OK;
 }
@@ -798,7 +727,6 @@ int pbm_graph_destroy(pbm_graph* g) {
     pbm::DeviceScope scope(g->device);
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
-    cudaFree(g->d_step);
     cudaFree(g->d_pools);
     cudaFree(g->d_prefix);
     delete g;

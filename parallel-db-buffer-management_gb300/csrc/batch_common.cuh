@@ -2,6 +2,8 @@
 // the groups' prefix sums (as a block-level routine and as a kernel), the
 // group lookup, the step advance of the graph form, and the graph handle.
 #pragma once
+#include <cstring>
+
 #include "internal.cuh"
 
 namespace pbm {
@@ -24,12 +26,19 @@ __device__ __forceinline__ uint32_t find_group_any(const unsigned long long* pre
     return lo;
 }
 
-__device__ __forceinline__ uint32_t find_group(const unsigned long long* prefix, uint32_t n_groups,
-                                               unsigned long long q, uint32_t lo) {
+// Last g in [lo, n_groups) with prefix[g] <= q (prefix[lo] <= q), searched
+// by the whole warp: 32 evenly spaced probes and a ballot narrow the range
+// 32-fold per round (two rounds for 256 groups).
+__device__ __forceinline__ uint32_t find_group_warp(const unsigned long long* prefix, uint32_t n_groups,
+                                                    unsigned long long q, uint32_t lo) {
+    const uint32_t lane = threadIdx.x & 31u;
     uint32_t hi = n_groups;
-    while (lo + 1u < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(prefix + mid) <= q) lo = mid; else hi = mid;
+    while (hi - lo > 1u) {
+        const uint32_t stride = (hi - lo + 31u) >> 5;
+        const uint32_t idx = lo + lane * stride;
+        const uint32_t b = __ballot_sync(0xffffffffu, idx < hi && prefix[idx] <= q);
+        lo += (31u - (uint32_t)__clz((int)b)) * stride;
+        hi = min(hi, lo + stride);
     }
     return lo;
 }
@@ -72,43 +81,97 @@ __device__ __forceinline__ void block_exclusive_prefix(const pbm_group* g, uint3
     __syncthreads();
 }
 
-// Exclusive prefix of one step's groups (one block of 1024 threads).
-// Graph forms keep a monotone replay counter -- in device memory (d_step) or
-// in the launch's parameters (step, when d_step is null); replay k reads
-// descriptor table k mod n_steps (so a graph may be replayed any number of
-// times).
-__global__ void k_batch_prefix(const pbm_group* groups, uint32_t n_groups, const uint32_t* d_step,
-                               uint32_t step, uint32_t n_steps, unsigned long long* prefix) {
-    const uint32_t k = (d_step ? *d_step : step) % (n_steps ? n_steps : 1u);
-    block_exclusive_prefix(groups + (size_t)k * n_groups, n_groups, prefix);
-}
-
-__global__ void k_step_advance(uint32_t* d_step) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *d_step += 1u;
+// Exclusive prefix of one step's groups (one block of 1024 threads), for
+// batches of more groups than a block scans itself.  Replay k of a graph reads
+// descriptor table k mod n_steps (so a graph may be replayed any number of times).
+__global__ void k_batch_prefix(const pbm_group* groups, uint32_t n_groups, uint32_t step, uint32_t n_steps,
+                               unsigned long long* prefix) {
+    block_exclusive_prefix(groups + (size_t)(step % n_steps) * n_groups, n_groups, prefix);
 }
 
 }  // namespace
 }  // namespace pbm
 
-// A captured graph.  Its replay counter lives either in device memory
-// (d_step, advanced by a kernel of the graph) or on the host (host_step,
-// written into the kernels' parameters before each replay: the launches
-// then read the step with their parameters instead of from memory).
+// A captured graph: one kernel (and, for batches of many groups, the prefix kernel
+// before it).  Its replays are counted on the host, and the count is written into the
+// kernels' parameters before each one, so a launch reads its step with its
+// parameters and not from memory.
 struct pbm_graph {
     cudaGraph_t graph;
     cudaGraphExec_t exec;
-    uint32_t* d_step;                 // device replay counter (null: host_step)
     uint32_t host_step;
     unsigned long long* d_pools;      // the batch kernel's tail-pool counters (may be null)
-    unsigned long long* d_prefix;
+    unsigned long long* d_prefix;     // the prefix kernel's output (may be null)
     unsigned long long launches_per_replay;
     int device;                       // the pool's device: replays run there
-    // host-counted form: the kernel nodes whose parameters carry the step,
-    // their launch settings, and the parameter values they were captured with
-    cudaGraphNode_t batch_node, prefix_node;
-    cudaKernelNodeParams batch_kp, prefix_kp;
-    alignas(16) unsigned char batch_args[256];
+    // the kernel nodes whose parameters carry the step, their launch settings, and
+    // the main kernel's argument structure, with the step at step_offset
+    cudaGraphNode_t main_node, prefix_node;
+    cudaKernelNodeParams main_kp, prefix_kp;
+    alignas(16) unsigned char main_args[320];
+    size_t step_offset;
     const pbm_group* prefix_groups;
     uint32_t prefix_n_groups, prefix_n_steps;
-    unsigned long long* prefix_out;
 };
+
+namespace pbm {
+namespace {
+
+// Captures the graph's kernels -- the prefix kernel unless `fused`, then what launch(stream)
+// launches, one kernel whose argument structure is `args` -- and instantiates
+// them.  On failure the graph holds no capture.  Captured on a private stream:
+// the legacy default stream cannot be.
+template <typename Args, typename Launch>
+int graph_capture(pbm_graph* g, const Args& args, size_t step_offset, const pbm_group* d_groups, uint32_t n_groups,
+                  uint32_t n_steps, bool fused, Launch launch) {
+    static_assert(sizeof(Args) <= sizeof(g->main_args), "graph keeps the kernel's arguments");
+    std::memcpy(g->main_args, &args, sizeof(Args));
+    g->step_offset = step_offset;
+    g->prefix_groups = d_groups;
+    g->prefix_n_groups = n_groups;
+    g->prefix_n_steps = n_steps;
+    auto fail = [&](int code) {
+        if (g->exec) cudaGraphExecDestroy(g->exec);
+        if (g->graph) cudaGraphDestroy(g->graph);
+        g->exec = nullptr;
+        g->graph = nullptr;
+        cudaGetLastError();
+        return code;
+    };
+    cudaStream_t cap = nullptr;
+    if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess) return fail(PBM_ERR_CUDA);
+    if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        cudaStreamDestroy(cap);
+        return fail(PBM_ERR_CUDA);
+    }
+    if (!fused) k_batch_prefix<<<1, 1024, 0, cap>>>(d_groups, n_groups, 0u, n_steps, g->d_prefix);
+    const int rc = launch(cap);
+    const cudaError_t e = cudaStreamEndCapture(cap, &g->graph);
+    cudaStreamDestroy(cap);
+    if (rc != PBM_OK || e != cudaSuccess) return fail(rc != PBM_OK ? rc : PBM_ERR_CUDA);
+    cudaGraphNode_t nodes[2] = {};
+    size_t nn = 2;
+    if (cudaGraphGetNodes(g->graph, nodes, &nn) != cudaSuccess) return fail(PBM_ERR_CUDA);
+    for (size_t i = 0; i < nn && i < 2; ++i) {
+        cudaGraphNodeType t;
+        cudaKernelNodeParams kp{};
+        if (cudaGraphNodeGetType(nodes[i], &t) != cudaSuccess || t != cudaGraphNodeTypeKernel) continue;
+        if (cudaGraphKernelNodeGetParams(nodes[i], &kp) != cudaSuccess) return fail(PBM_ERR_CUDA);
+        kp.kernelParams = nullptr;   // pointed into the graph; replays pass their own
+        kp.extra = nullptr;
+        if (kp.func == (void*)k_batch_prefix) {
+            g->prefix_node = nodes[i];
+            g->prefix_kp = kp;
+        } else {
+            g->main_node = nodes[i];
+            g->main_kp = kp;
+        }
+    }
+    if (!g->main_node || (!fused && !g->prefix_node)) return fail(PBM_ERR_CUDA);
+    if (cudaGraphInstantiate(&g->exec, g->graph, 0) != cudaSuccess) return fail(PBM_ERR_CUDA);
+    g->launches_per_replay = fused ? 1u : 2u;
+    return PBM_OK;
+}
+
+}  // namespace
+}  // namespace pbm

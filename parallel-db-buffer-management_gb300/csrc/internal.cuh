@@ -75,8 +75,8 @@ __device__ __forceinline__ void stream_wait() {
 }
 
 template <typename... P, typename... A>
-inline cudaError_t launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                               A&&... args) {
+inline cudaError_t launch_next_if(bool overlap, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                                  cudaStream_t s, A&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -86,8 +86,14 @@ inline cudaError_t launch_next(void (*kernel)(P...), unsigned grid, unsigned blo
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                               A&&... args) {
+    return launch_next_if(true, kernel, grid, block, smem, s, args...);
 }
 
 // Copies the first `bytes` bytes of rows ids[0 .. n) of a table (row i at base + i *

@@ -7,6 +7,8 @@
 // Reference: mallocRW / freeRW (source/RWMalloc.cuh:299-334), the
 // KernelMallocCollab allocator (source/malloc.cu:223-320) and the
 // malloc/free drivers (unitTests/unitTest3.cu, unitTestMalloc1.cu).
+#include <atomic>
+#include <cstddef>
 #include <mutex>
 #include <new>
 
@@ -22,13 +24,14 @@ struct MArgs {
     QMallocView qm;
     const pbm_group* groups;
     uint32_t n_groups;
-    const uint32_t* d_step;
-    uint32_t n_steps;                 // graph form: replay k uses descriptor table k mod n_steps
+    uint32_t step;                    // graph form: the replay (set on the host before each launch)
+    uint32_t n_steps;                 // descriptor tables (replay k uses table k mod n_steps; >= 1)
     uint32_t seed;
     const uint32_t* sizes;            // per slot
     unsigned long long* ptrs;         // per slot (device addresses, 0 = none)
     unsigned long long arena_len;
-    const unsigned long long* prefix;
+    const unsigned long long* prefix;   // not fused: n_groups + 1 exclusive prefix
+    int32_t fuse;                     // each block scans the groups itself
     uint32_t max_steps;
     DevStats* stats;
     int32_t op;                       // plain form: the one group this launch serves
@@ -55,8 +58,10 @@ __device__ __forceinline__ void malloc_round(const MArgs& a, uint32_t seed, bool
     const bool do_free = active && op == PBM_OP_MFREE;
     const uint64_t size = do_malloc ? (uint64_t)a.sizes[slot] : 0ull;
     int32_t s = 0;
-    void* p;
-    if constexpr (Q) {
+    void* p = nullptr;
+    // a chunk usually lies in one group, so it is all mallocs or all frees
+    if (!__any_sync(0xffffffffu, do_malloc)) {
+    } else if constexpr (Q) {
         p = qmalloc_group(a.qm, 0xffffffffu, size, request_seed(seed, (uint32_t)q), a.max_steps, SERIAL, &s);
     } else {
         p = malloc_group(a.m, 0xffffffffu, size, request_seed(seed ^ 0x9E3779B9u, (uint32_t)q0),
@@ -70,6 +75,7 @@ __device__ __forceinline__ void malloc_round(const MArgs& a, uint32_t seed, bool
             acc.steps += (unsigned long long)s;
         }
     }
+    if (!__any_sync(0xffffffffu, do_free)) return;
     const void* fp = do_free ? (const void*)a.ptrs[slot] : nullptr;
     bool ok;
     if constexpr (Q) ok = qfree_group(a.qm, 0xffffffffu, fp);
@@ -88,31 +94,46 @@ __device__ __forceinline__ void flush_macc(const MAcc& c, DevStats* st) {
                           {&st->successes, &st->failures, &st->steps, &st->frees, &st->bad_frees});
 }
 
+// With a.fuse each block scans the step's group counts into shared memory itself, and
+// the graph form's step comes with the launch's parameters, so a replay is one
+// launch (a prefix kernel before it and a step kernel after it took 7 us of 39).  The
+// chunks are dealt round robin over the blocks (mallocs and frees, whose chunks cost
+// differently, come in long runs) and a block's warps take its next one from a shared counter.
 template <bool SERIAL, bool Q>
 __global__ void __launch_bounds__(256) k_malloc_persistent(MArgs a) {
+    stream_wait();
+    extern __shared__ unsigned long long s_prefix[];
+    __shared__ unsigned int s_next;
     MAcc acc;
-    const uint32_t step = a.d_step ? *a.d_step : 0u;
-    const pbm_group* groups = a.groups + (a.d_step ? (size_t)(step % a.n_steps) * a.n_groups : 0);
-    const uint32_t seed = a.seed + step;
-    const unsigned long long total = a.prefix[a.n_groups];
+    const pbm_group* groups = a.groups + (size_t)(a.step % a.n_steps) * a.n_groups;
+    const uint32_t seed = a.seed + a.step;
+    const unsigned long long* pre = a.prefix;
+    if (threadIdx.x == 0) s_next = 0u;
+    if (a.fuse) {
+        block_exclusive_prefix(groups, a.n_groups, s_prefix);
+        pre = s_prefix;
+    } else {
+        __syncthreads();
+    }
+    const unsigned long long total = pre[a.n_groups];
     const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long warp0 = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-    for (unsigned long long chunk = warp0; chunk * 32ull < total; chunk += nwarps) {
-        const unsigned long long q0 = chunk * 32ull;
+    for (;;) {
+        unsigned int k = 0;
+        if (lane == 0) k = atomicAdd(&s_next, 1u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        const unsigned long long q0 = ((unsigned long long)k * gridDim.x + blockIdx.x) * 32ull;
+        if (q0 >= total) break;
         const unsigned long long q = q0 + lane;
         const bool active = q < total;
-        uint32_t g0 = 0;
-        if (lane == 0) g0 = find_group(a.prefix, a.n_groups, q0, 0u);
-        g0 = __shfl_sync(0xffffffffu, g0, 0);
-        const unsigned long long g0_end = __ldg(a.prefix + g0 + 1u);
+        const uint32_t g0 = find_group_warp(pre, a.n_groups, q0, 0u);
+        const unsigned long long g0_end = pre[g0 + 1u];
         int op = PBM_OP_MALLOC;
         unsigned long long slot = 0;
         if (active) {
-            const uint32_t g = q < g0_end ? g0 : find_group(a.prefix, a.n_groups, q, g0);
+            const uint32_t g = q < g0_end ? g0 : find_group_any(pre, a.n_groups, q, g0);
             const pbm_group gd = groups[g];
             op = gd.op;
-            slot = wrap(gd.offset + (q - __ldg(a.prefix + g)), a.arena_len);
+            slot = wrap(gd.offset + (q - pre[g]), a.arena_len);
         }
         malloc_round<SERIAL, Q>(a, seed, active, op, q0, q, slot, acc);
     }
@@ -121,6 +142,7 @@ __global__ void __launch_bounds__(256) k_malloc_persistent(MArgs a) {
 
 template <bool Q>
 __global__ void __launch_bounds__(256) k_malloc_plain(MArgs a) {
+    stream_wait();
     MAcc acc;
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long warp0 = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -269,11 +291,27 @@ bool ensure_prefix(MallocTables* t, uint32_t n_groups) {
     return true;
 }
 
+// Resident blocks per SM of the persistent kernel (asked once).
 template <bool Q>
 int persistent_blocks() {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_malloc_persistent<false, Q>, 256, 0);
-    return per_sm < 1 ? 1 : per_sm;
+    static std::atomic<int> cache{0};
+    int per_sm = cache.load(std::memory_order_relaxed);
+    if (!per_sm) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_malloc_persistent<false, Q>, 256, kFusedPrefixBytes);
+        if (per_sm < 1) per_sm = 1;
+        cache.store(per_sm, std::memory_order_relaxed);
+    }
+    return per_sm;
+}
+
+// The persistent kernel's launch (plain stream order when captured).
+void launch_persistent(const MArgs& a, bool queue, bool serial, bool captured, cudaStream_t s) {
+    const size_t smem = a.fuse ? sizeof(unsigned long long) * (a.n_groups + 1u) : 0u;
+    const unsigned block = serial ? 32u : 256u;
+    const unsigned grid = serial ? 1u : (unsigned)(sm_count() * (queue ? persistent_blocks<true>() : persistent_blocks<false>()));
+    auto kernel = queue ? (serial ? k_malloc_persistent<true, true> : k_malloc_persistent<false, true>)
+                        : (serial ? k_malloc_persistent<true, false> : k_malloc_persistent<false, false>);
+    launch_next_if(!captured, kernel, grid, block, smem, s, a);
 }
 
 int batch_impl(pbm_pool* pool, bool queue, const pbm_group* d_groups, const pbm_group* h_groups, uint32_t n_groups,
@@ -306,28 +344,24 @@ int batch_impl(pbm_pool* pool, bool queue, const pbm_group* d_groups, const pbm_
             a.q_base = q;
             const unsigned long long warps = (gd.count + 31ull) / 32ull;
             const unsigned grid = (unsigned)((warps * 32ull + 255ull) / 256ull);
-            if (queue) k_malloc_plain<true><<<grid, 256, 0, s>>>(a);
-            else k_malloc_plain<false><<<grid, 256, 0, s>>>(a);
+            launch_next(queue ? k_malloc_plain<true> : k_malloc_plain<false>, grid, 256, 0, s, a);
             PBM_LAUNCH_CHECK();
             q += gd.count;
         }
         return PBM_OK;
     }
     if ((mode != PBM_LAUNCH_PERSISTENT && mode != PBM_LAUNCH_SERIAL) || !d_groups) return PBM_ERR_INVALID;
-    if (!ensure_prefix(t, n_groups)) return PBM_ERR_NOMEM;
-    k_batch_prefix<<<1, 1024, 0, s>>>(d_groups, n_groups, nullptr, 0u, 1u, t->prefix);
-    PBM_LAUNCH_CHECK();
     a.groups = d_groups;
     a.n_groups = n_groups;
-    a.prefix = t->prefix;
-    if (mode == PBM_LAUNCH_SERIAL) {
-        if (queue) k_malloc_persistent<true, true><<<1, 32, 0, s>>>(a);
-        else k_malloc_persistent<true, false><<<1, 32, 0, s>>>(a);
-    } else if (queue) {
-        k_malloc_persistent<false, true><<<sm_count() * persistent_blocks<true>(), 256, 0, s>>>(a);
-    } else {
-        k_malloc_persistent<false, false><<<sm_count() * persistent_blocks<false>(), 256, 0, s>>>(a);
+    a.n_steps = 1u;
+    a.fuse = n_groups <= kFusedGroups ? 1 : 0;
+    if (!a.fuse) {
+        if (!ensure_prefix(t, n_groups)) return PBM_ERR_NOMEM;
+        k_batch_prefix<<<1, 1024, 0, s>>>(d_groups, n_groups, 0u, 1u, t->prefix);
+        PBM_LAUNCH_CHECK();
+        a.prefix = t->prefix;
     }
+    launch_persistent(a, queue, mode == PBM_LAUNCH_SERIAL, false, s);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }
@@ -340,28 +374,22 @@ int graph_impl(pbm_pool* pool, bool queue, const pbm_group* d_groups, uint32_t n
         !arena_len)
         return PBM_ERR_INVALID;
     *out = nullptr;
-    cudaStream_t s = (cudaStream_t)stream;
     pbm_graph* g = new (std::nothrow) pbm_graph();
     if (!g) return PBM_ERR_NOMEM;
     g->device = pool->device;
-    g->graph = nullptr;
-    g->exec = nullptr;
-    if (cudaMalloc(&g->d_step, sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&g->d_prefix, sizeof(unsigned long long) * (n_groups + 1u)) != cudaSuccess) {
+    const bool fuse = n_groups <= kFusedGroups;
+    if (!fuse && cudaMalloc(&g->d_prefix, sizeof(unsigned long long) * (n_groups + 1u)) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(g->d_step);
         delete g;
         return PBM_ERR_NOMEM;
     }
-    PBM_CUDA_TRY(cudaMemsetAsync(g->d_step, 0, sizeof(uint32_t), s));
-    PBM_CUDA_TRY(cudaStreamSynchronize(s));
     MArgs a{};
     if (queue) a.qm = qview_of(pool, t);
     else a.m = view_of(pool, t);
     a.groups = d_groups;
     a.n_groups = n_groups;
-    a.d_step = g->d_step;
     a.n_steps = n_steps;
+    a.fuse = fuse ? 1 : 0;
     a.seed = seed0;
     a.sizes = d_sizes;
     a.ptrs = d_ptrs;
@@ -369,32 +397,18 @@ int graph_impl(pbm_pool* pool, bool queue, const pbm_group* d_groups, uint32_t n
     a.prefix = g->d_prefix;
     a.max_steps = max_steps ? max_steps : kDefaultMaxSteps;
     a.stats = pool->d_stats;
-    const int per_sm = queue ? persistent_blocks<true>() : persistent_blocks<false>();
-    cudaStream_t cap = nullptr;
-    PBM_CUDA_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        k_batch_prefix<<<1, 1024, 0, cap>>>(d_groups, n_groups, g->d_step, 0u, n_steps, g->d_prefix);
-        if (queue) k_malloc_persistent<false, true><<<sm_count() * per_sm, 256, 0, cap>>>(a);
-        else k_malloc_persistent<false, false><<<sm_count() * per_sm, 256, 0, cap>>>(a);
-        k_step_advance<<<1, 32, 0, cap>>>(g->d_step);
-        cudaGraph_t graph = nullptr;
-        e = cudaStreamEndCapture(cap, &graph);
-        if (e == cudaSuccess) {
-            g->graph = graph;
-            e = cudaGraphInstantiate(&g->exec, graph, 0);
-        }
-    }
-    cudaStreamDestroy(cap);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        if (g->graph) cudaGraphDestroy(g->graph);
-        cudaFree(g->d_step);
+    if (queue) persistent_blocks<true>();   // asked before the capture
+    else persistent_blocks<false>();
+    const int rc = graph_capture(g, a, offsetof(MArgs, step), d_groups, n_groups, n_steps, fuse,
+                                 [&](cudaStream_t cap) {
+                                     launch_persistent(a, queue, false, true, cap);
+                                     return cudaGetLastError() == cudaSuccess ? PBM_OK : PBM_ERR_CUDA;
+                                 });
+    if (rc != PBM_OK) {
         cudaFree(g->d_prefix);
         delete g;
-        return PBM_ERR_CUDA;
+        return rc;
     }
-    g->launches_per_replay = 3;
     pool->fifo_valid = false;
     *out = g;
     return PBM_OK;
