@@ -1004,16 +1004,20 @@ __device__ __forceinline__ int32_t walk_span(const PoolView& v, uint32_t n, int3
 
 // Runs of need_n <= 32 pages (0 = none) for the lanes of a whole warp, each
 // lane on its own LCG sequence from seed0; steps = jumps.  Every needing
-// lane first takes one jump of its own (all in parallel).  Each lane still
-// unserved is then walked by the whole warp, 32 of its jumps at a time:
-// lane j judges the lane's jump s + j + 1 (its LCG state advanced j + 1
-// steps at once) and the runs found are claimed in jump order.  In a run
+// lane first takes one jump of its own (all in parallel).  The walks still unserved
+// then share the warp: with m of them each gets 2^floor(log2(32 / m)) lanes, lane j
+// of a walk judging its jump s + j + 1 (its LCG state advanced j + 1 steps at once),
+// and the runs found are claimed in jump order, the walks side by side.  In a run
 // without races a lane gets the page the one-lane walk would give it, after
-// the same jumps; a walk that keeps missing costs max_steps / 32 rounds
-// instead of max_steps jumps.  The whole warp calls converged.
+// the same jumps; a walk that keeps missing alone costs max_steps / 32 rounds
+// instead of max_steps jumps.  (One walk at a time with all 32 lanes took a round of
+// two round trips per unserved walk.  Measured on GB300, mallocs of 16 B .. 64 KiB and
+// their frees: 524,288 into 2^22 pages 62 -> 58 us, 192,155 into 1.5 M pages 48 -> 33 us.)
+// The whole warp calls converged.
 __device__ __forceinline__ int32_t walk_span_warp(const PoolView& v, uint32_t need_n, int32_t seed0,
                                                   uint32_t max_steps, int32_t* steps_out) {
     const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lt = (1u << lane) - 1u;
     const uint32_t L = v.n_words32;
     int32_t x = seed0 & 0x7fffffff;   // walks run on 31-bit states
     uint32_t s = 0;
@@ -1031,41 +1035,43 @@ __device__ __forceinline__ int32_t walk_span_warp(const PoolView& v, uint32_t ne
     uint32_t aj = 0u, cj = 0u;                             // jump ahead by lane + 1 steps
     if (pend) lcg_jump<6>(lane + 1u, aj, cj);
     while (pend) {
-        const int l0 = __ffs((int)pend) - 1;
-        const uint32_t x0 = (uint32_t)__shfl_sync(kFull32, x, l0);
-        const uint32_t n0 = __shfl_sync(kFull32, need_n, l0);
-        const uint32_t s0 = __shfl_sync(kFull32, s, l0);
-        const int32_t xj = (int32_t)((aj * x0 + cj) & 0x7fffffffu);
+        const uint32_t m = (uint32_t)__popc(pend);
+        const uint32_t sh = (uint32_t)__clz((int)(m - 1u)) - 27u;   // floor(log2(32 / m)): clz(0) is 32
+        const uint32_t j = lane & ((1u << sh) - 1u);
+        const uint32_t rank = lane >> sh;
+        const uint32_t owner = rank < m ? nth_set_bit(pend, (int)rank) : 0u;
+        const uint32_t x0 = (uint32_t)__shfl_sync(kFull32, x, (int)owner);
+        const uint32_t n0 = __shfl_sync(kFull32, need_n, (int)owner);
+        const uint32_t s0 = __shfl_sync(kFull32, s, (int)owner);
+        const uint32_t a = __shfl_sync(kFull32, aj, (int)j), c = __shfl_sync(kFull32, cj, (int)j);
+        const int32_t xj = (int32_t)((a * x0 + c) & 0x7fffffffu);
         const uint32_t wj = idx_hi(xj, L);
         int32_t fj = -1;
-        if (s0 + lane + 1u <= max_steps) {
+        if (rank < m && j < max_steps - s0) {
             const uint32_t a0 = load_word(v.words + wj);
             const uint32_t a1 = wj + 1u < L ? load_word(v.words + wj + 1u) : kFull32;
             fj = span_in_pair(wj, a0, a1, n0, L);
         }
-        uint32_t cm = __ballot_sync(kFull32, fj >= 0);
-        int32_t got = -1;
-        uint32_t used = 32u;
-        while (cm) {                                       // claims in jump order
-            const int j = __ffs((int)cm) - 1;
-            cm &= cm - 1u;
-            bool ok = false;
-            if ((int)lane == j) ok = claim_span(v, (uint32_t)fj, n0);
-            if (__shfl_sync(kFull32, ok, j)) {
-                got = __shfl_sync(kFull32, fj, j);
-                used = (uint32_t)j + 1u;
-                break;
-            }
+        // claims in jump order: each walk's first candidate, the next one where that was lost
+        const uint32_t gm = (uint32_t)(((1ull << (1u << sh)) - 1ull) << (lane - j));   // this walk's lanes
+        uint32_t open = __ballot_sync(kFull32, fj >= 0), won = 0u;
+        while (open) {
+            const bool first = ((open >> lane) & 1u) && !(open & gm & lt);
+            const bool ok = first && claim_span(v, (uint32_t)fj, n0);
+            won |= __ballot_sync(kFull32, ok);
+            open = __ballot_sync(kFull32, ((open >> lane) & 1u) && !first && !(won & gm));
         }
-        const int32_t x_last = __shfl_sync(kFull32, xj, 31);   // the state 32 jumps on
-        if ((int)lane == l0) {
-            if (got >= 0) {
-                id = got;
-                s = s0 + used;
-            } else {
-                s = s0 + 32u < max_steps ? s0 + 32u : max_steps;
-                x = x_last;
-            }
+        const uint32_t base = ((uint32_t)__popc(pend & lt) << sh) & 31u;   // the first lane of this lane's walk
+        const uint32_t last = base + (1u << sh) - 1u;
+        const uint32_t mine = (won >> base) << base;
+        const uint32_t low = mine ? (uint32_t)__ffs((int)mine) - 1u : 32u;
+        const uint32_t src = low <= last ? low : last;
+        const int32_t xs = __shfl_sync(kFull32, xj, (int)src);
+        const int32_t fs = __shfl_sync(kFull32, fj, (int)src);
+        if ((pend >> lane) & 1u) {
+            s += min(src - base + 1u, max_steps - s);
+            x = xs;
+            if (low <= last) id = fs;
         }
         pend = __ballot_sync(kFull32, need_n > 0u && id < 0 && s < max_steps);
     }
