@@ -262,3 +262,63 @@ def test_budget_pass_beside_another_stream(cuda, pbm_mod, orc):
         pool.free(cfg, both.numel(), both)
         assert pool.used() == base
     pool.close()
+
+
+@pytest.mark.parametrize("max_steps", [1, 31, 32, 33, 100, 4096])
+@pytest.mark.parametrize("T,occ", [(33, 0.5), (96, 0.9), (1000, 0.99), (65536 + 17, 0.995)])
+def test_distributed_clock_counts_positions(cuda, pbm_mod, orc, T, occ, max_steps):
+    """Word-wise reading changes neither the pages nor the steps nor the arms, across the pool's end and
+    where the bound ends a sweep inside a word."""
+    torch, pbm = cuda, pbm_mod
+    slots, n = 3, 3
+    pool = pbm.Pool(T, 64, max_slots=slots)
+    pool.prefill(occ, 2)
+    words = orc.bernoulli_bitmap(T, occ, 2)
+    arms = np.array([orc.lib().orc_dist_clock_arm0(0, i, T) for i in range(slots)], dtype=np.int64)
+    cfg = pbm.walk_config(pbm.DIST_CLOCK, max_steps=max_steps)
+    ids = torch.empty(n, dtype=torch.int32, device="cuda")
+    steps = torch.empty(n, dtype=torch.int32, device="cuda")
+    for S in range(8):
+        pool.alloc(cfg, n, S, ids, steps, serial=True)
+        e_ids, e_steps = orc.replay_alloc(words, T, pbm.DIST_CLOCK, n, S, max_steps=max_steps, arms=arms)
+        assert np.array_equal(ids.cpu().numpy(), e_ids) and np.array_equal(steps.cpu().numpy(), e_steps)
+        assert np.array_equal(pool.read_bitmap(), words)
+    pool.close()
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 4000])
+@pytest.mark.parametrize("max_run", [1, 8, 32, 60])
+def test_spans_of_sharing_warps(cuda, pbm_mod, orc, n, max_run):
+    """Runs walked for by whole warps (longer ones by their own lane): one request alone equals the
+    sequential walk; many are disjoint, were free, and come back."""
+    torch, pbm = cuda, pbm_mod
+    T = 1 << 18
+    rng = np.random.default_rng(n + max_run)
+    k = rng.integers(1, max_run + 1, n).astype(np.int32)
+    if n > 1:
+        k[rng.random(n) < 0.05] = 0                     # not a run: fails at once
+    dk = torch.from_numpy(k).cuda()
+    ids = torch.empty(n, dtype=torch.int32, device="cuda")
+    steps = torch.empty(n, dtype=torch.int32, device="cuda")
+    pool = pbm.Pool(T, 64)
+    for occ in (0.0, 0.02, 0.08):
+        pool.reset()
+        pool.prefill(occ, 3)
+        words = orc.bernoulli_bitmap(T, occ, 3)
+        bits = np.unpackbits(words.view(np.uint8), bitorder="little")[:T].astype(np.int32)
+        pool.alloc_spans(n, dk, 9, ids, steps)
+        got, st = ids.cpu().numpy(), steps.cpu().numpy()
+        if n == 1:
+            e_ids, e_steps = orc.replay_spans(words, T, k, 9)
+            assert np.array_equal(got, e_ids) and np.array_equal(st, e_steps)
+            assert np.array_equal(pool.read_bitmap(), words)
+        assert (got[k == 0] == -1).all() and (st[k == 0] == 0).all()
+        cover = bits.copy()
+        for i, c in zip(got[got >= 0], k[got >= 0]):
+            cover[i:i + c] += 1
+        assert cover.max() == 1 and (got[got >= 0] + k[got >= 0] <= T).all()
+        if max_run <= 32:
+            assert (got[k > 0] >= 0).all()
+        pool.free_runs(n, ids, dk)
+        assert np.array_equal(np.unpackbits(pool.read_bitmap().view(np.uint8), bitorder="little")[:T], bits)
+    pool.close()
