@@ -921,10 +921,13 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     // Blocks of 64 threads for rounds that would not give every SM two blocks of 256 (a
     // round of 16,384 fetches is 64 such blocks), and for rounds that copy, whose
     // staging buffers (32 KiB a warp) are then shared out in small blocks.  A larger round
-    // that copies nothing merges its requests over 256 threads.
+    // that copies nothing merges its requests over 256 threads, over 128 with private
+    // hands, whose kernel has 78 registers (eight rounds of 131,072 and 262,144 fetches, blocks of
+    // 64 / 128 / 256: 150 / 135 / 127 and 246 / 226 / 219 us with the single hand, 183 / 168 / 184
+    // and 194 / 172 / 188 us with private ones).
     const bool copy = m->v.backing && m->v.frames;
     const bool small = copy || work < (uint32_t)sm_count() * 512u;
-    const int block = serial ? 1 : small ? 64 : 256;
+    const int block = serial ? 1 : small ? 64 : m->v.dist ? 128 : 256;
     const int grid = serial ? 1 : (int)(((uint64_t)work + (uint32_t)block - 1u) / (uint32_t)block);
     const size_t stage = copy && !serial ? 2u * (size_t)copy_slots(m->v.frame_size) * copy_piece(m->v.frame_size) : 0u;
     cudaError_t attr = cudaSuccess;
@@ -945,7 +948,7 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
             by_page ? go(k_round<false, true, false, 64>) : go(k_round<false, false, false, 64>);
     } else {
         if (m->v.dist)
-            by_page ? go(k_round<true, true, false, 256>) : go(k_round<true, false, false, 256>);
+            by_page ? go(k_round<true, true, false, 128>) : go(k_round<true, false, false, 128>);
         else
             by_page ? go(k_round<false, true, false, 256>) : go(k_round<false, false, false, 256>);
     }
