@@ -43,16 +43,30 @@ __device__ __forceinline__ void flush_acc(const Acc& a, DevStats* st) {
 // requests lost their page meanwhile and walk (or the pass served none).
 __device__ __forceinline__ bool finish_listed(const AllocArgs& a, Acc& acc) {
     if (!a.budget || !__ldcg(&a.budget->list_mode) || __ldcg(&a.budget->lost)) return false;
-    // the first kFinishBlocks blocks do it: each block that counts something ends in an atomic at one address
-    constexpr uint32_t kFinishBlocks = 1024;
-    const uint64_t nthr = (uint64_t)min(gridDim.x, kFinishBlocks) * blockDim.x;
-    if (blockIdx.x >= kFinishBlocks) return true;
-    for (uint64_t r = (uint64_t)__ldcg(&a.budget->free_at_start) + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < a.n;
-         r += nthr) {
+    // the first kFinishBlocks blocks do it (each block that counts something ends in an atomic at one
+    // address), four requests a store where the outputs allow it
+    constexpr uint32_t kFinishBlocks = 608;
+    const uint32_t blocks = min(gridDim.x, kFinishBlocks);
+    if (blockIdx.x >= blocks) return true;
+    const uint32_t nthr = blocks * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned long long F = (unsigned long long)__ldcg(&a.budget->free_at_start);
+    if (F >= a.n) return true;
+    const uint32_t f = (uint32_t)F, n = a.n;
+    uint32_t lo = f, hi = f;                       // [lo, hi): stored four at a time
+    if ((((uintptr_t)a.ids | (uintptr_t)a.steps) & 15u) == 0u && n - f >= 8u) {
+        lo = (f + 3u) & ~3u;
+        hi = n & ~3u;
+        for (uint32_t i = (lo >> 2) + tid; i < hi >> 2; i += nthr) {
+            reinterpret_cast<int4*>(a.ids)[i] = make_int4(-1, -1, -1, -1);
+            if (a.steps) reinterpret_cast<int4*>(a.steps)[i] = make_int4(0, 0, 0, 0);
+        }
+    }
+    for (uint64_t i = tid; i < (lo - f) + (n - hi); i += nthr) {
+        const uint64_t r = i < lo - f ? f + i : hi + (i - (lo - f));
         a.ids[r] = -1;
         if (a.steps) a.steps[r] = 0;
-        ++acc.fail;
     }
+    if (tid == 0) acc.fail += n - f;
     return true;
 }
 

@@ -246,9 +246,14 @@ int fifo_build(pbm_pool* pool, cudaStream_t s) {
 }
 
 // ---- fail-fast launch budget ----
+// Both passes run at most kBudgetPerSm blocks of kBudgetThreads per SM, what the second
+// one's shared memory lets fit: on 2^24 pages a block's slice is then one word per thread.
+constexpr int kBudgetThreads = 288;
+constexpr int kBudgetPerSm = 6;
+
 // Pass 1: the free pages (clear bits; padding bits stay set) of each block's
 // contiguous slice of `per` 64-bit words, into counts[block].
-__global__ void __launch_bounds__(256) k_free_budget(const unsigned long long* words, uint32_t n_words64, uint32_t per,
+__global__ void __launch_bounds__(kBudgetThreads) k_free_budget(const unsigned long long* words, uint32_t n_words64, uint32_t per,
                                                      unsigned long long* counts, LaunchBudget* b) {
     stream_wait();
     const uint64_t w0 = (uint64_t)blockIdx.x * per;
@@ -274,13 +279,15 @@ __global__ void __launch_bounds__(256) k_free_budget(const unsigned long long* w
 // a list of pages here and taking each page of it with an atomic of its own in that kernel
 // moved 8 more bytes per page and took an atomic per page instead of per
 // word.  Measured on GB300, 2^22 requests on 2^24 pages at 90% (1.68 M granted) and
-// their frees: 63 -> 37 us.
-__global__ void __launch_bounds__(256) k_take_free(unsigned long long* words, uint32_t n_words64, uint32_t per,
+// their frees: 63 -> 37 us, and 29 with a word per thread here and refusals stored four
+// at a time behind it.
+__global__ void __launch_bounds__(kBudgetThreads, kBudgetPerSm) k_take_free(unsigned long long* words, uint32_t n_words64, uint32_t per,
                                                    const unsigned long long* counts, LaunchBudget* b, uint32_t n_requests,
                                                    unsigned long long cap, int32_t* ids, int32_t* steps, DevStats* stats) {
-    __shared__ uint32_t warp_tot[8];
+    constexpr uint32_t kWarps = kBudgetThreads / 32;
+    __shared__ uint32_t warp_tot[kWarps];
     __shared__ unsigned long long s_sum[2];
-    __shared__ uint16_t stage[8][2048];        // per warp: page offsets within its 32 words
+    __shared__ uint16_t stage[kWarps][2048];   // per warp: page offsets within its 32 words
     stream_wait();
     unsigned long long off = 0, F = 0;
     for (uint32_t k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
@@ -310,7 +317,7 @@ __global__ void __launch_bounds__(256) k_take_free(unsigned long long* words, ui
     const uint64_t w0 = (uint64_t)blockIdx.x * per;
     const uint64_t w1 = min((uint64_t)n_words64, w0 + per);
     uint32_t done = 0, lost = 0;               // requests behind this chunk (block-uniform); lost: this thread's
-    for (uint64_t base = w0; base < w1 && done < quota; base += 256u) {
+    for (uint64_t base = w0; base < w1 && done < quota; base += kBudgetThreads) {
         const uint64_t w = base + threadIdx.x;
         const uint64_t fr = w < w1 ? ~(uint64_t)__ldcg(words + w) : 0ull;
         const int c = __popcll(fr);
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(256) k_take_free(unsigned long long* words, ui
         __syncthreads();
         uint32_t before = 0, total = 0;
 #pragma unroll
-        for (uint32_t i = 0; i < 8u; ++i) {
+        for (uint32_t i = 0; i < kWarps; ++i) {
             const uint32_t x = warp_tot[i];
             if (i < warp) before += x;
             total += x;
@@ -354,7 +361,7 @@ __global__ void __launch_bounds__(256) k_take_free(unsigned long long* words, ui
     }
     // pages counted here but gone before they were read
     uint32_t missing = 0;
-    for (uint32_t i = done + threadIdx.x; i < quota; i += 256u) {
+    for (uint32_t i = done + threadIdx.x; i < quota; i += kBudgetThreads) {
         out[i] = kLostPage;
         ++missing;
     }
@@ -375,9 +382,9 @@ int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t*
     const uint32_t nb = pool->budget_blocks;
     const uint32_t per = (nw64 + nb - 1u) / nb;
     unsigned long long* words = reinterpret_cast<unsigned long long*>(pool->d_words);
-    launch_next(k_free_budget, nb, 256, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget);
+    launch_next(k_free_budget, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget);
     PBM_LAUNCH_CHECK();
-    launch_next(k_take_free, nb, 256, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget, n_requests,
+    launch_next(k_take_free, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget, n_requests,
                 pool->list_cap, d_ids, d_steps, pool->d_stats);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
@@ -471,9 +478,10 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
     p->view.page_size = cfg->page_size;
     const uint32_t nb_scan = (uint32_t)((p->view.n_words32 + 4095u) / 4096u) + 1u;
     p->prefix_cap = 0;
-    // the budget pass: one block per 256 64-bit words, at most 4 per SM; it hands
+    // the budget pass: a block per kBudgetThreads 64-bit words, at most kBudgetPerSm per SM; it hands
     // pages out itself in a pool at least half full
-    p->budget_blocks = (uint32_t)std::min<uint64_t>((uint64_t)sm_count() * 4u, std::max<uint64_t>(1u, (nw64 + 255u) / 256u));
+    p->budget_blocks = (uint32_t)std::min<uint64_t>((uint64_t)sm_count() * kBudgetPerSm,
+                                                 (nw64 + kBudgetThreads - 1u) / kBudgetThreads);
     p->list_cap = std::max<uint64_t>(1024u, cfg->n_pages / 2u);
     bool ok = cudaMalloc(&p->d_words, p->bitmap_bytes) == cudaSuccess &&
               cudaMalloc(&p->d_stats, sizeof(DevStats)) == cudaSuccess &&
