@@ -406,8 +406,8 @@ __device__ __forceinline__ void bulk_stores_done() {
 // sends it to the frame with one bulk store, so a warp has kCopyStage bytes
 // in flight with two instructions per piece.  Copying through registers, four 16-byte
 // loads per lane, kept 2 KiB per warp in flight: a round of 16,384 fetches (30%
-// misses) of 4 KiB pages took 41 us, of which COPY_NOTE.  The whole warp
-// calls converged.
+// misses) of 4 KiB pages took 41 us, 18 this way (6 of them here, 3.5 TB/s read).  The
+// whole warp calls converged.
 constexpr uint32_t kCopyPiece = 4096;
 constexpr uint32_t kCopyStage = 32768;   // per warp
 
@@ -506,7 +506,10 @@ __device__ __forceinline__ bool release_target(const BmView& b, int32_t v, uint3
 // merging within the block rather than the warp divides the atomics that
 // queue on one page's entry by the block's warps.  Releases by page share
 // the fetches' table: a block that releases and fetches one page moves its
-// pins with one atomic.
+// pins with one atomic.  Every lane inserts its own key: finding a warp's equal
+// keys first (__match_any_sync) cost more than the shared-memory atomics it
+// saved (eight rounds of 131,072 Zipf(0.99) fetches 133 -> 122 us without it, of 262,144
+// 220 -> 196; 131,072 fetches of one page 10.4 -> 8.0 us a round).
 // A table has twice as many slots as the block can have keys (KEYS: a power of two).
 constexpr uint32_t kMergeEmpty = 0xffffffffu;   // no page or frame id reaches it
 constexpr uint32_t kMergeFirst = 1u << 31;
@@ -521,24 +524,24 @@ struct MergeTables {
     uint32_t rcnt[FRAMES ? 2 * KEYS : 1];
 };
 
-// Adds c to cnt[slot of key]; returns the slot, with kMergeFirst set for the
-// lane whose add came first (the slot's leader for that count).  A table
+// Counts one request for key in cnt[its slot]; returns the slot, with kMergeFirst
+// set for the lane that came first (the slot's leader for that count).  A table
 // never holds more keys than half its slots, so a slot is found.
 template <uint32_t KEYS>
-__device__ __forceinline__ uint32_t merge_insert(uint32_t* keys, uint32_t* cnt, uint32_t key, uint32_t c) {
+__device__ __forceinline__ uint32_t merge_insert(uint32_t* keys, uint32_t* cnt, uint32_t key) {
     uint32_t h = (uint32_t)(((unsigned long long)(key * 2654435761u) * (2u * KEYS)) >> 32);
     for (uint32_t probe = 0; probe < 2u * KEYS; ++probe) {
         const uint32_t prev = atomicCAS(keys + h, kMergeEmpty, key);
-        if (prev == kMergeEmpty || prev == key) return atomicAdd(cnt + h, c) == 0u ? (h | kMergeFirst) : h;
+        if (prev == kMergeEmpty || prev == key) return atomicAdd(cnt + h, 1u) == 0u ? (h | kMergeFirst) : h;
         h = (h + 1u) & (2u * KEYS - 1u);
     }
     return kMergeEmpty;   // not reached
 }
 
 // The many-thread round.  Per block iteration every lane takes release i
-// and fetch i (i = the block's base + threadIdx.x); lanes merge by key in the
-// warp (match) and then in the block (the tables), and each key's leader
-// issues its atomic: the fetch's pin (with the block's releases of the page,
+// and fetch i (i = the block's base + threadIdx.x); equal keys meet in the
+// block's tables, and each key's leader issues its atomic: the fetch's pin (with
+// the block's releases of the page,
 // releasing by page), and other releases while the pins are in flight.  The
 // fetch's result goes back through the table to every lane that asked for
 // the page.  With the single hand each warp also takes and examines its
@@ -585,13 +588,10 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
             }
         }
         const bool valid = p >= 0 && (uint32_t)p < b.n_logical;
-        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? (uint32_t)p : 0x80000000u + lane);
-        const uint32_t leader = (uint32_t)__ffs((int)peers) - 1u;
         const int32_t rv = ri >= 0 ? __ldcg(release_of + ri) : -1;
-        const uint32_t rpeers = __match_any_sync(0xffffffffu, rv >= 0 ? (uint32_t)rv : 0x80000000u + lane);
         // releases by page name pages outside the table's range as bad here
         const bool rin = rv >= 0 && (!BYPAGE || (uint32_t)rv < b.n_logical);
-        if (BYPAGE && rv >= 0 && !rin && (uint32_t)(__ffs((int)rpeers) - 1) == lane) bad += (uint32_t)__popc(rpeers);
+        if (BYPAGE && rv >= 0 && !rin) ++bad;
         __syncthreads();   // tables clear
         SweepWin w0{};
         if (!DIST) {
@@ -600,10 +600,9 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
             w0.q = __ldcg(b.frame_page + w0.f);
         }
         uint32_t fslot = kMergeEmpty, rslot = kMergeEmpty;
-        if (valid && lane == leader) fslot = merge_insert<KEYS>(t.fkey, t.fcnt, (uint32_t)p, (uint32_t)__popc(peers));
-        if (rin && (uint32_t)(__ffs((int)rpeers) - 1) == lane)
-            rslot = BYPAGE ? merge_insert<KEYS>(t.fkey, t.frel, (uint32_t)rv, (uint32_t)__popc(rpeers))
-                           : merge_insert<KEYS>(t.rkey, t.rcnt, (uint32_t)rv, (uint32_t)__popc(rpeers));
+        if (valid) fslot = merge_insert<KEYS>(t.fkey, t.fcnt, (uint32_t)p);
+        if (rin)
+            rslot = BYPAGE ? merge_insert<KEYS>(t.fkey, t.frel, (uint32_t)rv) : merge_insert<KEYS>(t.rkey, t.rcnt, (uint32_t)rv);
         __syncthreads();   // counts complete
         if (!DIST) w0.e = w0.q < b.n_logical ? __ldcg(b.pt + w0.q) : 0ull;
         // the page's fetch leader moves the block's pins of it with one atomic
@@ -674,9 +673,8 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
         }
         if (lead) t.fres[fs] = f;
         __syncthreads();   // results in the table
-        const uint32_t my_slot = __shfl_sync(0xffffffffu, fslot, (int)leader) & ~kMergeFirst;
         if (i < n) {
-            const int32_t got = valid ? t.fres[my_slot] : -1;
+            const int32_t got = valid ? t.fres[fs] : -1;
             frames_out[i] = got;
             if (held_out) held_out[i] = got >= 0 ? p : -1;
         }
@@ -687,8 +685,8 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
 // A round of releases only (no fetch): the block's releases of one name meet
 // in a shared-memory table and go as one atomic, and no sweep runs, so the hand
 // stays where it is.  BYPAGE as for k_round.  Merged within the warp only, the
-// hottest page's entry took an atomic from nearly every warp: 471,000 releases of a
-// Zipf(0.99) stream took REL_NOTE us.
+// hottest page's entry took an atomic from nearly every warp (471,000 releases of a
+// Zipf(0.99) stream: 46 us, 17 merged over the block).
 constexpr int kReleaseItems = 2;   // per thread, their reads in flight together
 
 template <bool BYPAGE>
@@ -698,7 +696,6 @@ __global__ void __launch_bounds__(256) k_release(BmView b, const int32_t* releas
     constexpr uint32_t KEYS = 256u * kReleaseItems;
     __shared__ uint32_t keys[2 * KEYS], cnt[2 * KEYS];
     unsigned long long ok = 0, bad = 0;
-    const uint32_t lane = threadIdx.x & 31u;
     const uint64_t base = (uint64_t)blockIdx.x * (256u * kReleaseItems) + threadIdx.x;
     int32_t rv[kReleaseItems];
 #pragma unroll
@@ -718,10 +715,8 @@ __global__ void __launch_bounds__(256) k_release(BmView b, const int32_t* releas
 #pragma unroll
     for (int u = 0; u < kReleaseItems; ++u) {
         const bool have = base + (uint64_t)u * 256u < n_release && rv[u] >= 0;
-        const uint32_t peers = __match_any_sync(0xffffffffu, have ? (uint32_t)rv[u] : 0x80000000u + lane);
         slot[u] = kMergeEmpty;
-        if (have && (uint32_t)(__ffs((int)peers) - 1) == lane)
-            slot[u] = merge_insert<KEYS>(keys, cnt, (uint32_t)rv[u], (uint32_t)__popc(peers));
+        if (have) slot[u] = merge_insert<KEYS>(keys, cnt, (uint32_t)rv[u]);
     }
     __syncthreads();   // counts complete
 #pragma unroll
