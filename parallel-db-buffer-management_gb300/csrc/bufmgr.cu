@@ -541,10 +541,9 @@ __device__ __forceinline__ uint32_t merge_insert(uint32_t* keys, uint32_t* cnt, 
 // The many-thread round.  Per block iteration every lane takes release i
 // and fetch i (i = the block's base + threadIdx.x); equal keys meet in the
 // block's tables, and each key's leader issues its atomic: the fetch's pin (with
-// the block's releases of the page,
-// releasing by page), and other releases while the pins are in flight.  The
-// fetch's result goes back through the table to every lane that asked for
-// the page.  With the single hand each warp also takes and examines its
+// the block's releases of the page, releasing by page), and other releases while
+// the pins are in flight.  The fetch's result goes back through the table to every
+// lane that asked for the page.  With the single hand each warp also takes and examines its
 // first sweep window while its pins are in flight: nearly every warp has a
 // miss, and one that has none has still moved the hand over 32 frames as a
 // sweep does (clearing reference bits, evicting nothing).  Releases of one
