@@ -147,36 +147,48 @@ __device__ __forceinline__ void* malloc_group(const MallocView& m, uint32_t acti
     return out;
 }
 
-// Free of one block per calling lane (nullptr = nothing).  Lanes freeing
-// blocks of the same run merge their decrements; the decrement that reaches
-// zero releases the run.  Returns false for a pointer outside the pool or a
-// run with no live block (double free), which is then left untouched.
-__device__ __forceinline__ bool free_group(const MallocView& m, uint32_t active, const void* ptr) {
-    const uint32_t lane = threadIdx.x & 31u;
-    int32_t run = -1;
-    bool ok = true;
-    if (ptr) {
-        const char* p = (const char*)ptr;
-        const size_t span = (size_t)m.pool.n_pages << m.page_shift;
-        if (p < m.pool.base || (size_t)(p - m.pool.base) >= span) {
-            ok = false;
-        } else {
-            const int32_t pg = (int32_t)((size_t)(p - m.pool.base) >> m.page_shift);
-            run = __ldcg(m.start_of + pg);
-        }
+// The run that holds a block: its first page, or -1 (no block, or `ok` = false: the
+// pointer lies outside the pool).
+__device__ __forceinline__ int32_t run_of_block(const MallocView& m, const void* ptr, bool& ok) {
+    ok = true;
+    if (!ptr) return -1;
+    const char* p = (const char*)ptr;
+    const size_t span = (size_t)m.pool.n_pages << m.page_shift;
+    if (p < m.pool.base || (size_t)(p - m.pool.base) >= span) {
+        ok = false;
+        return -1;
     }
+    return __ldcg(m.start_of + ((size_t)(p - m.pool.base) >> m.page_shift));
+}
+
+// Takes one block per calling lane off its run (run < 0: none).  Lanes whose blocks
+// share a run merge their decrements; the decrement that reaches zero releases
+// the run.  Returns false for a run with no live block (double free), which is
+// left untouched.
+__device__ __forceinline__ bool release_run(const MallocView& m, uint32_t active, int32_t run) {
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t peers = __match_any_sync(active, (uint32_t)run);
+    bool ok = true;
     if (run >= 0 && (__ffs((int)peers) - 1) == (int)lane) {
         const int32_t k = __popc(peers);
+        const uint32_t len = __ldcg(m.len_of + run);   // read beside the count, not after it
         const int32_t old = atomicSub(m.live + run, k);
         if (old == k) {
-            free_span(m.pool, run, m.len_of[run]);
+            free_span(m.pool, run, len);
         } else if (old < k) {
             atomicAdd(m.live + run, k);   // double free: undo, report
             ok = false;
         }
     }
-    return __shfl_sync(active, ok ? 1 : 0, lane) != 0;
+    return ok;
+}
+
+// Free of one block per calling lane (nullptr = nothing).  Returns false for a
+// pointer outside the pool or a double free.
+__device__ __forceinline__ bool free_group(const MallocView& m, uint32_t active, const void* ptr) {
+    bool ok;
+    const int32_t run = run_of_block(m, ptr, ok);
+    return release_run(m, active, run) && ok;
 }
 
 #endif  // __CUDACC__

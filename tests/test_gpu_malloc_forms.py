@@ -63,6 +63,49 @@ def test_blocks_are_disjoint_and_come_back(cuda, pbm_mod, n_groups, backend, for
     pool.close()
 
 
+def test_batch_large_enough_for_paired_rounds(cuda, pbm_mod):
+    """More requests than 64 for every warp of the launch, in groups that end inside a chunk, mallocs and
+    frees in one batch: all served, blocks disjoint, everything back at the end."""
+    torch, pbm = cuda, pbm_mod
+    T, page = 1 << 18, 4096
+    rng = np.random.default_rng(1)
+    counts = rng.integers(900, 2000, 256)
+    n = int(counts.sum())
+    pool = pbm.Pool(T, page, materialize=True)
+    pool.malloc_init()
+    sizes_h = np.exp(rng.uniform(np.log(16), np.log(4096), 2 * n)).astype(np.int32)
+    sizes = torch.from_numpy(sizes_h).cuda()
+    ptrs = torch.zeros(2 * n, dtype=torch.int64, device="cuda")
+
+    def table(op, offset):
+        t = np.zeros(256, dtype=[("op", "<i4"), ("count", "<u4"), ("offset", "<u8")])
+        t["op"], t["count"] = op, counts
+        t["offset"] = offset + np.concatenate([[0], np.cumsum(counts)[:-1]])
+        return t
+
+    def step(tables):
+        t = np.concatenate(tables)
+        if len(tables) == 2:                           # mallocs and frees by turns
+            t = t.reshape(2, -1).T.reshape(-1)
+        d = torch.from_numpy(np.ascontiguousarray(t).view(np.uint8).copy()).cuda()
+        pool.malloc_batch(d, None, len(t), sizes, ptrs, 2 * n, 3, pbm.LAUNCH_PERSISTENT)
+
+    step([table(pbm.OP_MALLOC, 0)])
+    step([table(pbm.OP_MALLOC, n), table(pbm.OP_MFREE, 0)])
+    p = ptrs.cpu().numpy()
+    assert not p[:n].any() and p[n:].all()
+    blk = np.maximum(16, 1 << np.ceil(np.log2(sizes_h[n:])).astype(np.int64))
+    off = p[n:] - pool.base_ptr
+    assert (off >= 0).all() and (off + blk <= T * page).all()
+    order = np.argsort(off)
+    assert (off[order][1:] >= (off + blk)[order][:-1]).all()
+    step([table(pbm.OP_MFREE, n)])
+    assert not ptrs.any() and pool.used() == 0 and pool.malloc_counts() == (0, 0)
+    s = pool.stats()
+    assert (s.successes, s.failures, s.frees) == (2 * n, 0, 2 * n)
+    pool.close()
+
+
 def test_runs_found_by_a_sharing_warp_are_free_runs(cuda, pbm_mod, orc):
     """A nearly full pool, so most walks of a warp go on together for many rounds: every run
     granted was free, lies inside the pool and overlaps no other, and the failures took max_steps."""
