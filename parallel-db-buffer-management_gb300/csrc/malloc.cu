@@ -454,17 +454,14 @@ int pbm_malloc_init(pbm_pool* pool) {
     if (!t) return PBM_ERR_NOMEM;
     if (t->start_of) return PBM_OK;
     const size_t n = pool->n_pages;
-    if (cudaMalloc(&t->start_of, n * 4) != cudaSuccess || cudaMalloc(&t->live, n * 4) != cudaSuccess ||
-        cudaMalloc(&t->len_of, n) != cudaSuccess) {
+    if (cudaMalloc(&t->start_of, n * 9) != cudaSuccess) {   // the three tables, one allocation
         cudaGetLastError();
-        cudaFree(t->start_of);
-        cudaFree(t->live);
         t->start_of = nullptr;
-        t->live = nullptr;
-        t->len_of = nullptr;
         drop_if_empty(pool);
         return PBM_ERR_NOMEM;
     }
+    t->live = t->start_of + n;
+    t->len_of = reinterpret_cast<uint8_t*>(t->live + n);
     k_malloc_init<<<sm_count() * 4, 256>>>(t->start_of, t->live, t->len_of, (uint32_t)n);
     PBM_LAUNCH_CHECK();
     PBM_CUDA_TRY(cudaDeviceSynchronize());
@@ -488,9 +485,7 @@ int pbm_malloc_release(pbm_pool* pool) {
     MallocTables* t = tables_of(pool);
     if (!t) return PBM_ERR_INVALID;
     cudaDeviceSynchronize();
-    cudaFree(t->start_of);
-    cudaFree(t->live);
-    cudaFree(t->len_of);
+    cudaFree(t->start_of);   // and live, len_of behind it
     t->start_of = nullptr;
     t->live = nullptr;
     t->len_of = nullptr;

@@ -416,19 +416,9 @@ using namespace pbm;
 
 static void pool_free_all(pbm_pool* p) {
     if (!p) return;
-    cudaFree(p->d_words);
+    cudaFree(p->d_words);   // and all that lies behind it
     cudaFree(p->d_base);
-    cudaFree(p->d_stats);
-    cudaFree(p->d_cursors);
-    cudaFree(p->d_arms);
-    cudaFree(p->d_arm);
     cudaFree(p->d_ring);
-    cudaFree(p->d_fifo);
-    cudaFree(p->d_seen);
-    cudaFree(p->d_check);
-    cudaFree(p->d_budget);
-    cudaFree(p->d_budget_blocks);
-    cudaFree(p->d_scan);
     cudaFree(p->d_prefix);
     delete p;
 }
@@ -489,17 +479,35 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
     p->budget_blocks = (uint32_t)std::min<uint64_t>((uint64_t)sm_count() * kBudgetPerSm,
                                                  (nw64 + kBudgetThreads - 1u) / kBudgetThreads);
     p->list_cap = std::max<uint64_t>(1024u, cfg->n_pages / 2u);
-    bool ok = cudaMalloc(&p->d_words, p->bitmap_bytes) == cudaSuccess &&
-              cudaMalloc(&p->d_stats, sizeof(DevStats)) == cudaSuccess &&
-              cudaMalloc(&p->d_cursors, sizeof(int32_t) * p->max_slots) == cudaSuccess &&
-              cudaMalloc(&p->d_arms, sizeof(uint32_t) * p->max_slots) == cudaSuccess &&
-              cudaMalloc(&p->d_arm, sizeof(unsigned long long)) == cudaSuccess &&
-              cudaMalloc(&p->d_fifo, sizeof(FifoState)) == cudaSuccess &&
-              cudaMalloc(&p->d_seen, p->bitmap_bytes) == cudaSuccess &&
-              cudaMalloc(&p->d_check, sizeof(CheckCounters)) == cudaSuccess &&
-              cudaMalloc(&p->d_budget, sizeof(LaunchBudget)) == cudaSuccess &&
-              cudaMalloc(&p->d_budget_blocks, sizeof(unsigned long long) * p->budget_blocks) == cudaSuccess &&
-              cudaMalloc(&p->d_scan, sizeof(unsigned long long) * nb_scan) == cudaSuccess;
+    // everything but the page memory and the free list in one allocation, the bitmap first
+    size_t at = 0;
+    auto place = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255u) & ~(size_t)255u;
+        return o;
+    };
+    const size_t o_words = place(p->bitmap_bytes), o_seen = place(p->bitmap_bytes);
+    const size_t o_cursors = place(sizeof(int32_t) * p->max_slots), o_arms = place(sizeof(uint32_t) * p->max_slots);
+    const size_t o_stats = place(sizeof(DevStats)), o_arm = place(sizeof(unsigned long long));
+    const size_t o_fifo = place(sizeof(FifoState)), o_check = place(sizeof(CheckCounters));
+    const size_t o_budget = place(sizeof(LaunchBudget));
+    const size_t o_budget_blocks = place(sizeof(unsigned long long) * p->budget_blocks);
+    const size_t o_scan = place(sizeof(unsigned long long) * nb_scan);
+    char* all = nullptr;
+    bool ok = cudaMalloc(&all, at) == cudaSuccess;
+    if (ok) {
+        p->d_words = reinterpret_cast<uint32_t*>(all + o_words);
+        p->d_seen = reinterpret_cast<uint32_t*>(all + o_seen);
+        p->d_cursors = reinterpret_cast<int32_t*>(all + o_cursors);
+        p->d_arms = reinterpret_cast<uint32_t*>(all + o_arms);
+        p->d_stats = reinterpret_cast<DevStats*>(all + o_stats);
+        p->d_arm = reinterpret_cast<unsigned long long*>(all + o_arm);
+        p->d_fifo = reinterpret_cast<FifoState*>(all + o_fifo);
+        p->d_check = reinterpret_cast<CheckCounters*>(all + o_check);
+        p->d_budget = reinterpret_cast<LaunchBudget*>(all + o_budget);
+        p->d_budget_blocks = reinterpret_cast<unsigned long long*>(all + o_budget_blocks);
+        p->d_scan = reinterpret_cast<unsigned long long*>(all + o_scan);
+    }
     if (ok && (cfg->flags & PBM_POOL_MATERIALIZE)) {
         ok = cudaMalloc(&p->d_base, (size_t)cfg->n_pages * cfg->page_size) == cudaSuccess;
     }
