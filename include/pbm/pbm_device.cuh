@@ -1038,16 +1038,20 @@ __device__ __forceinline__ int32_t walk_span(const PoolView& v, uint32_t n, int3
 // lane first takes kOwnJumps jumps of its own (all in parallel; one, two, three:
 // 30,000 runs of 1..8 pages and their frees on 2^18 pages took 19.8, 14.6, 13.3 us, 20,000
 // of 1..32 on 2^20 pages 22.2, 22.9, 23.3).  The walks still unserved
-// then share the warp: with m of them each gets 2^floor(log2(32 / m)) lanes, lane j
-// of a walk judging its jump s + j + 1 (its LCG state advanced j + 1 steps at once),
-// and the runs found are claimed in jump order, the walks side by side.  In a run
-// without races a lane gets the page the one-lane walk would give it, after
-// the same jumps; a walk that keeps missing alone costs max_steps / 32 rounds
-// instead of max_steps jumps.  (One walk at a time with all 32 lanes took a round of
-// two round trips per unserved walk.  Measured on GB300, mallocs of 16 B .. 64 KiB and
-// their frees: 524,288 into 2^22 pages 62 -> 58 us, 192,155 into 1.5 M pages 48 -> 33 us.)
+// then share the warp for kShareRounds rounds: with m of them each gets
+// 2^floor(log2(32 / m)) lanes, lane j of a walk judging its jump s + j + 1 (its LCG
+// state advanced j + 1 steps at once), and the runs found are claimed in jump order, the
+// walks side by side.  Those that are left look for runs that are rare, in a pool that is
+// nearly full, and are walked one after the other with all lanes and kSpanWide jumps a
+// lane in flight.  In a run without races a lane gets the page the one-lane walk would
+// give it, after the same jumps.  Measured on GB300: mallocs of 16 B .. 64 KiB and their
+// frees, 524,288 into 2^22 pages, one walk at a time 62 us, sharing 58; 192,155 into
+// 1.5 M pages 48 and 33; but the malloc trace that outgrows its pool, where a quarter of
+// the requests fail after 512 jumps, 5.1 and 4.6 G ops/s, and 6.2 with both.
 // The whole warp calls converged.
 constexpr uint32_t kOwnJumps = 2;
+constexpr uint32_t kShareRounds = 3;
+constexpr uint32_t kSpanWide = 2;
 
 __device__ __forceinline__ int32_t walk_span_warp(const PoolView& v, uint32_t need_n, int32_t seed0,
                                                   uint32_t max_steps, int32_t* steps_out) {
@@ -1071,7 +1075,7 @@ __device__ __forceinline__ int32_t walk_span_warp(const PoolView& v, uint32_t ne
     uint32_t pend = __ballot_sync(kFull32, need_n > 0u && id < 0 && s < max_steps);
     uint32_t aj = 0u, cj = 0u;                             // jump ahead by lane + 1 steps
     if (pend) lcg_jump<6>(lane + 1u, aj, cj);
-    while (pend) {
+    for (uint32_t round = 0; pend && round < kShareRounds; ++round) {
         const uint32_t m = (uint32_t)__popc(pend);
         const uint32_t sh = (uint32_t)__clz((int)(m - 1u)) - 27u;   // floor(log2(32 / m)): clz(0) is 32
         const uint32_t j = lane & ((1u << sh) - 1u);
@@ -1111,6 +1115,49 @@ __device__ __forceinline__ int32_t walk_span_warp(const PoolView& v, uint32_t ne
             if (low <= last) id = fs;
         }
         pend = __ballot_sync(kFull32, need_n > 0u && id < 0 && s < max_steps);
+    }
+    // the walks that are left, in a pool where their runs are rare: one after the other with the
+    // whole warp, kSpanWide jumps a lane in flight
+    while (pend) {
+        const int l0 = __ffs((int)pend) - 1;
+        uint32_t x0 = (uint32_t)__shfl_sync(kFull32, x, l0);
+        const uint32_t n0 = __shfl_sync(kFull32, need_n, l0);
+        uint32_t s0 = __shfl_sync(kFull32, s, l0);
+        int32_t got = -1;
+        while (got < 0 && s0 < max_steps) {
+            uint32_t wj[kSpanWide], a0[kSpanWide], a1[kSpanWide];
+#pragma unroll
+            for (uint32_t u = 0; u < kSpanWide; ++u) {
+                const uint32_t xj = (aj * x0 + cj) & 0x7fffffffu;      // jump s0 + 32 u + lane + 1
+                x0 = __shfl_sync(kFull32, xj, 31);
+                wj[u] = idx_hi((int32_t)xj, L);
+                const bool in = 32u * u + lane < max_steps - s0;
+                a0[u] = in ? load_word(v.words + wj[u]) : kFull32;
+                a1[u] = in && wj[u] + 1u < L ? load_word(v.words + wj[u] + 1u) : kFull32;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kSpanWide; ++u) {
+                if (got >= 0) break;
+                const int32_t fj = span_in_pair(wj[u], a0[u], a1[u], n0, L);
+                uint32_t open = __ballot_sync(kFull32, fj >= 0);
+                while (open) {                                         // claims in jump order
+                    const int j = __ffs((int)open) - 1;
+                    open &= open - 1u;
+                    const bool ok = (int)lane == j && claim_pair(v, (uint32_t)fj, n0);
+                    if (__any_sync(kFull32, ok)) {
+                        got = __shfl_sync(kFull32, fj, j);
+                        s0 += 32u * u + (uint32_t)j + 1u;
+                        break;
+                    }
+                }
+            }
+            if (got < 0) s0 = max_steps - s0 < 32u * kSpanWide ? max_steps : s0 + 32u * kSpanWide;
+        }
+        if ((int)lane == l0) {
+            id = got;
+            s = s0;
+        }
+        pend &= pend - 1u;
     }
     if (steps_out) *steps_out = (int32_t)s;
     return id;

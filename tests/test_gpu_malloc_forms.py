@@ -133,3 +133,34 @@ def test_runs_found_by_a_sharing_warp_are_free_runs(cuda, pbm_mod, orc):
     s = pool.stats()
     assert s.failures == int((~ok).sum()) and s.steps >= 300 * s.failures
     pool.close()
+
+
+@pytest.mark.parametrize("backend", ["runs", "queue"])
+@pytest.mark.parametrize("max_steps", [1, 2, 40, 97, 512])
+def test_overfull_pool_fails_within_the_bound(cuda, pbm_mod, backend, max_steps):
+    """Many more pages asked for than there are: every request ends, after at most max_steps jumps, served
+    ones hold blocks of their own, and freeing gives every page back."""
+    torch, pbm = cuda, pbm_mod
+    T, page, n = 4096, 4096, 3000
+    pool = pbm.Pool(T, page, materialize=True)
+    getattr(pool, "malloc_init" if backend == "runs" else "qmalloc_init")()
+    rng = np.random.default_rng(5)
+    npg = rng.choice([1, 2, 4, 8, 16], n)
+    sizes = torch.from_numpy((npg * page).astype(np.int32)).cuda()
+    ptrs = torch.zeros(n, dtype=torch.int64, device="cuda")
+    run = getattr(pool, "malloc_batch" if backend == "runs" else "qmalloc_batch")
+    run(_table(torch, pbm.OP_MALLOC, np.array([n])), None, 1, sizes, ptrs, n, 3, pbm.LAUNCH_PERSISTENT,
+        max_steps=max_steps)
+    p = ptrs.cpu().numpy()
+    ok = p != 0
+    first = (p[ok] - pool.base_ptr) // page
+    cover = np.zeros(T, dtype=np.int32)
+    for f, k in zip(first, npg[ok]):
+        cover[f:f + k] += 1
+    assert cover.max() == 1 and pool.used() == cover.sum()
+    s = pool.stats()
+    assert (s.successes, s.failures) == (int(ok.sum()), int((~ok).sum())) and s.failures > 0
+    assert s.steps <= max_steps * n and s.steps >= max_steps * s.failures
+    run(_table(torch, pbm.OP_MFREE, np.array([n])), None, 1, sizes, ptrs, n, 4, pbm.LAUNCH_PERSISTENT)
+    assert not ptrs.any() and (pool.used() == 0 if backend == "runs" else pool.qmalloc_counts()[2:] == (0, 0, 0))
+    pool.close()
