@@ -485,10 +485,14 @@ int check_cfg(const pbm_walk_config* c) {
 // Blocks for `threads` threads of work, at most what the SMs hold at once: the
 // kernels loop over the rest.  For kernels with little work per request, where
 // block starts and the counter atomic of each block's end were a good part
-// of the launch (the collaborative walk of 2^20 requests: 22.6 -> 15 us).  The
-// per-thread walks keep one block per 256 requests: their length varies, and
-// blocks started as others end even it out (2^20 word probes at 50%: 32.4 us, 34.4
-// with the grid cut).
+// of the launch (the collaborative walk of 2^20 requests: 22.6 -> 15 us).
+// For the per-thread walks it is two such grids: their length varies, and blocks that
+// start as others end even it out (2^22 word probes at 50%: 102 us, 106 with one grid,
+// 128 with a block per 256 requests and a counter flush that is dear; 2^22 page walks
+// 171, 171, 190).  Behind a budget one grid is enough, most requests being answered by
+// it: 2^22 page walks at 90% fail-fast 124 -> 31 us, word probes 108 -> 30.
+constexpr int kThreadBlocks = 16 * 256, kListedBlocks = 8 * 256;
+
 int capped_grid(uint64_t threads, int block, int per_sm) {
     const uint64_t need = (threads + (uint64_t)block - 1u) / (uint64_t)block;
     const uint64_t fit = (uint64_t)sm_count() * (uint64_t)(per_sm / block > 0 ? per_sm / block : 1);
@@ -530,7 +534,7 @@ int launch_alloc(pbm_pool* p, const pbm_walk_config* c, const AllocArgs& a, bool
     const int W = c->collab_width ? c->collab_width : 32;
     const bool w64 = c->word_bits == 64;
     int block = serial ? 1 : block_cfg;
-    const int grid = serial ? 1 : (int)((a.n + (uint32_t)block - 1u) / (uint32_t)block);
+    const int grid = serial ? 1 : capped_grid(a.n, block, a.budget ? kListedBlocks : kThreadBlocks);
     switch (c->strategy) {
     case PBM_RANDOM_WALK:
         launch_next(k_alloc_thread<Walk::Page>, grid, block, 0, s, a);
@@ -560,10 +564,11 @@ int launch_alloc(pbm_pool* p, const pbm_walk_config* c, const AllocArgs& a, bool
             int rc = fifo_build(p, s);
             if (rc) return rc;
         }
+        const int blocks = serial ? 1 : (int)((a.n + (uint32_t)block - 1u) / (uint32_t)block);
         if (serial || a.n < (uint32_t)(sm_count() * block * kFifoItems))
-            launch_next(k_fifo_alloc<1>, grid, block, 0, s, a, p->d_fifo, p->d_ring);
+            launch_next(k_fifo_alloc<1>, blocks, block, 0, s, a, p->d_fifo, p->d_ring);
         else
-            launch_next(k_fifo_alloc<kFifoItems>, (grid + kFifoItems - 1) / kFifoItems, block, 0, s, a, p->d_fifo, p->d_ring);
+            launch_next(k_fifo_alloc<kFifoItems>, (blocks + kFifoItems - 1) / kFifoItems, block, 0, s, a, p->d_fifo, p->d_ring);
         break;
     }
     default:
