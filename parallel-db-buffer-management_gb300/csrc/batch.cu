@@ -388,8 +388,14 @@ int persistent_blocks_per_sm(int block) {
 // >= kCappedBlocks: the variant whose registers are capped for kCappedBlocks
 // resident blocks (5 x 256 threads: at most 51 registers, no spills for the
 // collaborative walk on 32-bit words).
+// The page walk has the capped registers always: its look-ahead needs 70 otherwise, three
+// blocks an SM (swaps of 2^24 pages at 50 / 75 / 90 / 95% with them: 39 / 28 / 19 / 12.7 G
+// operations/s; capped for four blocks 47 / 32 / 20 / 14.3, five 51 / 33 / 20 / 14.4, six
+// 51 / 33 / 20 / 14.0, eight 46 / 31 / 19 / 13.7).
 // grid_cap > 0: at most that many blocks (a batch whose size the host knows
 // and that needs fewer blocks than fill the GPU).
+template <BWalk K> constexpr int kUncapped = K == BWalk::Page ? kCappedBlocks : 1;
+
 template <BWalk K, int W, typename Word, typename Tab, typename SlotT>
 void launch_persistent_slots(const BatchArgs& a, const Tab& tab, int block, int blocks_per_sm, size_t smem,
                              cudaStream_t s, unsigned grid_cap, bool captured) {
@@ -403,10 +409,10 @@ void launch_persistent_slots(const BatchArgs& a, const Tab& tab, int block, int 
         launch_next_if(!captured, k_batch_persistent<K, W, Word, kCappedBlocks, Tab, SlotT>, grid_of(per_sm),
                        (unsigned)block, smem, s, a, tab);
     } else {
-        int fit = persistent_blocks_per_sm<K, W, Word, 1, Tab, SlotT>(block);
+        int fit = persistent_blocks_per_sm<K, W, Word, kUncapped<K>, Tab, SlotT>(block);
         int per_sm = (blocks_per_sm > 0 && blocks_per_sm < fit) ? blocks_per_sm : fit;
-        launch_next_if(!captured, k_batch_persistent<K, W, Word, 1, Tab, SlotT>, grid_of(per_sm), (unsigned)block, smem, s,
-                       a, tab);
+        launch_next_if(!captured, k_batch_persistent<K, W, Word, kUncapped<K>, Tab, SlotT>, grid_of(per_sm),
+                       (unsigned)block, smem, s, a, tab);
     }
 }
 
@@ -488,7 +494,7 @@ int resolve_blocks_per_sm(const pbm_walk_config* c, unsigned long long arena_len
         return (c->blocks_per_sm > 0 && c->blocks_per_sm < fit1) ? c->blocks_per_sm : fit1;
     };
 #define PBM_FITS(K, W, T) \
-    pick(persistent_blocks_per_sm<K, W, T, 1>(block), persistent_blocks_per_sm<K, W, T, kCappedBlocks>(block))
+    pick(persistent_blocks_per_sm<K, W, T, kUncapped<K>>(block), persistent_blocks_per_sm<K, W, T, kCappedBlocks>(block))
     switch (c->strategy) {
     case PBM_RANDOM_WALK: return PBM_FITS(BWalk::Page, 32, uint32_t);
     case PBM_RANDOM_WALK_BM:
