@@ -403,20 +403,20 @@ __device__ __forceinline__ void bulk_stores_done() {
 // store with the whole warp, then publish the entries.  The warp's copies are a run
 // of pieces (loader by loader) of at most kCopyPiece bytes; a lane brings one
 // piece at a time into its own slot of the warp's staging buffer with one bulk load and
-// sends it to the frame with one bulk store, so a warp has kCopyStage bytes
+// sends it to the frame with one bulk store, so a warp has as many bytes as its buffer
 // in flight with two instructions per piece.  Copying through registers, four 16-byte
 // loads per lane, kept 2 KiB per warp in flight: a round of 16,384 fetches (30%
 // misses) of 4 KiB pages took 41 us, 18 this way (6 of them here, 3.5 TB/s read).  The
 // whole warp calls converged.
 constexpr uint32_t kCopyPiece = 4096;
-constexpr uint32_t kCopyStage = 32768;   // per warp
+constexpr uint32_t kCopyStage = 32768;   // per warp, at most
 
 __host__ __device__ __forceinline__ uint32_t copy_piece(uint32_t frame_size) {
     return frame_size < kCopyPiece ? frame_size : kCopyPiece;
 }
-// Pieces a warp has in flight: one slot per lane at most.
-__host__ __device__ __forceinline__ uint32_t copy_slots(uint32_t frame_size) {
-    const uint32_t s = kCopyStage / copy_piece(frame_size);
+// Pieces a warp with a staging buffer of so many bytes has in flight: one slot per lane at most.
+inline uint32_t copy_slots(uint32_t frame_size, uint32_t stage) {
+    const uint32_t s = stage / copy_piece(frame_size);
     return s < 32u ? s : 32u;
 }
 
@@ -424,6 +424,7 @@ struct CopyStage {
     uint32_t buf;      // this lane's slot (shared address)
     uint32_t bar;      // its barrier
     uint32_t parity;   // of the barrier's next completion
+    uint32_t slots;    // slots of the warp's buffer
 };
 
 template <bool COPY>
@@ -432,7 +433,7 @@ __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs
     if (COPY) {
         const uint32_t lane = threadIdx.x & 31u;
         const uint32_t todo = __ballot_sync(0xffffffffu, loader && h >= 0);
-        const uint32_t slots = copy_slots(b.frame_size), piece = copy_piece(b.frame_size);
+        const uint32_t slots = cs.slots, piece = copy_piece(b.frame_size);
         const uint32_t per = (b.frame_size + piece - 1u) / piece;          // pieces per page
         const uint32_t total = (uint32_t)__popc(todo) * per;
         for (uint32_t base = 0; base < total; base += slots) {
@@ -553,8 +554,8 @@ __device__ __forceinline__ uint32_t merge_insert(uint32_t* keys, uint32_t* cnt, 
 template <bool DIST, bool BYPAGE, bool COPY, int BLOCK>
 __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* release_of, const int32_t* release_idx,
                                              uint32_t n_release, const int32_t* pages, uint32_t n, uint32_t slot0,
-                                             int32_t* frames_out, int32_t* held_out, unsigned long long& ok,
-                                             unsigned long long& bad, BmAcc& acc) {
+                                             int32_t* frames_out, int32_t* held_out, uint32_t slots,
+                                             unsigned long long& ok, unsigned long long& bad, BmAcc& acc) {
     constexpr uint32_t KEYS = 2u * BLOCK;   // BLOCK fetches and BLOCK releases
     __shared__ MergeTables<KEYS, !BYPAGE> t;
     __shared__ uint32_t s_hand;   // the block's first sweep windows
@@ -563,7 +564,8 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
     if constexpr (COPY) {
         extern __shared__ __align__(128) unsigned char stage[];
         __shared__ unsigned long long bars[BLOCK];
-        const uint32_t piece = copy_piece(b.frame_size), slots = copy_slots(b.frame_size);
+        const uint32_t piece = copy_piece(b.frame_size);
+        cs.slots = slots;
         cs.buf = smem_addr(stage) + ((threadIdx.x >> 5) * slots + (lane < slots ? lane : 0u)) * piece;
         cs.bar = smem_addr(bars + threadIdx.x);
         mbar_init(cs.bar);
@@ -739,7 +741,7 @@ __global__ void __launch_bounds__(256) k_release(BmView b, const int32_t* releas
 template <bool DIST, bool BYPAGE, bool COPY, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_round(BmView b, const int32_t* release_of, const int32_t* release_idx,
                                                uint32_t n_release, const int32_t* pages, uint32_t n, uint32_t slot0,
-                                               int32_t* frames_out, int32_t* held_out) {
+                                               int32_t* frames_out, int32_t* held_out, uint32_t slots) {
     stream_wait();
     unsigned long long ok = 0, bad = 0;
     BmAcc acc;
@@ -759,8 +761,8 @@ __global__ void __launch_bounds__(BLOCK) k_round(BmView b, const int32_t* releas
             if (held_out) held_out[i] = f >= 0 ? p : -1;
         }
     } else {
-        round_blocks<DIST, BYPAGE, COPY, BLOCK>(b, release_of, release_idx, n_release, pages, n, slot0, frames_out, held_out, ok,
-                                   bad, acc);
+        round_blocks<DIST, BYPAGE, COPY, BLOCK>(b, release_of, release_idx, n_release, pages, n, slot0, frames_out, held_out, slots,
+                                                ok, bad, acc);
     }
     block_add_counters<7>({ok, bad, acc.hits, acc.misses, acc.evictions, acc.failures, acc.timeouts},
                           {&b.stats->unpins, &b.stats->bad_unpins, &b.stats->hits, &b.stats->misses,
@@ -914,7 +916,7 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     }
     // Blocks of 64 threads for rounds that would not give every SM two blocks of 256 (a
     // round of 16,384 fetches is 64 such blocks), and for rounds that copy, whose
-    // staging buffers (32 KiB a warp) are then shared out in small blocks.  A larger round
+    // staging buffers are then shared out in small blocks.  A larger round
     // that copies nothing merges its requests over 256 threads, over 128 with private
     // hands, whose kernel has 78 registers (eight rounds of 131,072 and 262,144 fetches, blocks of
     // 64 / 128 / 256: 150 / 135 / 127 and 246 / 226 / 219 us with the single hand, 183 / 168 / 184
@@ -923,12 +925,18 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     const bool small = copy || work < (uint32_t)sm_count() * 512u;
     const int block = serial ? 1 : small ? 64 : m->v.dist ? 128 : 256;
     const int grid = serial ? 1 : (int)(((uint64_t)work + (uint32_t)block - 1u) / (uint32_t)block);
-    const size_t stage = copy && !serial ? 2u * (size_t)copy_slots(m->v.frame_size) * copy_piece(m->v.frame_size) : 0u;
+    // Three blocks with full staging buffers fit an SM.  A copying round of more blocks than
+    // that has half the buffer, and twice the blocks at once (rounds of 16,384 / 24,000 /
+    // 32,768 / 65,536 / 131,072 fetches of 4 KiB, single hand: 125 / 147 / 204 / 323 / 548 us
+    // with the full one, 131 / 151 / 173 / 298 / 488 with half; private hands from 32,768:
+    // 241 / 383 / 683 and 194 / 340 / 563).
+    const uint32_t slots = copy ? copy_slots(m->v.frame_size, grid > 3 * sm_count() ? kCopyStage / 2u : kCopyStage) : 0u;
+    const size_t stage = copy && !serial ? 2u * (size_t)slots * copy_piece(m->v.frame_size) : 0u;
     cudaError_t attr = cudaSuccess;
     auto go = [&](auto kernel) {
         if (stage) attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)kCopyStage);
         if (attr == cudaSuccess)
-            launch_next(kernel, grid, block, stage, s, m->v, d_release_of, d_release_idx, n_release, d_pages, n, slot0, d_frames_out, d_held_out);
+            launch_next(kernel, grid, block, stage, s, m->v, d_release_of, d_release_idx, n_release, d_pages, n, slot0, d_frames_out, d_held_out, slots);
     };
     if (copy) {
         if (m->v.dist)

@@ -50,6 +50,34 @@ def test_every_copied_frame_holds_its_page(cuda, pbm_mod, frame_size, policy, by
     bm.close()
 
 
+@pytest.mark.parametrize("extra", [0, 1, 5000])
+@pytest.mark.parametrize("frame_size", [16, 2048, 4112])
+@pytest.mark.parametrize("policy", [0, 1])
+def test_large_copying_rounds_hold_their_pages(cuda, pbm_mod, frame_size, policy, extra):
+    """Rounds on both sides of three blocks of 64 fetches an SM, where the staging buffers halve."""
+    torch, pbm = cuda, pbm_mod
+    R = 3 * 64 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    n_logical, n_frames, words = 60000, 40000, frame_size // 4
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(frame_size + extra)
+    backing = torch.randint(-2**31, 2**31 - 1, (n_logical, words), generator=gen, device="cuda", dtype=torch.int32)
+    bm = pbm.BufferManager(n_logical, n_frames, frame_size=frame_size, policy=policy, n_arms=R if policy else 1,
+                           backing=backing)
+    prev = idx = None
+    for r in range(3):
+        d = torch.randint(0, n_logical, (R,), generator=gen, device="cuda", dtype=torch.int32)
+        frames = torch.empty(R, dtype=torch.int32, device="cuda")
+        bm.round(prev, idx, R if r else 0, d, R, r * R, frames)
+        out = torch.empty(R, words, dtype=torch.int32, device="cuda")
+        bm.gather(frames, R, frame_size, out)
+        assert (frames >= 0).all() and torch.equal(out, backing[d.long()])
+        prev, idx = frames, torch.randperm(R, generator=gen, device="cuda").to(torch.int32)
+    c, chk = bm.counters(), bm.check()
+    assert (c.bad_unpins, c.timeouts, c.failures, chk.mismatches, chk.loading, chk.pins) == (0, 0, 0, 0, 0, R)
+    assert c.hits + c.misses == 3 * R and c.evictions > 0
+    bm.close()
+
+
 @pytest.mark.parametrize("n", [1, 33, 511, 513, 5000, 80001])
 @pytest.mark.parametrize("by_page", [True, False])
 def test_release_rounds_move_exactly_the_listed_pins(cuda, pbm_mod, n, by_page):
