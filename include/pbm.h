@@ -77,13 +77,14 @@ typedef struct {
     uint32_t max_steps;     /* bound on random jumps per request (0 = 4096) */
     int32_t  block_size;    /* threads per block (0 = 256) */
     int32_t  blocks_per_sm; /* persistent form: resident blocks per SM (0 = occupancy limit;
-                               >= 5 selects the register-capped kernels, 5 blocks) */
+                               >= 5 selects the register-capped kernels, 5 blocks; the
+                               page probe always runs those) */
     int32_t  free_merge;    /* 1 = merge frees of one word within a warp */
     int32_t  fail_fast;     /* pbm_alloc: 1 = count the free pages F before the launch (a pass over
                                the bitmap); requests r >= F fail at once instead of walking to
                                max_steps, the others walk as usual -- or, when the launch asks for
                                at least half of the F pages, request r takes the r-th free page in
-                               ascending order (one atomic, no walk) */
+                               ascending order (no walk) */
     int32_t  reserved;
 } pbm_walk_config;
 
