@@ -1247,13 +1247,13 @@ __device__ __forceinline__ void free_page_warp(const PoolView& v, uint32_t activ
 // granted than were free at the start -- with no atomic at all, so the
 // launch never contends on a shared counter.  When the launch asks for at
 // least half of the F free pages (`list_mode`), the pass also claims them, the
-// r-th free page in ascending order for request r, and only the requests whose
-// page another stream took in between (`lost` of them, their ids kLostPage) are left
-// to walk.  A null budget grants every request.
+// r-th free page in ascending order for request r, and refuses the requests past F; only
+// those whose page another stream took in between (`lost` of them, their ids kLostPage) are
+// left to walk.  A null budget grants every request.
 // ---------------------------------------------------------------------------
 struct LaunchBudget {
     long long free_at_start;    // F
-    int32_t list_mode;          // 1: requests 0 .. F - 1 have been served in order
+    int32_t list_mode;          // 1: requests 0 .. F - 1 served in order, the others refused
     uint32_t lost;              // but for these
 };
 constexpr int32_t kLostPage = -2;

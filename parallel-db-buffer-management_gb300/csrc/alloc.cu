@@ -31,43 +31,18 @@ struct AllocArgs {
 
 // Per-thread accumulators reduced once per block.
 struct Acc {
-    unsigned long long ok = 0, fail = 0, steps = 0;
+    uint32_t ok = 0, fail = 0;      // a launch has at most 2^32 - 1 requests
+    unsigned long long steps = 0;
 };
 
 __device__ __forceinline__ void flush_acc(const Acc& a, DevStats* st) {
     block_add_counters<3>({a.ok, a.fail, a.steps}, {&st->successes, &st->failures, &st->steps});
 }
 
-// A launch whose budget pass served the requests in order (list mode) has only the
-// refused ones left: ids -1, no steps.  Returns true when that is all; false when some
-// requests lost their page meanwhile and walk (or the pass served none).
-__device__ __forceinline__ bool finish_listed(const AllocArgs& a, Acc& acc) {
-    if (!a.budget || !__ldcg(&a.budget->list_mode) || __ldcg(&a.budget->lost)) return false;
-    // the first kFinishBlocks blocks do it (each block that counts something ends in an atomic at one
-    // address), four requests a store where the outputs allow it
-    constexpr uint32_t kFinishBlocks = 608;
-    const uint32_t blocks = min(gridDim.x, kFinishBlocks);
-    if (blockIdx.x >= blocks) return true;
-    const uint32_t nthr = blocks * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned long long F = (unsigned long long)__ldcg(&a.budget->free_at_start);
-    if (F >= a.n) return true;
-    const uint32_t f = (uint32_t)F, n = a.n;
-    uint32_t lo = f, hi = f;                       // [lo, hi): stored four at a time
-    if ((((uintptr_t)a.ids | (uintptr_t)a.steps) & 15u) == 0u && n - f >= 8u) {
-        lo = (f + 3u) & ~3u;
-        hi = n & ~3u;
-        for (uint32_t i = (lo >> 2) + tid; i < hi >> 2; i += nthr) {
-            reinterpret_cast<int4*>(a.ids)[i] = make_int4(-1, -1, -1, -1);
-            if (a.steps) reinterpret_cast<int4*>(a.steps)[i] = make_int4(0, 0, 0, 0);
-        }
-    }
-    for (uint64_t i = tid; i < (lo - f) + (n - hi); i += nthr) {
-        const uint64_t r = i < lo - f ? f + i : hi + (i - (lo - f));
-        a.ids[r] = -1;
-        if (a.steps) a.steps[r] = 0;
-    }
-    if (tid == 0) acc.fail += n - f;
-    return true;
+// A launch whose budget pass served the requests in order (list mode) is done, unless
+// some lost their page meanwhile: those walk.
+__device__ __forceinline__ bool all_listed(const AllocArgs& a) {
+    return a.budget && __ldcg(&a.budget->list_mode) && !__ldcg(&a.budget->lost);
 }
 
 // Whether request r walks: granted by the budget and not served by its pass.
@@ -79,18 +54,23 @@ enum class Walk { Page, Word32, Word64, Crw, SingleClock, DistClock };
 
 // Per-thread strategies.  The loop runs whole warps (uniform trip count) so
 // the block-level flush can use full-warp shuffles.
+// Eight blocks an SM for the walks; the page walk spills a little to fit 32 registers, and its
+// counts of requests are 32-bit for that (2^20 page walks at 50% 43.7 -> 41.4 us).  With 40 or
+// 48 registers it is faster in an empty pool (250,007 requests 12.3 -> 10.3 / 11.0 us) and
+// slower in a crowded one (at 90% 33 -> 40 / 34, at 95% 52 -> 67 / 54).
 template <Walk K>
 __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 5 : 8) k_alloc_thread(AllocArgs a) {
     stream_wait();
     Acc acc;
-    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t nthr = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t n_round = ((uint64_t)a.n + 31u) & ~31ull;
-    // whole warps iterate together (n_round and nthr are multiples of 32), or
-    // one thread in the serial replay
-    const bool done = finish_listed(a, acc);
+    if (all_listed(a)) return;
     const bool listed = a.budget && __ldcg(&a.budget->list_mode);
-    for (uint64_t r = tid; r < n_round && !done; r += nthr) {
+    // whole warps iterate together (nthr is a multiple of 32), or one thread in the serial
+    // replay; r stays below the requests rounded up to 32s, at most 2^32
+    const uint32_t nthr = gridDim.x * blockDim.x;
+    uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t r0 = r & ~31u;
+    const uint32_t trips = r0 < a.n ? (a.n - 1u - r0) / nthr + 1u : 0u;
+    for (uint32_t k = 0; k < trips; ++k, r += nthr) {
         const bool go = must_walk(a, listed, r);
         int32_t s = 0, id = -1;
         if (K == Walk::Page && blockDim.x >= 32u) {
@@ -122,7 +102,7 @@ __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 5 : 8) k_alloc_t
             id = sweep_dist(a.v, &ar, a.max_steps, &s);
             *arm = ar;
         }
-        if (r >= a.n || (listed && !go && budget_grants(a.budget, r))) continue;   // served by the budget pass
+        if (r >= a.n || (listed && !go)) continue;   // answered by the budget pass
         a.ids[r] = id;
         if (a.steps) a.steps[r] = s;
         acc.ok += id >= 0;
@@ -151,16 +131,16 @@ __global__ void __launch_bounds__(256, kCollabBlocks) k_alloc_collab(AllocArgs a
     const uint32_t L = WordTraits<Word>::count(a.v);
     const uint32_t lane_off = (uint32_t)(((unsigned long long)gl * a.stride) % L);
     volatile int32_t* my_slots = slots + (threadIdx.x & ~(uint32_t)(W - 1));
-    const bool done = finish_listed(a, acc);
+    if (all_listed(a)) return;
     const bool listed = a.budget && __ldcg(&a.budget->list_mode);
     // trip count uniform across each group of W lanes
-    for (uint64_t base = tid - gl; base < a.n && !done; base += nthr) {
+    for (uint64_t base = tid - gl; base < a.n; base += nthr) {
         const uint64_t r = base + gl;
         const bool need = must_walk(a, listed, r);
         int32_t s = 0;
         const int32_t id = walk_collab<W, Word>(a.v, need, request_seed(a.seed, base), lane_off, a.dedupe != 0, a.max_steps,
                                                 my_slots, &s);
-        if (r < a.n && (need || !listed || !budget_grants(a.budget, r))) {   // else served by the budget pass
+        if (r < a.n && (need || !listed)) {          // else answered by the budget pass
             a.ids[r] = id;
             if (a.steps) a.steps[r] = need ? s : 0;   // refused by the budget: no walk
             acc.ok += id >= 0;
@@ -490,7 +470,8 @@ int check_cfg(const pbm_walk_config* c) {
 // start as others end even it out (2^22 word probes at 50%: 102 us, 106 with one grid,
 // 128 with a block per 256 requests and a counter flush that is dear; 2^22 page walks
 // 171, 171, 190).  Behind a budget one grid is enough, most requests being answered by
-// it: 2^22 page walks at 90% fail-fast 124 -> 31 us, word probes 108 -> 30.
+// it: 2^22 page walks at 90% fail-fast 124 -> 31 us, word probes 108 -> 30 (the refusals
+// have since moved to the budget's pass: 23).
 constexpr int kThreadBlocks = 16 * 256, kListedBlocks = 8 * 256;
 
 int capped_grid(uint64_t threads, int block, int per_sm) {

@@ -279,8 +279,8 @@ __global__ void __launch_bounds__(kBudgetThreads) k_free_budget(const unsigned l
 // a list of pages here and taking each page of it with an atomic of its own in that kernel
 // moved 8 more bytes per page and took an atomic per page instead of per
 // word.  Measured on GB300, 2^22 requests on 2^24 pages at 90% (1.68 M granted) and
-// their frees: 63 -> 37 us, and 28 with a word per thread here and refusals stored four
-// at a time behind it.
+// their frees: 63 -> 37 us, 28 with a word per thread here and refusals stored four at
+// a time behind it, 23 with the refusals stored here, under way while the words are claimed.
 __global__ void __launch_bounds__(kBudgetThreads, kBudgetPerSm) k_take_free(unsigned long long* words, uint32_t n_words64, uint32_t per,
                                                    const unsigned long long* counts, LaunchBudget* b, uint32_t n_requests,
                                                    unsigned long long cap, int32_t* ids, int32_t* steps, DevStats* stats) {
@@ -304,12 +304,33 @@ __global__ void __launch_bounds__(kBudgetThreads, kBudgetPerSm) k_take_free(unsi
     __syncthreads();
     F = s_sum[0];
     off = s_sum[1];
-    const bool mode = F > 0ull && 2ull * n_requests >= F && F <= cap;
+    const bool mode = 2ull * n_requests >= F && F <= cap;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         b->free_at_start = (long long)F;
         b->list_mode = mode ? 1 : 0;
     }
-    if (!mode || off >= n_requests) return;
+    if (!mode) return;
+    // the requests past the free pages: refused here, their stores under way behind the words'
+    if (F < n_requests) {
+        const uint32_t nthr = gridDim.x * kBudgetThreads, tid = blockIdx.x * kBudgetThreads + threadIdx.x;
+        const uint32_t f = (uint32_t)F, n = n_requests;
+        uint32_t lo = f, hi = f;                   // [lo, hi): stored four at a time
+        if ((((uintptr_t)ids | (uintptr_t)steps) & 15u) == 0u && n - f >= 8u) {
+            lo = (f + 3u) & ~3u;
+            hi = n & ~3u;
+            for (uint32_t i = (lo >> 2) + tid; i < hi >> 2; i += nthr) {
+                reinterpret_cast<int4*>(ids)[i] = make_int4(-1, -1, -1, -1);
+                if (steps) reinterpret_cast<int4*>(steps)[i] = make_int4(0, 0, 0, 0);
+            }
+        }
+        for (uint64_t i = tid; i < (lo - f) + (n - hi); i += nthr) {
+            const uint64_t r = i < lo - f ? f + i : hi + (i - (lo - f));
+            ids[r] = -1;
+            if (steps) steps[r] = 0;
+        }
+        if (tid == 0) atomicAdd(&stats->failures, (unsigned long long)(n - f));
+    }
+    if (off >= n_requests) return;
     // this slice's requests: off .. off + quota - 1
     const uint32_t quota = (uint32_t)min(__ldcg(counts + blockIdx.x), (unsigned long long)n_requests - off);
     int32_t* out = ids + off;

@@ -202,6 +202,39 @@ def test_clock_sweep_of_many_warps(cuda, pbm_mod, orc, T, occ, n, max_steps):
     pool.close()
 
 
+@pytest.mark.parametrize("strategy", [0, 3, 5])
+@pytest.mark.parametrize("shift", [0, 1, 3])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 40, 100003])
+@pytest.mark.parametrize("free", [0, 1, 5])
+def test_budget_pass_refuses_past_the_free_pages(cuda, pbm_mod, strategy, shift, n, free):
+    """Refusals in outputs that start off a 16-byte boundary, in a pool with no free page or a few, with and
+    without steps: nothing outside the outputs is written."""
+    torch, pbm = cuda, pbm_mod
+    T = 5000
+    pool = pbm.Pool(T, 64)
+    words = np.full_like(pool.read_bitmap(), 0xffffffff)
+    pages = np.array([3, 64, 65, 2047, 4999][:free], dtype=np.int64)
+    for p in pages:
+        words[p >> 5] &= ~np.uint32(1 << (p & 31))
+    pool.write_bitmap(words)
+    k = min(n, free)
+    for with_steps in (True, False):
+        pool.write_bitmap(words)
+        s0 = pool.stats()
+        buf = torch.full((2, n + 16), -9, dtype=torch.int32, device="cuda")
+        ids, steps = buf[0, 4 + shift:4 + shift + n], buf[1, 4 + shift:4 + shift + n]
+        pool.alloc(pbm.walk_config(strategy, fail_fast=1, max_steps=1 << 20), n, 3, ids, steps if with_steps else None)
+        h = buf.cpu().numpy()
+        i, s = h[0, 4 + shift:4 + shift + n], h[1, 4 + shift:4 + shift + n]
+        assert np.array_equal(np.sort(i[:k]), pages[:k]) if 2 * n >= free else set(i[:k]) <= set(pages)
+        assert (i[k:] == -1).all()
+        assert (s == (np.arange(n) < k)).all() if with_steps and 2 * n >= free else with_steps or (s == -9).all()
+        assert (h[:, :4 + shift] == -9).all() and (h[:, 4 + shift + n:] == -9).all()
+        st = pool.stats()
+        assert (st.successes - s0.successes, st.failures - s0.failures) == (k, n - k)
+    pool.close()
+
+
 @pytest.mark.parametrize("strategy", [0, 1, 2, 3, 5, 6])
 @pytest.mark.parametrize("T,occ", [(64, 0.5), (2000, 0.7), (65536 + 17, 0.9), (1 << 20, 0.6), (3000001, 0.95)])
 def test_budget_pass_hands_the_free_pages_out_in_order(cuda, pbm_mod, orc, strategy, T, occ):
