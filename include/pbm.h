@@ -84,7 +84,8 @@ typedef struct {
                                the bitmap); requests r >= F fail at once instead of walking to
                                max_steps, the others walk as usual -- or, when the launch asks for
                                at least half of the F pages, request r takes the r-th free page in
-                               ascending order (no walk) */
+                               ascending order (no walk).  A captured launch may be replayed
+                               beside other launches; instances of one capture one after another */
     int32_t  reserved;
 } pbm_walk_config;
 

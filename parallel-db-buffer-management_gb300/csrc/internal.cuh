@@ -1,5 +1,6 @@
 // internal.cuh -- host/device internals shared by the libpbm translation units.
 #pragma once
+#include <mutex>
 #include <cuda_runtime.h>
 #include <atomic>
 #include <cstdint>
@@ -160,6 +161,17 @@ struct DeviceScope {
     DeviceScope& operator=(const DeviceScope&) = delete;
 };
 
+// Workspaces of a pool's fail-fast launches: a launch of one stream may run beside one of
+// another.  kBudgetSlots of them go round; a launch that gets one last used in
+// another stream waits for that launch's end.  A launch under capture has one of
+// kBudgetCaptures for good, and past those shares one more that lists no pages.
+constexpr uint32_t kBudgetSlots = 8, kBudgetCaptures = 24, kBudgetSpaces = kBudgetSlots + kBudgetCaptures + 1;
+struct BudgetSlot {
+    cudaEvent_t done;
+    unsigned long long stream;   // id of the stream that used it last
+    bool used;
+};
+
 constexpr int kDefaultBlock = 256;
 constexpr int kCappedBlocks = 5;   // resident blocks the register-capped batch kernels are built for
 
@@ -186,9 +198,13 @@ struct pbm_pool {
     pbm::CheckCounters* d_check;
     unsigned long long* d_scan;     // scratch for prefix sums (per-block partials)
     unsigned long long* d_prefix;   // batch prefix (n_groups + 1)
-    pbm::LaunchBudget* d_budget;    // fail-fast launch budget: free pages at launch start
+    // fail-fast launches: one workspace per launch (see budget_prepare)
+    std::mutex budget_mu;
+    pbm::BudgetSlot budget_slots[pbm::kBudgetSlots];
+    uint32_t budget_next, budget_captured;
+    pbm::LaunchBudget* d_budget;    // per workspace: free pages at launch start
     uint64_t list_cap;              // free pages up to which the budget pass may hand them out itself
-    unsigned long long* d_budget_blocks;   // free pages per block slice of the budget pass
+    unsigned long long* d_budget_blocks;   // per workspace: free pages per block slice of the budget pass
     uint32_t budget_blocks;
     uint32_t prefix_cap;
     int device;
@@ -225,5 +241,6 @@ int popcount_used(pbm_pool* pool, uint64_t* used, cudaStream_t s);
 // Counts the pool's free pages into pool->d_budget on stream s (no sync); a
 // launch of n_requests that asks for at least half of them is served in order by
 // the same pass (list mode).
-int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s);
+int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s, uint32_t* space);
+int budget_launched(pbm_pool* pool, uint32_t space, cudaStream_t s);
 }  // namespace pbm

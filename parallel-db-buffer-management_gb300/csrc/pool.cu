@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kBudgetThreads) k_free_budget(const unsigned l
 }
 
 // Pass 2: F, the sum of the counts, and, when the launch asks for at least half of
-// the F free pages (and F is at most `cap`), the pages themselves: request r takes
+// the F free pages (and F is below `cap`), the pages themselves: request r takes
 // the r-th free page in ascending order.  Each block claims its slice's
 // pages word by word with one atomicOr and writes their ids to the requests that
 // start at its offset (the counts of the blocks before it); the ids of a warp's 32 words
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kBudgetThreads, kBudgetPerSm) k_take_free(unsi
     __syncthreads();
     F = s_sum[0];
     off = s_sum[1];
-    const bool mode = 2ull * n_requests >= F && F <= cap;
+    const bool mode = 2ull * n_requests >= F && F < cap;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         b->free_at_start = (long long)F;
         b->list_mode = mode ? 1 : 0;
@@ -404,16 +404,47 @@ __global__ void __launch_bounds__(kBudgetThreads, kBudgetPerSm) k_take_free(unsi
     }
 }
 
-int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s) {
+// Both passes of a launch, in a workspace of its own (*space); pool->budget_mu is held until
+// budget_launched, so that the launches of two threads do not mix in one stream.  The
+// workspace's counts and places must be the launch's own: with another launch's, two
+// blocks could give one request its page.
+int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s, uint32_t* space) {
+    unsigned long long cap = pool->list_cap + 1u;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PBM_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+    if (capture == cudaStreamCaptureStatusNone) {
+        *space = pool->budget_next++ % kBudgetSlots;
+        const BudgetSlot& slot = pool->budget_slots[*space];
+        unsigned long long id = 0;
+        PBM_CUDA_TRY(cudaStreamGetId(s, &id));
+        if (slot.used && slot.stream != id) PBM_CUDA_TRY(cudaStreamWaitEvent(s, slot.done, 0));
+    } else if (pool->budget_captured < kBudgetCaptures) {
+        *space = kBudgetSlots + pool->budget_captured++;
+    } else {
+        *space = kBudgetSlots + kBudgetCaptures;
+        cap = 0ull;
+    }
+    LaunchBudget* budget = pool->d_budget + *space;
+    unsigned long long* counts = pool->d_budget_blocks + (size_t)*space * pool->budget_blocks;
     const uint32_t nw64 = (uint32_t)(pool->bitmap_bytes / 8u);
     const uint32_t nb = pool->budget_blocks;
     const uint32_t per = (nw64 + nb - 1u) / nb;
     unsigned long long* words = reinterpret_cast<unsigned long long*>(pool->d_words);
-    launch_next(k_free_budget, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget);
+    launch_next(k_free_budget, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, counts, budget);
     PBM_LAUNCH_CHECK();
-    launch_next(k_take_free, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, pool->d_budget_blocks, pool->d_budget, n_requests,
-                pool->list_cap, d_ids, d_steps, pool->d_stats);
+    launch_next(k_take_free, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, counts, budget, n_requests,
+                cap, d_ids, d_steps, pool->d_stats);
     PBM_LAUNCH_CHECK();
+    return PBM_OK;
+}
+
+// The launch that uses the workspace is queued in s (or was refused).
+int budget_launched(pbm_pool* pool, uint32_t space, cudaStream_t s) {
+    if (space >= kBudgetSlots) return PBM_OK;
+    BudgetSlot& slot = pool->budget_slots[space];
+    PBM_CUDA_TRY(cudaStreamGetId(s, &slot.stream));
+    PBM_CUDA_TRY(cudaEventRecord(slot.done, s));
+    slot.used = true;
     return PBM_OK;
 }
 
@@ -441,6 +472,8 @@ static void pool_free_all(pbm_pool* p) {
     cudaFree(p->d_base);
     cudaFree(p->d_ring);
     cudaFree(p->d_prefix);
+    for (BudgetSlot& slot : p->budget_slots)
+        if (slot.done) cudaEventDestroy(slot.done);
     delete p;
 }
 
@@ -478,9 +511,8 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
     if (!cfg || !out) return PBM_ERR_INVALID;
     *out = nullptr;
     if (cfg->n_pages == 0 || cfg->n_pages > 0x7fffffffull || cfg->page_size == 0) return PBM_ERR_INVALID;
-    pbm_pool* p = new (std::nothrow) pbm_pool();
+    pbm_pool* p = new (std::nothrow) pbm_pool();   // value-initialised: all zero
     if (!p) return PBM_ERR_NOMEM;
-    std::memset((void*)p, 0, sizeof(*p));
     p->n_pages = cfg->n_pages;
     p->page_size = cfg->page_size;
     p->flags = cfg->flags;
@@ -511,8 +543,8 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
     const size_t o_cursors = place(sizeof(int32_t) * p->max_slots), o_arms = place(sizeof(uint32_t) * p->max_slots);
     const size_t o_stats = place(sizeof(DevStats)), o_arm = place(sizeof(unsigned long long));
     const size_t o_fifo = place(sizeof(FifoState)), o_check = place(sizeof(CheckCounters));
-    const size_t o_budget = place(sizeof(LaunchBudget));
-    const size_t o_budget_blocks = place(sizeof(unsigned long long) * p->budget_blocks);
+    const size_t o_budget = place(sizeof(LaunchBudget) * kBudgetSpaces);
+    const size_t o_budget_blocks = place(sizeof(unsigned long long) * p->budget_blocks * kBudgetSpaces);
     const size_t o_scan = place(sizeof(unsigned long long) * nb_scan);
     char* all = nullptr;
     bool ok = cudaMalloc(&all, at) == cudaSuccess;
@@ -529,6 +561,8 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
         p->d_budget_blocks = reinterpret_cast<unsigned long long*>(all + o_budget_blocks);
         p->d_scan = reinterpret_cast<unsigned long long*>(all + o_scan);
     }
+    for (BudgetSlot& slot : p->budget_slots)
+        ok = ok && cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming) == cudaSuccess;
     if (ok && (cfg->flags & PBM_POOL_MATERIALIZE)) {
         ok = cudaMalloc(&p->d_base, (size_t)cfg->n_pages * cfg->page_size) == cudaSuccess;
     }

@@ -202,6 +202,78 @@ def test_clock_sweep_of_many_warps(cuda, pbm_mod, orc, T, occ, n, max_steps):
     pool.close()
 
 
+@pytest.mark.parametrize("threads", [1, 2])
+@pytest.mark.parametrize("n_streams", [2, 3, 11])
+def test_budget_launches_side_by_side(cuda, pbm_mod, n_streams, threads):
+    """Fail-fast launches of one pool in several streams, from one host thread or two, each asking for more
+    pages than are free: every request is answered, no page goes to two holders, none is lost."""
+    import threading
+    torch, pbm = cuda, pbm_mod
+    T, n, rounds = 1 << 20, 90000, 30
+    pool = pbm.Pool(T, 64)
+    pool.prefill(0.9, 5)
+    before = pool.read_bitmap()
+    base = pool.used()
+    cfg = pbm.walk_config(pbm.COLLAB_RW_BM, fail_fast=1, max_steps=64)
+    streams = [torch.cuda.Stream() for _ in range(n_streams)]
+    for k in range(rounds):
+        ids = [torch.full((n,), -9, dtype=torch.int32, device="cuda") for _ in streams]
+        torch.cuda.synchronize()
+
+        def issue(part):
+            for j in range(part, n_streams, threads):
+                pool.alloc(cfg, n, 100 * k + j, ids[j], stream=streams[j].cuda_stream)
+
+        ts = [threading.Thread(target=issue, args=(i,)) for i in range(threads)]
+        [x.start() for x in ts]
+        [x.join() for x in ts]
+        torch.cuda.synchronize()
+        got = torch.cat(ids).cpu().numpy()
+        held = got[got >= 0]
+        assert (got >= -1).all() and np.unique(held).size == held.size
+        assert not ((before[held >> 5] >> (held & 31).astype(np.uint32)) & 1).any()
+        assert pool.used() == base + held.size
+        for j, s in enumerate(streams):
+            pool.free(cfg, n, ids[j], stream=s.cuda_stream)
+        torch.cuda.synchronize()
+        assert np.array_equal(pool.read_bitmap(), before)
+    pool.close()
+
+
+def test_budget_launches_under_capture(cuda, pbm_mod):
+    """More captured fail-fast launches than there are workspaces for them, replayed beside launches that are
+    not captured: the first hand the free pages out in order, all answer every request."""
+    torch, pbm = cuda, pbm_mod
+    T, n, m = 1 << 16, 40000, 30
+    pool = pbm.Pool(T, 64)
+    pool.prefill(0.6, 5)   # pages are listed in a pool at least half full
+    before = pool.read_bitmap()
+    free = np.nonzero(np.unpackbits(before.view(np.uint8), bitorder="little")[:T] == 0)[0]
+    cfg = pbm.walk_config(pbm.COLLAB_RW_BM, fail_fast=1)
+    ids = torch.full((m, n), -9, dtype=torch.int32, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        for k in range(m):
+            pool.alloc(cfg, n, k, ids[k], stream=s.cuda_stream)
+            pool.free(cfg, n, ids[k], stream=s.cuda_stream)
+    for _ in range(3):
+        ids.fill_(-9)
+        g.replay()
+        torch.cuda.synchronize()
+        got = ids.cpu().numpy()
+        assert np.array_equal(pool.read_bitmap(), before)
+        for k in range(m):
+            assert np.array_equal(np.sort(got[k][:len(free)]), free) and (got[k][len(free):] == -1).all()
+            assert k >= 24 or np.array_equal(got[k][:len(free)], free)
+        one = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        pool.alloc(cfg, n, 9, one)
+        assert np.array_equal(one.cpu().numpy()[:len(free)], free)
+        pool.free(cfg, n, one)
+    pool.close()
+
+
 @pytest.mark.parametrize("strategy", [0, 3, 5])
 @pytest.mark.parametrize("shift", [0, 1, 3])
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 40, 100003])
