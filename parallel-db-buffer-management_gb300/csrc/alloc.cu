@@ -413,11 +413,12 @@ __global__ void __launch_bounds__(256) k_free_runs(PoolView v, uint32_t n, const
 // again is better walked for alone: its thread frees it at once, and not when its
 // warp's longest walk is done (32,768 requests for 32,768 free pages: 3.6 probes and 20 us
 // alone, 5.4 probes and 24 us together).
+// The counters are 64-bit throughout: with 32-bit ones (38 registers instead of 40) claiming,
+// reading and freeing 16,384 pages took 14.3 us instead of 12.2.
 template <bool HOLD>
 __global__ void __launch_bounds__(256) k_claim_write_free(AllocArgs a, uint32_t payload_words) {
     stream_wait();
-    Acc acc;
-    unsigned long long frees = 0;
+    unsigned long long ok = 0, fail = 0, walked = 0, frees = 0;
     const uint64_t n_round = ((uint64_t)a.n + 31u) & ~31ull;   // whole warps walk together
     for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_round;
          r += (uint64_t)gridDim.x * blockDim.x) {
@@ -438,11 +439,11 @@ __global__ void __launch_bounds__(256) k_claim_write_free(AllocArgs a, uint32_t 
             for (; k < payload_words; ++k) pg[k] = (int32_t)r;
             if (!HOLD) { free_page(a.v, id); ++frees; }
         }
-        acc.ok += id >= 0;
-        acc.fail += id < 0;
-        acc.steps += (unsigned long long)s;
+        ok += id >= 0;
+        fail += id < 0;
+        walked += (unsigned long long)s;
     }
-    block_add_counters<4>({acc.ok, acc.fail, acc.steps, frees},
+    block_add_counters<4>({ok, fail, walked, frees},
                           {&a.stats->successes, &a.stats->failures, &a.stats->steps, &a.stats->frees});
 }
 
