@@ -55,6 +55,9 @@ constexpr unsigned long long kEntryNotResident = ((unsigned long long)(uint32_t)
 constexpr unsigned long long kEntryFailed = ((unsigned long long)(uint32_t)kFailed << 32) | kGuard;
 constexpr uint32_t kFetchSpinLimit = 1u << 16;   // polls of a page another request is loading
 constexpr uint32_t kFetchAttempts = 1024u;        // fetches retried after a failed load
+#ifndef PBM_COPY_POLLS
+#define PBM_COPY_POLLS kFetchSpinLimit               // polls of a piece's load before its page is copied by hand
+#endif
 
 __device__ __forceinline__ int32_t e_frame(unsigned long long e) { return (int32_t)(e >> 32); }
 // Pins of an entry; while another release's over-subtraction has borrowed
@@ -377,8 +380,8 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < kFetchSpinLimit; ++i) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t polls) {
+    for (uint32_t i = 0; i < polls; ++i) {
         uint32_t ok;
         asm volatile(
             "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
@@ -406,8 +409,10 @@ __device__ __forceinline__ void bulk_stores_done() {
 // sends it to the frame with one bulk store, so a warp has as many bytes as its buffer
 // in flight with two instructions per piece.  Copying through registers, four 16-byte
 // loads per lane, kept 2 KiB per warp in flight: a round of 16,384 fetches (30%
-// misses) of 4 KiB pages took 41 us, 18 this way (6 of them here, 3.5 TB/s read).  The
-// whole warp calls converged.
+// misses) of 4 KiB pages took 41 us, 18 this way (6 of them here, 3.5 TB/s read).  A
+// piece whose load has not arrived after PBM_COPY_POLLS polls keeps its slot for the rest of the
+// kernel (the load may still write to it), and its page, before it is published, is copied
+// through registers.  The whole warp calls converged.
 constexpr uint32_t kCopyPiece = 4096;
 constexpr uint32_t kCopyStage = 32768;   // per warp, at most
 
@@ -425,7 +430,27 @@ struct CopyStage {
     uint32_t bar;      // its barrier
     uint32_t parity;   // of the barrier's next completion
     uint32_t slots;    // slots of the warp's buffer
+    bool late;         // a load that was given up may still be on its way to the slot
 };
+
+// The whole pages of the lanes in `todo`, copied by the warp through registers as
+// one flat run of 16-byte pieces.
+__device__ __forceinline__ void copy_pages_warp(const BmView& b, uint32_t todo, uint32_t page, int32_t h) {
+    const uint32_t n16 = b.frame_size / 16u;
+    const uint64_t total = (uint64_t)__popc(todo) * n16;
+    for (uint64_t base = 0; base < total; base += 32u) {
+        const uint64_t c = base + (threadIdx.x & 31u);
+        const uint32_t rank = (uint32_t)((c < total ? c : 0u) / n16);
+        const int l = (int)nth_set_bit(todo, (int)rank);                   // every lane shuffles
+        const uint32_t pg = __shfl_sync(0xffffffffu, page, l);
+        const int32_t fr = __shfl_sync(0xffffffffu, h, l);
+        if (c < total) {
+            const size_t j = (size_t)(c - (uint64_t)rank * n16);
+            reinterpret_cast<int4*>(b.frames + (size_t)(uint32_t)fr * b.frame_size)[j] =
+                reinterpret_cast<const int4*>(b.backing + (size_t)pg * b.frame_size)[j];
+        }
+    }
+}
 
 template <bool COPY>
 __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs, bool loader, uint32_t page, int32_t h,
@@ -436,6 +461,7 @@ __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs
         const uint32_t slots = cs.slots, piece = copy_piece(b.frame_size);
         const uint32_t per = (b.frame_size + piece - 1u) / piece;          // pieces per page
         const uint32_t total = (uint32_t)__popc(todo) * per;
+        uint32_t by_hand = 0u;                                             // lanes whose page has a late piece
         for (uint32_t base = 0; base < total; base += slots) {
             const uint32_t c = base + lane;
             const bool mine = lane < slots && c < total;
@@ -443,17 +469,23 @@ __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs
             const int l = (int)nth_set_bit(todo, (int)li);                 // every lane shuffles
             const uint32_t pg = __shfl_sync(0xffffffffu, page, l);
             const int32_t fr = __shfl_sync(0xffffffffu, h, l);
-            if (mine) {
+            if (mine && !cs.late) {
                 const uint32_t off = (c - li * per) * piece;
                 const uint32_t bytes = b.frame_size - off < piece ? b.frame_size - off : piece;
                 bulk_stores_read();                                        // the slot's last piece has left it
                 bulk_load(cs.buf, b.backing + (size_t)pg * b.frame_size + off, bytes, cs.bar);
-                if (!mbar_wait(cs.bar, cs.parity)) ++acc.timeouts;         // reported: the page's bytes are late
-                cs.parity ^= 1u;
-                bulk_store(b.frames + (size_t)(uint32_t)fr * b.frame_size + off, cs.buf, bytes);
+                if (mbar_wait(cs.bar, cs.parity, PBM_COPY_POLLS)) {
+                    cs.parity ^= 1u;
+                    bulk_store(b.frames + (size_t)(uint32_t)fr * b.frame_size + off, cs.buf, bytes);
+                } else {
+                    cs.late = true;
+                }
             }
+            by_hand |= __reduce_or_sync(0xffffffffu, mine && cs.late ? 1u << l : 0u);
         }
         if (total) bulk_stores_done();
+        __syncwarp();
+        if (by_hand) copy_pages_warp(b, by_hand, page, h);
         __syncwarp();
     }
     if (loader) publish(b, page, h, old_page, k, acc);
@@ -681,6 +713,8 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
         }
         __syncthreads();   // the tables are reused by the next iteration
     }
+    // a load that was given up must have ended before the block does; if it has not, that is reported
+    if (COPY && cs.late && !mbar_wait(cs.bar, cs.parity, kFetchSpinLimit)) ++acc.timeouts;
 }
 
 // A round of releases only (no fetch): the block's releases of one name meet
