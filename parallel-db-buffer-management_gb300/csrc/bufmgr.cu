@@ -433,35 +433,51 @@ struct CopyStage {
     bool late;         // a load that was given up may still be on its way to the slot
 };
 
+// How a round fills the frames of its misses: not at all, by bulk copies, or through registers.
+enum class Copy { None, Bulk, Plain };
+
 // The whole pages of the lanes in `todo`, copied by the warp through registers as
-// one flat run of 16-byte pieces.
+// one flat run of 16-byte pieces, IN_FLIGHT of them per lane at a time.
+template <uint32_t IN_FLIGHT>
 __device__ __forceinline__ void copy_pages_warp(const BmView& b, uint32_t todo, uint32_t page, int32_t h) {
     const uint32_t n16 = b.frame_size / 16u;
     const uint64_t total = (uint64_t)__popc(todo) * n16;
-    for (uint64_t base = 0; base < total; base += 32u) {
-        const uint64_t c = base + (threadIdx.x & 31u);
-        const uint32_t rank = (uint32_t)((c < total ? c : 0u) / n16);
-        const int l = (int)nth_set_bit(todo, (int)rank);                   // every lane shuffles
-        const uint32_t pg = __shfl_sync(0xffffffffu, page, l);
-        const int32_t fr = __shfl_sync(0xffffffffu, h, l);
-        if (c < total) {
-            const size_t j = (size_t)(c - (uint64_t)rank * n16);
-            reinterpret_cast<int4*>(b.frames + (size_t)(uint32_t)fr * b.frame_size)[j] =
-                reinterpret_cast<const int4*>(b.backing + (size_t)pg * b.frame_size)[j];
+    for (uint64_t base = 0; base < total; base += 32u * IN_FLIGHT) {
+        int4 v[IN_FLIGHT];
+        int4* dst[IN_FLIGHT];
+#pragma unroll
+        for (uint32_t u = 0; u < IN_FLIGHT; ++u) {
+            const uint64_t c = base + u * 32u + (threadIdx.x & 31u);
+            const uint32_t rank = (uint32_t)((c < total ? c : 0u) / n16);
+            const int l = (int)nth_set_bit(todo, (int)rank);               // every lane shuffles
+            const uint32_t pg = __shfl_sync(0xffffffffu, page, l);
+            const int32_t fr = __shfl_sync(0xffffffffu, h, l);
+            dst[u] = nullptr;
+            if (c < total) {
+                const size_t j = (size_t)(c - (uint64_t)rank * n16);
+                v[u] = reinterpret_cast<const int4*>(b.backing + (size_t)pg * b.frame_size)[j];
+                dst[u] = reinterpret_cast<int4*>(b.frames + (size_t)(uint32_t)fr * b.frame_size) + j;
+            }
         }
+#pragma unroll
+        for (uint32_t u = 0; u < IN_FLIGHT; ++u)
+            if (dst[u]) *dst[u] = v[u];
     }
 }
 
-template <bool COPY>
+template <Copy COPY>
 __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs, bool loader, uint32_t page, int32_t h,
                                                   uint32_t old_page, uint32_t k, BmAcc& acc) {
-    if (COPY) {
+    if constexpr (COPY == Copy::Plain) {
+        copy_pages_warp<4>(b, __ballot_sync(0xffffffffu, loader && h >= 0), page, h);
+        __syncwarp();
+    } else if constexpr (COPY == Copy::Bulk) {
         const uint32_t lane = threadIdx.x & 31u;
         const uint32_t todo = __ballot_sync(0xffffffffu, loader && h >= 0);
         const uint32_t slots = cs.slots, piece = copy_piece(b.frame_size);
         const uint32_t per = (b.frame_size + piece - 1u) / piece;          // pieces per page
         const uint32_t total = (uint32_t)__popc(todo) * per;
-        uint32_t by_hand = 0u;                                             // lanes whose page has a late piece
+        uint32_t by_hand = 0u;                                             // loaders whose page has a late piece
         for (uint32_t base = 0; base < total; base += slots) {
             const uint32_t c = base + lane;
             const bool mine = lane < slots && c < total;
@@ -481,11 +497,11 @@ __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs
                     cs.late = true;
                 }
             }
-            by_hand |= __reduce_or_sync(0xffffffffu, mine && cs.late ? 1u << l : 0u);
+            if (mine && cs.late) by_hand |= 1u << l;
         }
         if (total) bulk_stores_done();
-        __syncwarp();
-        if (by_hand) copy_pages_warp(b, by_hand, page, h);
+        by_hand = __reduce_or_sync(0xffffffffu, by_hand);
+        if (by_hand) copy_pages_warp<1>(b, by_hand, page, h);
         __syncwarp();
     }
     if (loader) publish(b, page, h, old_page, k, acc);
@@ -583,7 +599,7 @@ __device__ __forceinline__ uint32_t merge_insert(uint32_t* keys, uint32_t* cnt, 
 // round may land after other blocks' fetches of the same round; a sweep
 // that meets a page whose release has not landed yet passes it as pinned,
 // as it would any pinned page.
-template <bool DIST, bool BYPAGE, bool COPY, int BLOCK>
+template <bool DIST, bool BYPAGE, Copy COPY, int BLOCK>
 __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* release_of, const int32_t* release_idx,
                                              uint32_t n_release, const int32_t* pages, uint32_t n, uint32_t slot0,
                                              int32_t* frames_out, int32_t* held_out, uint32_t slots,
@@ -593,7 +609,7 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
     __shared__ uint32_t s_hand;   // the block's first sweep windows
     const uint32_t lane = threadIdx.x & 31u;
     CopyStage cs{};
-    if constexpr (COPY) {
+    if constexpr (COPY == Copy::Bulk) {
         extern __shared__ __align__(128) unsigned char stage[];
         __shared__ unsigned long long bars[BLOCK];
         const uint32_t piece = copy_piece(b.frame_size);
@@ -714,7 +730,7 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
         __syncthreads();   // the tables are reused by the next iteration
     }
     // a load that was given up must have ended before the block does; if it has not, that is reported
-    if (COPY && cs.late && !mbar_wait(cs.bar, cs.parity, kFetchSpinLimit)) ++acc.timeouts;
+    if (COPY == Copy::Bulk && cs.late && !mbar_wait(cs.bar, cs.parity, kFetchSpinLimit)) ++acc.timeouts;
 }
 
 // A round of releases only (no fetch): the block's releases of one name meet
@@ -769,10 +785,10 @@ __global__ void __launch_bounds__(256) k_release(BmView b, const int32_t* releas
 // One round: release the listed pins, then fetch this round's pages.
 // With one thread this is the deterministic replay of the round.
 // DIST: per-slot hands (b.dist), else the single shared hand.  BYPAGE:
-// release_of names pages, else frames.  COPY: misses copy their page from
-// the backing store (b.backing and b.frames set).  held_out (may be null)
+// release_of names pages, else frames.  COPY: how misses copy their page
+// from the backing store (not Copy::None: b.backing and b.frames set).  held_out (may be null)
 // receives each fetch's page, or -1 where the fetch got no frame.
-template <bool DIST, bool BYPAGE, bool COPY, int BLOCK>
+template <bool DIST, bool BYPAGE, Copy COPY, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_round(BmView b, const int32_t* release_of, const int32_t* release_idx,
                                                uint32_t n_release, const int32_t* pages, uint32_t n, uint32_t slot0,
                                                int32_t* frames_out, int32_t* held_out, uint32_t slots) {
@@ -858,6 +874,7 @@ struct pbm_bufmgr {
     BmCheck* d_check;
     size_t frames_bytes;
     int device;   // the device current at create: every later call runs there
+    bool bulk;    // the backing store lies in that device's own memory
 };
 
 extern "C" {
@@ -879,6 +896,14 @@ int pbm_bufmgr_create(const pbm_bufmgr_config* cfg, const void* d_backing, pbm_b
     b.n_arms = cfg->n_arms ? cfg->n_arms : 1u;
     b.dist = cfg->policy;
     b.backing = (const char*)d_backing;
+    // Bulk copies are for memory of this device.  A backing store elsewhere (pinned or managed
+    // host memory, another device's) is read by ordinary loads, which have no wait of their own that
+    // could run out when the memory is slow.
+    cudaPointerAttributes at{};
+    if (d_backing && cudaPointerGetAttributes(&at, d_backing) == cudaSuccess)
+        m->bulk = at.type == cudaMemoryTypeDevice && at.device == m->device;
+    else
+        cudaGetLastError();
     bool ok = cudaMalloc(&b.pt, sizeof(unsigned long long) * b.n_logical) == cudaSuccess &&
               cudaMalloc(&b.frame_page, sizeof(uint32_t) * b.n_frames) == cudaSuccess &&
               cudaMalloc(&b.single_hand, sizeof(unsigned long long)) == cudaSuccess &&
@@ -964,29 +989,34 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     // 32,768 / 65,536 / 131,072 fetches of 4 KiB, single hand: 125 / 147 / 204 / 323 / 548 us
     // with the full one, 131 / 151 / 173 / 298 / 488 with half; private hands from 32,768:
     // 241 / 383 / 683 and 194 / 340 / 563).
-    const uint32_t slots = copy ? copy_slots(m->v.frame_size, grid > 3 * sm_count() ? kCopyStage / 2u : kCopyStage) : 0u;
-    const size_t stage = copy && !serial ? 2u * (size_t)slots * copy_piece(m->v.frame_size) : 0u;
+    const uint32_t slots = copy && m->bulk ? copy_slots(m->v.frame_size, grid > 3 * sm_count() ? kCopyStage / 2u : kCopyStage) : 0u;
+    const size_t stage = slots && !serial ? 2u * (size_t)slots * copy_piece(m->v.frame_size) : 0u;
     cudaError_t attr = cudaSuccess;
     auto go = [&](auto kernel) {
         if (stage) attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)kCopyStage);
         if (attr == cudaSuccess)
             launch_next(kernel, grid, block, stage, s, m->v, d_release_of, d_release_idx, n_release, d_pages, n, slot0, d_frames_out, d_held_out, slots);
     };
-    if (copy) {
+    if (copy && m->bulk) {
         if (m->v.dist)
-            by_page ? go(k_round<true, true, true, 64>) : go(k_round<true, false, true, 64>);
+            by_page ? go(k_round<true, true, Copy::Bulk, 64>) : go(k_round<true, false, Copy::Bulk, 64>);
         else
-            by_page ? go(k_round<false, true, true, 64>) : go(k_round<false, false, true, 64>);
+            by_page ? go(k_round<false, true, Copy::Bulk, 64>) : go(k_round<false, false, Copy::Bulk, 64>);
+    } else if (copy) {
+        if (m->v.dist)
+            by_page ? go(k_round<true, true, Copy::Plain, 64>) : go(k_round<true, false, Copy::Plain, 64>);
+        else
+            by_page ? go(k_round<false, true, Copy::Plain, 64>) : go(k_round<false, false, Copy::Plain, 64>);
     } else if (small) {
         if (m->v.dist)
-            by_page ? go(k_round<true, true, false, 64>) : go(k_round<true, false, false, 64>);
+            by_page ? go(k_round<true, true, Copy::None, 64>) : go(k_round<true, false, Copy::None, 64>);
         else
-            by_page ? go(k_round<false, true, false, 64>) : go(k_round<false, false, false, 64>);
+            by_page ? go(k_round<false, true, Copy::None, 64>) : go(k_round<false, false, Copy::None, 64>);
     } else {
         if (m->v.dist)
-            by_page ? go(k_round<true, true, false, 128>) : go(k_round<true, false, false, 128>);
+            by_page ? go(k_round<true, true, Copy::None, 128>) : go(k_round<true, false, Copy::None, 128>);
         else
-            by_page ? go(k_round<false, true, false, 256>) : go(k_round<false, false, false, 256>);
+            by_page ? go(k_round<false, true, Copy::None, 256>) : go(k_round<false, false, Copy::None, 256>);
     }
     PBM_CUDA_TRY(attr);
     PBM_LAUNCH_CHECK();

@@ -136,3 +136,34 @@ def test_gather_copies_rows(cuda, pbm_mod, page_size, nbytes, shift):
     assert torch.equal(out.view(n, -1), want)
     assert (buf[:shift] == -7).all() and (buf[shift + n * nbytes // 4:] == -7).all()
     pool.close()
+
+
+@pytest.mark.parametrize("frame_size,R", [(16, 333), (4112, 333), (4096, 30000)])
+@pytest.mark.parametrize("policy", [0, 1])
+@pytest.mark.parametrize("by_page", [True, False])
+def test_backing_store_in_host_memory(cuda, pbm_mod, frame_size, R, policy, by_page):
+    """Pages filled from pinned host memory, which the device reads over the link."""
+    torch, pbm = cuda, pbm_mod
+    n_logical, n_frames, words = 4 * R, 2 * R, frame_size // 4
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(frame_size)
+    want = torch.randint(-2**31, 2**31 - 1, (n_logical, words), generator=gen, device="cuda", dtype=torch.int32)
+    backing = want.cpu().pin_memory()
+    bm = pbm.BufferManager(n_logical, n_frames, frame_size=frame_size, policy=policy, n_arms=R if policy else 1,
+                           backing=backing)
+    prev = idx = None
+    for r in range(4):
+        d = torch.randint(0, n_logical, (R,), generator=gen, device="cuda", dtype=torch.int32)
+        frames, held = (torch.empty(R, dtype=torch.int32, device="cuda") for _ in range(2))
+        if by_page:
+            bm.round_pages(prev, idx, R if r else 0, d, R, r * R, frames, held)
+        else:
+            bm.round(prev, idx, R if r else 0, d, R, r * R, frames)
+        out = torch.empty(R, words, dtype=torch.int32, device="cuda")
+        bm.gather(frames, R, frame_size, out)
+        assert (frames >= 0).all() and torch.equal(out, want[d.long()])
+        prev, idx = (held if by_page else frames), torch.randperm(R, generator=gen, device="cuda").to(torch.int32)
+    c, chk = bm.counters(), bm.check()
+    assert (c.bad_unpins, c.timeouts, c.failures, chk.mismatches, chk.loading, chk.pins) == (0, 0, 0, 0, 0, R)
+    assert c.hits + c.misses == 4 * R and c.evictions > 0
+    bm.close()
