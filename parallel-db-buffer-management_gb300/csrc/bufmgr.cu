@@ -625,8 +625,8 @@ __device__ __forceinline__ void round_blocks(const BmView& b, const int32_t* rel
     for (uint64_t bbase = (uint64_t)blockIdx.x * blockDim.x; bbase < work; bbase += stride) {
         const uint64_t i = bbase + threadIdx.x;
         if (!DIST && threadIdx.x == 0) s_hand = atomicAdd(b.single_hand, (unsigned long long)BLOCK) % b.n_frames;
-        const int32_t ri = i < n_release ? __ldg(release_idx + i) : -1;
-        const int32_t p = i < n ? __ldg(pages + i) : -1;
+        const int32_t ri = i < n_release ? __ldcg(release_idx + i) : -1;
+        const int32_t p = i < n ? __ldcg(pages + i) : -1;
         for (uint32_t s = threadIdx.x; s < 2u * KEYS; s += BLOCK) {
             t.fkey[s] = kMergeEmpty;
             t.fcnt[s] = 0u;
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(256) k_release(BmView b, const int32_t* releas
 #pragma unroll
     for (int u = 0; u < kReleaseItems; ++u) {
         const uint64_t j = base + (uint64_t)u * 256u;
-        rv[u] = j < n_release ? __ldg(release_idx + j) : -1;
+        rv[u] = j < n_release ? __ldcg(release_idx + j) : -1;
     }
     for (uint32_t s = threadIdx.x; s < 2u * KEYS; s += 256u) {
         keys[s] = kMergeEmpty;

@@ -79,7 +79,10 @@ __device__ __forceinline__ void block_add_counters(const unsigned long long (&v)
 // get its blocks onto the SMs while the kernel before it in the stream still runs;
 // it calls stream_wait() before its first access to global memory, which returns once
 // that kernel has ended and its writes are visible (at once after an ordinary
-// predecessor), and then lets the kernel after it do the same.  Most calls here are
+// predecessor), and then lets the kernel after it do the same.  Because the kernel before may
+// still write while this one is alive, nothing it could write is read with __ldg or
+// through a const __restrict__ pointer, which promise data that never changes in the
+// kernel's lifetime.  Most calls here are
 // kernels of 3-20 us launched one after another, and the start of a launch is 2-3 us of
 // each.  Measured on GB300, a call and the calls after it in a stream: 32 claims + frees
 // 8.2 -> 6.3 us; claim, read and free of 16,384 pages 18.5 -> 12.7; eight
@@ -125,7 +128,7 @@ __global__ void __launch_bounds__(256) k_gather_rows(const char* base, size_t st
     for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += step) {
         const uint32_t r = total <= 0xffffffffull ? (uint32_t)i / per_row : (uint32_t)(i / per_row);
         const uint32_t k = (uint32_t)(i - (unsigned long long)r * per_row);
-        const int32_t id = __ldg(ids + r);
+        const int32_t id = ids[r];
         V v{};
         if (id >= 0 && (uint32_t)id < n_rows) v = reinterpret_cast<const V*>(base + (size_t)(uint32_t)id * stride)[k];
         out[i] = v;
