@@ -571,6 +571,12 @@ int pbm_alloc(pbm_pool* pool, const pbm_walk_config* cfg, uint32_t n, uint32_t s
     int rc = check_cfg(cfg);
     if (rc) return rc;
     if (n == 0) return PBM_OK;
+    if (cfg->fail_fast && cfg->block_size > kDefaultBlock) {
+        // the walks are built for at most that many threads, and a launch of more is refused: refuse it
+        // before the budget's passes take pages for it
+        std::fprintf(stderr, "[pbm] pbm_alloc: blocks of %d threads cannot be launched\n", cfg->block_size);
+        return PBM_ERR_CUDA;
+    }
     AllocArgs a = make_args(pool, cfg, n, seed, d_ids, d_steps);
     if (cfg->strategy != PBM_LINKED_LIST) pool->fifo_valid = false;
     if (cfg->fail_fast && cfg->strategy != PBM_LINKED_LIST) {   // the free list counts its pages itself

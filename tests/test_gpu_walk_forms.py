@@ -427,3 +427,30 @@ def test_spans_of_sharing_warps(cuda, pbm_mod, orc, n, max_run):
         pool.free_runs(n, ids, dk)
         assert np.array_equal(np.unpackbits(pool.read_bitmap().view(np.uint8), bitorder="little")[:T], bits)
     pool.close()
+
+
+@pytest.mark.parametrize("strategy", [0, 1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("block_size", [288, 512, 1024])
+def test_refused_block_sizes_take_no_page(cuda, pbm_mod, strategy, block_size):
+    """Blocks larger than the walks are built for: the call is refused and the pool, the outputs and the
+    counters are as before it, with a budget and without one; the next call is served."""
+    torch, pbm = cuda, pbm_mod
+    n = 40000
+    pool = pbm.Pool(1 << 16, 64)
+    pool.prefill(0.6, 4)   # pages are listed in a pool at least half full
+    before = pool.read_bitmap()
+    for fail_fast in (1, 0):
+        ids = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        steps = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        with pytest.raises(pbm.PbmError) as e:
+            pool.alloc(pbm.walk_config(strategy, fail_fast=fail_fast, block_size=block_size), n, 3, ids, steps)
+        assert e.value.rc == pbm.ERR_CUDA
+        torch.cuda.synchronize()
+        assert np.array_equal(pool.read_bitmap(), before)
+        assert (ids == -9).all() and (steps == -9).all()
+        s = pool.stats()
+        assert (s.successes, s.failures, s.steps) == (0, 0, 0)
+    ids = torch.full((100,), -9, dtype=torch.int32, device="cuda")
+    pool.alloc(pbm.walk_config(strategy, fail_fast=1), 100, 3, ids)
+    assert (ids >= 0).all()
+    pool.close()
