@@ -240,7 +240,8 @@ int pbm_batch_launch_results(pbm_pool *pool, const pbm_walk_config *cfg, const p
  * d_groups + (k mod n_steps)*n_groups with seed seed0 + k.  The batch graph
  * counts its replays on the host: pbm_graph_replay writes k into the kernel's
  * parameters before it launches (launches already queued keep their
- * own k) and advances it; pbm_graph_set_step sets it.  Replay any number of
+ * own k) and advances it; pbm_graph_set_step waits for the replays so far and
+ * sets it.  Replay any number of
  * times, from one host thread at a time and in stream order; replays in
  * different streams run one after the other.  The malloc graphs do the same. */
 typedef struct pbm_graph pbm_graph;

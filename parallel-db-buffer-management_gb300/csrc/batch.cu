@@ -767,6 +767,14 @@ int pbm_graph_replay(pbm_graph* g, void* stream) {
     ++g->host_step;
     PBM_CUDA_TRY(cudaGraphLaunch(g->exec, s));
     count_launch(g->launches_per_replay);
+    if (!g->graph_only) {
+        if (cudaEventRecord(g->done, s) == cudaSuccess) {
+            g->launched = true;
+        } else {                              // another device's stream
+            cudaGetLastError();
+            g->graph_only = true;
+        }
+    }
     return PBM_OK;
 }
 
@@ -775,7 +783,10 @@ int pbm_graph_set_step(pbm_graph* g, uint32_t step, void* stream) {
     pbm::DeviceScope scope(g->device);
     cudaStream_t s = (cudaStream_t)stream;
     g->host_step = step;
-    // both parities of the batch kernel's tail pools start empty again
+    // the last replay, in whatever stream, before both parities of the batch kernel's tail pools start
+    // empty again: cleared under its blocks, they would hand chunks out twice
+    if (g->graph_only) PBM_CUDA_TRY(cudaDeviceSynchronize());   // it may be in another device's stream
+    else if (g->launched) PBM_CUDA_TRY(cudaStreamWaitEvent(s, g->done, 0));
     if (g->d_pools) PBM_CUDA_TRY(cudaMemsetAsync(g->d_pools, 0, sizeof(unsigned long long) * 2u * kPools * 16u, s));
     PBM_CUDA_TRY(cudaStreamSynchronize(s));
     return PBM_OK;

@@ -112,8 +112,8 @@ struct pbm_graph {
     size_t step_offset;
     const pbm_group* prefix_groups;
     uint32_t prefix_n_groups, prefix_n_steps;
-    // a one-kernel graph's replays by plain launch: the last one's end, the stream it is in
-    // (by id: a handle may come back for another stream), and whether replays stay with the graph
+    // the last replay's end, the stream a plain launch of a one-kernel graph was in (by id: a handle
+    // may come back for another stream), and whether replays stay with the graph
     cudaEvent_t done;
     unsigned long long last_stream;
     bool launched, graph_only;

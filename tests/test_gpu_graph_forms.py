@@ -40,3 +40,35 @@ def test_replays_in_turn_in_two_streams(cuda, pbm_mod, n_groups, walk):
     ids = arena.cpu().numpy()
     assert np.unique(ids).size == n and ids.min() >= 0 and pool.used() == base + n
     pool.close()
+
+
+@pytest.mark.parametrize("n_groups", [256, 4097])
+def test_set_step_in_another_stream_than_the_replay(cuda, pbm_mod, n_groups):
+    """set_step waits for the replay ahead of it, whatever their streams: every request of every replay
+    is served once, with the groups scanned by the blocks and by a kernel before them."""
+    torch, pbm = cuda, pbm_mod
+    T, n, pairs = 1 << 22, 1_500_007, 12
+    pool = pbm.Pool(T, 64)
+    pool.prefill(0.5, 3)
+    base = pool.used()
+    arena = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    tab = np.zeros(2 * n_groups, dtype=[("op", "<i4"), ("count", "<u4"), ("offset", "<u8")])
+    cut = np.linspace(0, n, n_groups + 1).astype(np.int64)
+    tab["op"] = np.repeat([pbm.OP_ALLOC, pbm.OP_FREE], n_groups)
+    tab["count"] = np.tile(np.diff(cut), 2)
+    tab["offset"] = np.tile(cut[:-1], 2)
+    d_tab = torch.from_numpy(tab.view(np.uint8).copy()).cuda()
+    g = pool.graph(pbm.walk_config(pbm.COLLAB_RW_BM, collab_width=64), d_tab, n_groups, 2, arena, n, 11)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for k in range(pairs):
+        g.replay(a.cuda_stream)
+        g.set_step(1, b.cuda_stream)
+        assert pool.used(b.cuda_stream) == base + n
+        g.replay(b.cuda_stream)
+        g.set_step(0, a.cuda_stream)
+        assert pool.used(a.cuda_stream) == base
+    s = pool.stats()
+    assert (s.successes, s.failures, s.frees) == (pairs * n, 0, pairs * n)
+    g.close()
+    pool.close()
