@@ -571,7 +571,7 @@ bool plain_replay(pbm_graph* g, cudaStream_t s) {
 }
 
 // Replays of one graph never run side by side, whatever their streams: one in another
-// stream than the last waits for its end.
+// stream than the last waits for its end.  The step moves on with the launch.
 cudaError_t launch_replay(pbm_graph* g, void** params, cudaStream_t s) {
     unsigned long long id = 0;
     cudaError_t e = cudaStreamGetId(s, &id);
@@ -588,6 +588,7 @@ cudaError_t launch_replay(pbm_graph* g, void** params, cudaStream_t s) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     if ((e = cudaLaunchKernelExC(&cfg, g->main_kp.func, params)) != cudaSuccess) return e;
+    ++g->host_step;
     g->last_stream = id;
     g->launched = true;
     return cudaEventRecord(g->done, s);
@@ -748,7 +749,6 @@ int pbm_graph_replay(pbm_graph* g, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     if (plain_replay(g, s)) {
         PBM_CUDA_TRY(launch_replay(g, params, s));
-        ++g->host_step;
         count_launch(g->launches_per_replay);
         return PBM_OK;
     }
@@ -764,8 +764,8 @@ int pbm_graph_replay(pbm_graph* g, void* stream) {
         pkp.kernelParams = pargs;
         PBM_CUDA_TRY(cudaGraphExecKernelNodeSetParams(g->exec, g->prefix_node, &pkp));
     }
-    ++g->host_step;
     PBM_CUDA_TRY(cudaGraphLaunch(g->exec, s));
+    ++g->host_step;                           // a refused replay is none: the next one runs its step
     count_launch(g->launches_per_replay);
     if (!g->graph_only) {
         if (cudaEventRecord(g->done, s) == cudaSuccess) {
