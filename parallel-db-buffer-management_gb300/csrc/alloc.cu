@@ -581,12 +581,11 @@ int pbm_alloc(pbm_pool* pool, const pbm_walk_config* cfg, uint32_t n, uint32_t s
     if (cfg->strategy != PBM_LINKED_LIST) pool->fifo_valid = false;
     if (cfg->fail_fast && cfg->strategy != PBM_LINKED_LIST) {   // the free list counts its pages itself
         std::lock_guard<std::mutex> lk(pool->budget_mu);
-        uint32_t space = 0;
-        rc = budget_prepare(pool, n, d_ids, d_steps, (cudaStream_t)stream, &space);
+        uint32_t slot = 0;
+        rc = budget_prepare(pool, n, d_ids, d_steps, (cudaStream_t)stream, &a.budget, &slot);
         if (rc) return rc;
-        a.budget = pool->d_budget + space;
         rc = launch_alloc(pool, cfg, a, false, (cudaStream_t)stream);
-        const int rc2 = budget_launched(pool, space, (cudaStream_t)stream);
+        const int rc2 = budget_launched(pool, slot, (cudaStream_t)stream);
         return rc ? rc : rc2;
     }
     return launch_alloc(pool, cfg, a, false, (cudaStream_t)stream);

@@ -1,8 +1,10 @@
 // internal.cuh -- host/device internals shared by the libpbm translation units.
 #pragma once
-#include <mutex>
 #include <cuda_runtime.h>
 #include <atomic>
+#include <memory>
+#include <mutex>
+#include <vector>
 #include <cstdint>
 #include <cstdio>
 
@@ -166,13 +168,26 @@ struct DeviceScope {
 
 // Workspaces of a pool's fail-fast launches: a launch of one stream may run beside one of
 // another.  kBudgetSlots of them go round; a launch that gets one last used in
-// another stream waits for that launch's end.  A launch under capture has one of
-// kBudgetCaptures for good, and past those shares one more that lists no pages.
-constexpr uint32_t kBudgetSlots = 8, kBudgetCaptures = 24, kBudgetSpaces = kBudgetSlots + kBudgetCaptures + 1;
+// another stream waits for that launch's end.  A launch under capture has one that goes
+// back when the graph that was captured, and every graph made of it, is gone: at first
+// there are kBudgetCaptures of those, and as many more come with each device allocation.
+constexpr uint32_t kBudgetSlots = 8, kBudgetCaptures = 24, kBudgetSpaces = kBudgetSlots + kBudgetCaptures;
 struct BudgetSlot {
     cudaEvent_t done;
     unsigned long long stream;   // id of the stream that used it last
     bool used;
+};
+struct BudgetSpace {
+    LaunchBudget* budget;         // free pages at launch start
+    unsigned long long* counts;   // free pages per block slice of the budget pass
+};
+// The captured launches' workspaces.  The graphs that hold some may outlive the pool, so each
+// shares this list; the device memory goes with the pool.
+struct BudgetCaptureSpaces {
+    std::mutex mu;
+    std::vector<BudgetSpace> unused;   // room for all of them reserved: returning one cannot fail
+    size_t total = 0;
+    std::vector<char*> chunks;
 };
 
 constexpr int kDefaultBlock = 256;
@@ -204,10 +219,10 @@ struct pbm_pool {
     // fail-fast launches: one workspace per launch (see budget_prepare)
     std::mutex budget_mu;
     pbm::BudgetSlot budget_slots[pbm::kBudgetSlots];
-    uint32_t budget_next, budget_captured;
-    pbm::LaunchBudget* d_budget;    // per workspace: free pages at launch start
+    uint32_t budget_next;
+    pbm::BudgetSpace budget_space[pbm::kBudgetSlots];
+    std::shared_ptr<pbm::BudgetCaptureSpaces> budget_captures;
     uint64_t list_cap;              // free pages up to which the budget pass may hand them out itself
-    unsigned long long* d_budget_blocks;   // per workspace: free pages per block slice of the budget pass
     uint32_t budget_blocks;
     uint32_t prefix_cap;
     int device;
@@ -241,9 +256,10 @@ namespace pbm {
 // Implemented in pool.cu
 int fifo_build(pbm_pool* pool, cudaStream_t s);
 int popcount_used(pbm_pool* pool, uint64_t* used, cudaStream_t s);
-// Counts the pool's free pages into pool->d_budget on stream s (no sync); a
-// launch of n_requests that asks for at least half of them is served in order by
-// the same pass (list mode).
-int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s, uint32_t* space);
-int budget_launched(pbm_pool* pool, uint32_t space, cudaStream_t s);
+// Counts the pool's free pages into *budget on stream s (no sync); a launch of
+// n_requests that asks for at least half of them is served in order by the same
+// pass (list mode).  *slot is for budget_launched.
+int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s,
+                   LaunchBudget** budget, uint32_t* slot);
+int budget_launched(pbm_pool* pool, uint32_t slot, cudaStream_t s);
 }  // namespace pbm

@@ -404,47 +404,146 @@ __global__ void __launch_bounds__(kBudgetThreads, kBudgetPerSm) k_take_free(unsi
     }
 }
 
-// Both passes of a launch, in a workspace of its own (*space); pool->budget_mu is held until
+namespace {
+
+constexpr size_t kBudgetCounts = 128;   // the counts begin a line of their own
+size_t budget_space_bytes(uint32_t blocks) {
+    return (kBudgetCounts + sizeof(unsigned long long) * blocks + 255u) & ~(size_t)255u;
+}
+
+BudgetSpace budget_space_at(char* base, uint32_t blocks, size_t i) {
+    char* p = base + i * budget_space_bytes(blocks);
+    return {reinterpret_cast<LaunchBudget*>(p), reinterpret_cast<unsigned long long*>(p + kBudgetCounts)};
+}
+
+// Puts the kBudgetCaptures workspaces at `base` among the unused ones; `own`: a device
+// allocation that goes with the pool.  False: no host memory.
+bool budget_add_captures(BudgetCaptureSpaces& c, char* base, uint32_t blocks, bool own) {
+    std::lock_guard<std::mutex> lk(c.mu);
+    try {
+        c.unused.reserve(c.total + kBudgetCaptures);
+        if (own) c.chunks.push_back(base);
+    } catch (...) {
+        return false;
+    }
+    c.total += kBudgetCaptures;
+    for (uint32_t i = 0; i < kBudgetCaptures; ++i) c.unused.push_back(budget_space_at(base, blocks, i));
+    return true;
+}
+
+// One of the unused ones, if there is one.
+bool budget_take_unused(BudgetCaptureSpaces& c, BudgetSpace* space) {
+    std::lock_guard<std::mutex> lk(c.mu);
+    if (c.unused.empty()) return false;
+    *space = c.unused.back();
+    c.unused.pop_back();
+    return true;
+}
+
+// A workspace held by a graph.
+struct BudgetLoan {
+    std::shared_ptr<BudgetCaptureSpaces> of;
+    BudgetSpace space;
+};
+
+// The last graph that held the loan is gone (called by the CUDA runtime, on any thread).
+void CUDART_CB budget_return(void* p) {
+    BudgetLoan* loan = static_cast<BudgetLoan*>(p);
+    {
+        std::lock_guard<std::mutex> lk(loan->of->mu);
+        loan->of->unused.push_back(loan->space);
+    }
+    delete loan;
+}
+
+// A workspace for a launch captured into `graph`, which holds it from here on.
+int budget_borrow(pbm_pool* pool, cudaGraph_t graph, BudgetSpace* space) {
+    BudgetCaptureSpaces& c = *pool->budget_captures;
+    if (!budget_take_unused(c, space)) {
+        char* chunk = nullptr;
+        // an allocation is no part of the capture, nor of one in another thread
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        bool ok = cudaMalloc(&chunk, budget_space_bytes(pool->budget_blocks) * kBudgetCaptures) == cudaSuccess;
+        if (ok && !budget_add_captures(c, chunk, pool->budget_blocks, true)) {
+            cudaFree(chunk);
+            ok = false;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!ok || !budget_take_unused(c, space)) {
+            cudaGetLastError();
+            return PBM_ERR_NOMEM;
+        }
+    }
+    BudgetLoan* loan = new (std::nothrow) BudgetLoan{pool->budget_captures, *space};
+    if (!loan) {
+        std::lock_guard<std::mutex> lk(c.mu);
+        c.unused.push_back(*space);
+        return PBM_ERR_NOMEM;
+    }
+    cudaUserObject_t held = nullptr;
+    if (cudaUserObjectCreate(&held, loan, budget_return, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        cudaGetLastError();
+        budget_return(loan);
+        return PBM_ERR_CUDA;
+    }
+    if (cudaGraphRetainUserObject(graph, held, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaGetLastError();
+        cudaUserObjectRelease(held, 1);
+        return PBM_ERR_CUDA;
+    }
+    return PBM_OK;
+}
+
+}  // namespace
+
+// Both passes of a launch, in a workspace of its own; pool->budget_mu is held until
 // budget_launched, so that the launches of two threads do not mix in one stream.  The
 // workspace's counts and places must be the launch's own: with another launch's, two
 // blocks could give one request its page.
-int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s, uint32_t* space) {
-    unsigned long long cap = pool->list_cap + 1u;
+int budget_prepare(pbm_pool* pool, uint32_t n_requests, int32_t* d_ids, int32_t* d_steps, cudaStream_t s,
+                   LaunchBudget** budget, uint32_t* slot) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    PBM_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t* deps = nullptr;        // asked for only so that nothing is left out of the answer
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n_deps = 0;
+    PBM_CUDA_TRY(cudaStreamGetCaptureInfo(s, &capture, nullptr, &graph, &deps, &edges, &n_deps));
+    BudgetSpace space;
     if (capture == cudaStreamCaptureStatusNone) {
-        *space = pool->budget_next++ % kBudgetSlots;
-        const BudgetSlot& slot = pool->budget_slots[*space];
+        *slot = pool->budget_next++ % kBudgetSlots;
+        space = pool->budget_space[*slot];
+        const BudgetSlot& last = pool->budget_slots[*slot];
         unsigned long long id = 0;
         PBM_CUDA_TRY(cudaStreamGetId(s, &id));
-        if (slot.used && slot.stream != id) PBM_CUDA_TRY(cudaStreamWaitEvent(s, slot.done, 0));
-    } else if (pool->budget_captured < kBudgetCaptures) {
-        *space = kBudgetSlots + pool->budget_captured++;
+        if (last.used && last.stream != id) PBM_CUDA_TRY(cudaStreamWaitEvent(s, last.done, 0));
+    } else if (capture == cudaStreamCaptureStatusActive) {
+        *slot = kBudgetSlots;
+        const int rc = budget_borrow(pool, graph, &space);
+        if (rc) return rc;
     } else {
-        *space = kBudgetSlots + kBudgetCaptures;
-        cap = 0ull;
+        return PBM_ERR_CUDA;   // a capture that already failed
     }
-    LaunchBudget* budget = pool->d_budget + *space;
-    unsigned long long* counts = pool->d_budget_blocks + (size_t)*space * pool->budget_blocks;
+    *budget = space.budget;
     const uint32_t nw64 = (uint32_t)(pool->bitmap_bytes / 8u);
     const uint32_t nb = pool->budget_blocks;
     const uint32_t per = (nw64 + nb - 1u) / nb;
     unsigned long long* words = reinterpret_cast<unsigned long long*>(pool->d_words);
-    launch_next(k_free_budget, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, counts, budget);
+    launch_next(k_free_budget, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, space.counts, space.budget);
     PBM_LAUNCH_CHECK();
-    launch_next(k_take_free, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, counts, budget, n_requests,
-                cap, d_ids, d_steps, pool->d_stats);
+    launch_next(k_take_free, nb, (unsigned)kBudgetThreads, 0, s, words, nw64, per, space.counts, space.budget,
+                n_requests, (unsigned long long)pool->list_cap + 1ull, d_ids, d_steps, pool->d_stats);
     PBM_LAUNCH_CHECK();
     return PBM_OK;
 }
 
 // The launch that uses the workspace is queued in s (or was refused).
-int budget_launched(pbm_pool* pool, uint32_t space, cudaStream_t s) {
-    if (space >= kBudgetSlots) return PBM_OK;
-    BudgetSlot& slot = pool->budget_slots[space];
-    PBM_CUDA_TRY(cudaStreamGetId(s, &slot.stream));
-    PBM_CUDA_TRY(cudaEventRecord(slot.done, s));
-    slot.used = true;
+int budget_launched(pbm_pool* pool, uint32_t slot, cudaStream_t s) {
+    if (slot >= kBudgetSlots) return PBM_OK;
+    BudgetSlot& last = pool->budget_slots[slot];
+    PBM_CUDA_TRY(cudaStreamGetId(s, &last.stream));
+    PBM_CUDA_TRY(cudaEventRecord(last.done, s));
+    last.used = true;
     return PBM_OK;
 }
 
@@ -474,6 +573,8 @@ static void pool_free_all(pbm_pool* p) {
     cudaFree(p->d_prefix);
     for (BudgetSlot& slot : p->budget_slots)
         if (slot.done) cudaEventDestroy(slot.done);
+    if (p->budget_captures)
+        for (char* chunk : p->budget_captures->chunks) cudaFree(chunk);
     delete p;
 }
 
@@ -543,8 +644,7 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
     const size_t o_cursors = place(sizeof(int32_t) * p->max_slots), o_arms = place(sizeof(uint32_t) * p->max_slots);
     const size_t o_stats = place(sizeof(DevStats)), o_arm = place(sizeof(unsigned long long));
     const size_t o_fifo = place(sizeof(FifoState)), o_check = place(sizeof(CheckCounters));
-    const size_t o_budget = place(sizeof(LaunchBudget) * kBudgetSpaces);
-    const size_t o_budget_blocks = place(sizeof(unsigned long long) * p->budget_blocks * kBudgetSpaces);
+    const size_t o_budget = place(budget_space_bytes(p->budget_blocks) * kBudgetSpaces);
     const size_t o_scan = place(sizeof(unsigned long long) * nb_scan);
     char* all = nullptr;
     bool ok = cudaMalloc(&all, at) == cudaSuccess;
@@ -557,10 +657,16 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
         p->d_arm = reinterpret_cast<unsigned long long*>(all + o_arm);
         p->d_fifo = reinterpret_cast<FifoState*>(all + o_fifo);
         p->d_check = reinterpret_cast<CheckCounters*>(all + o_check);
-        p->d_budget = reinterpret_cast<LaunchBudget*>(all + o_budget);
-        p->d_budget_blocks = reinterpret_cast<unsigned long long*>(all + o_budget_blocks);
+        for (uint32_t i = 0; i < kBudgetSlots; ++i) p->budget_space[i] = budget_space_at(all + o_budget, p->budget_blocks, i);
         p->d_scan = reinterpret_cast<unsigned long long*>(all + o_scan);
     }
+    try {
+        p->budget_captures = std::make_shared<BudgetCaptureSpaces>();
+    } catch (...) {
+        ok = false;
+    }
+    ok = ok && budget_add_captures(*p->budget_captures, all + o_budget + kBudgetSlots * budget_space_bytes(p->budget_blocks),
+                                   p->budget_blocks, false);
     for (BudgetSlot& slot : p->budget_slots)
         ok = ok && cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming) == cudaSuccess;
     if (ok && (cfg->flags & PBM_POOL_MATERIALIZE)) {

@@ -454,3 +454,66 @@ def test_refused_block_sizes_take_no_page(cuda, pbm_mod, strategy, block_size):
     pool.alloc(pbm.walk_config(strategy, fail_fast=1), 100, 3, ids)
     assert (ids >= 0).all()
     pool.close()
+
+
+@pytest.mark.parametrize("keep", [True, False])
+@pytest.mark.parametrize("capture_mode", ["global", "thread_local", "relaxed"])
+def test_captured_budget_launches_of_many_graphs(cuda, pbm_mod, keep, capture_mode):
+    """Graph after graph of one pool, kept or thrown away, more than any fixed number of workspaces: every
+    captured launch hands the free pages out in order, with a walk that could not find them."""
+    torch, pbm = cuda, pbm_mod
+    T, n, per, graphs = 1 << 14, 9000, 7, 40
+    pool = pbm.Pool(T, 64)
+    pool.prefill(0.6, 5)
+    before = pool.read_bitmap()
+    free = np.nonzero(np.unpackbits(before.view(np.uint8), bitorder="little")[:T] == 0)[0]
+    want = np.concatenate([free, np.full(n - len(free), -1)])
+    cfg = pbm.walk_config(pbm.RANDOM_WALK, fail_fast=1, max_steps=1)
+    kept = []
+    s = torch.cuda.Stream()
+    for k in range(graphs):
+        ids = torch.full((per, n), -9, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s, capture_error_mode=capture_mode):
+            for j in range(per):
+                pool.alloc(cfg, n, j, ids[j], stream=s.cuda_stream)
+                pool.free(cfg, n, ids[j], stream=s.cuda_stream)
+        if keep:
+            kept.append((g, ids))
+        for _ in range(2):
+            ids.fill_(-9)
+            g.replay()
+            torch.cuda.synchronize()
+            assert (ids.cpu().numpy() == want).all()
+        if not keep:
+            g.reset()
+    for g, ids in kept:
+        ids.fill_(-9)
+    torch.cuda.synchronize()
+    for g, ids in kept:
+        g.replay()
+    torch.cuda.synchronize()
+    for g, ids in kept:
+        assert (ids.cpu().numpy() == want).all()
+    assert np.array_equal(pool.read_bitmap(), before)
+    pool.close()
+
+
+def test_captured_budget_launches_outlive_their_pool(cuda, pbm_mod):
+    """A graph that is thrown away after its pool returns its workspace to nobody."""
+    torch, pbm = cuda, pbm_mod
+    s = torch.cuda.Stream()
+    for _ in range(3):
+        pool = pbm.Pool(1 << 12, 64)
+        ids = torch.empty(100, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            pool.alloc(pbm.walk_config(pbm.RANDOM_WALK, fail_fast=1), 100, 1, ids, stream=s.cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        assert (ids >= 0).all()
+        pool.close()
+        g.reset()
+        torch.cuda.synchronize()
