@@ -702,16 +702,15 @@ __device__ __forceinline__ int32_t sweep_single(const PoolView& v, unsigned long
 // converged.  The shared arm is one address, and one atomic per position examined
 // (and warp) queued there: 300,007 requests at 75% moved it some 190,000 times.
 // Here a warp moves the arm once over a window of positions, long enough to hold the
-// free pages it needs at the density seen last (at first: in 32 words drawn at
-// random), each lane reads one word of the window, and the first free pages in
+// free pages it needs at the density seen last, each lane reads one word of the window, and the first free pages in
 // sweep order are claimed, one atomicOr per word, and go to the needing lanes in lane
 // order.  Pages of the window beyond the need are passed until the arm comes round
-// again.  `alone`: no other warp of the launch moves the arm much, so the
-// unused end of the last window is given back (when the arm is still where this
-// warp left it): a launch of one block leaves the arm just past its last page and
-// passes no free page, as the one-thread sweep does.  A request's steps are the
-// positions from the page before its own; requests that find no page end after
-// max_steps positions each, taken together.
+// again.  `alone`: no other warp of the launch moves the arm, so the unused end of
+// the last window is given back (when the arm is still where this warp left it): a
+// launch of one warp leaves the arm just past its last page and passes no free
+// page, as the one-thread sweep does.  A request's steps are the positions from the
+// page before its own; requests that find no page end after max_steps positions each,
+// taken together.  fr_seen: the free pages in 1024 positions, to begin with.
 constexpr uint32_t kClockWindow = 896;   // positions: at most 30 words, wrapped windows included
 
 __device__ __forceinline__ uint32_t clock_window(uint32_t m, uint32_t free_pages, uint32_t positions) {
@@ -722,7 +721,7 @@ __device__ __forceinline__ uint32_t clock_window(uint32_t m, uint32_t free_pages
     return p < kClockWindow ? p : kClockWindow;
 }
 
-__device__ __forceinline__ int32_t sweep_single_warp(const PoolView& v, unsigned long long* arm, bool need, int32_t seed,
+__device__ __forceinline__ int32_t sweep_single_warp(const PoolView& v, unsigned long long* arm, bool need, uint32_t fr_seen,
                                                      uint32_t max_steps, bool alone, int32_t* steps_out) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt = (1u << lane) - 1u;
@@ -734,7 +733,6 @@ __device__ __forceinline__ int32_t sweep_single_warp(const PoolView& v, unsigned
         return -1;
     }
     unsigned long long left = (unsigned long long)__popc(needm) * max_steps;   // positions the requests may examine
-    uint32_t fr_seen = __reduce_add_sync(kFull32, (uint32_t)__popc(~load_word(v.words + idx_hi(seed, v.n_words32))));
     uint32_t p_seen = 1024u;
     unsigned long long passed = 0;                                 // positions since the last page claimed
     while (needm && left) {

@@ -59,7 +59,7 @@ enum class Walk { Page, Word32, Word64, Crw, SingleClock, DistClock };
 // 48 registers it is faster in an empty pool (250,007 requests 12.3 -> 10.3 / 11.0 us) and
 // slower in a crowded one (at 90% 33 -> 40 / 34, at 95% 52 -> 67 / 54).
 template <Walk K>
-__global__ void __launch_bounds__(256, K == Walk::SingleClock ? 5 : 8) k_alloc_thread(AllocArgs a) {
+__global__ void __launch_bounds__(256, 8) k_alloc_thread(AllocArgs a) {
     stream_wait();
     Acc acc;
     if (all_listed(a)) return;
@@ -75,8 +75,6 @@ __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 5 : 8) k_alloc_t
         int32_t s = 0, id = -1;
         if (K == Walk::Page && blockDim.x >= 32u) {
             id = walk_page_warp(a.v, go, request_seed(a.seed, (uint32_t)r), a.max_steps, &s);
-        } else if (K == Walk::SingleClock && blockDim.x >= 32u) {
-            id = sweep_single_warp(a.v, a.arm, go, request_seed(a.seed, (uint32_t)r), a.max_steps, gridDim.x == 1u, &s);
         } else if (!go) {
             // past the last request, or past the launch budget: no free page is left for this request
         } else if constexpr (K == Walk::Page) {
@@ -95,7 +93,7 @@ __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 5 : 8) k_alloc_t
             id = walk_crw(a.v, &c, seed0, a.max_steps, &s);
             *cur = c;
         } else if constexpr (K == Walk::SingleClock) {
-            id = sweep_single(a.v, a.arm, a.max_steps, &s);
+            id = sweep_single(a.v, a.arm, a.max_steps, &s);   // the one-thread replay; blocks: k_alloc_clock
         } else {
             uint32_t* arm = a.arms + (r % a.max_slots);
             uint32_t ar = *arm;
@@ -108,6 +106,206 @@ __global__ void __launch_bounds__(256, K == Walk::SingleClock ? 5 : 8) k_alloc_t
         acc.ok += id >= 0;
         acc.fail += id < 0;
         acc.steps += (unsigned long long)s;
+    }
+    flush_acc(acc, a.stats);
+}
+
+// ---- the single clock's sweep ----
+// While there are plenty of free pages each warp sweeps for itself (sweep_single_warp), and
+// the pages that its window holds beyond its need are passed until the arm comes round.  A
+// launch that asks for most of the free pages cannot pass any: it would go round the pool
+// again and again for the last of them, and fail requests that use up their positions on
+// the way.  Its blocks share the positions out: a block moves the arm over those that it
+// needs on average, its threads read one word each, and the end of the window
+// that was not needed goes to a list, where a block that is short looks before it moves
+// the arm again.  On average as many blocks leave an end as are short; with many ends in the list first
+// windows are a standard deviation shorter.
+// Measured on GB300, launches for exactly the free pages, us and requests that fail, one
+// position an atomic / every warp for itself / as here:
+//   2^20 pages at 50%: 107, 0 / 213-249, 50-200 / 85-95, 0
+//   2^24 pages at 90%: 1400, 0 / 390-450, 400-2,200 / 146, 0
+//   2^20 pages at 50% with a bound of 64 positions: 89, 0 / 46-50, 19,400-20,200 / 70, 0
+// and 300,007 requests for 1 M free pages with their frees, alone in a stream: 116 / 16.8 / 17.3 (shared out: 27).
+// The line lies at two thirds of the free pages: a warp's window is on average a fifth to a
+// quarter longer than its need, so what is asked for and what is passed stay
+// below what is there (launches for half of the free pages of 2^24 at 90%: 41 us both ways).
+constexpr int kClockBlocks = 5;              // of 256 threads an SM
+constexpr uint32_t kClockSpins = 1u << 12;   // polls of a slot that is being filled
+constexpr long long kClockMany = 1024;       // ends in the list from which first windows are a little shorter
+constexpr uint32_t kClockWaits = 32;         // looks at the list when no positions are left,
+constexpr uint32_t kClockPause = 1000;       // and ns between them: for ends that other blocks are just leaving
+
+// Whether the list has room for one more, `avail` being its count a moment ago.
+__device__ __forceinline__ bool clock_room(long long avail) { return avail < (long long)(kClockSlots / 2u); }
+
+__device__ __forceinline__ void clock_fill(ClockList* q, unsigned long long ticket, uint32_t pos, uint32_t len) {
+    atomicExch(q->slot + ticket % kClockSlots, ((unsigned long long)pos << 32) | len);
+    atomicAdd(&q->avail, 1ull);
+}
+
+__device__ __forceinline__ bool clock_take(ClockList* q, uint32_t* pos, uint32_t* len) {
+    if ((long long)atomicAdd(&q->avail, ~0ull) <= 0) {
+        atomicAdd(&q->avail, 1ull);
+        return false;
+    }
+    unsigned long long* slot = q->slot + atomicAdd(&q->head, 1ull) % kClockSlots;
+    unsigned long long e = 0ull;
+    for (uint32_t k = 0; !e && k < kClockSpins; ++k) e = atomicExch(slot, 0ull);
+    *pos = (uint32_t)(e >> 32);
+    *len = (uint32_t)e;
+    return e != 0ull;
+}
+
+// Exclusive prefix of v over the block, and its total.  `warp_tot`: a word per warp, not in use
+// between the caller's last barrier and its next one.
+__device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* warp_tot, uint32_t* total) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const uint32_t incl = (uint32_t)group_incl_scan<32>((int)v, lane, kFull32);
+    if (lane == 31u) warp_tot[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (uint32_t i = 0; i < nwarps; ++i) {
+        const uint32_t x = warp_tot[i];
+        if (i < warp) before += x;
+        all += x;
+    }
+    *total = all;
+    return before + incl - v;
+}
+
+// The sweep of a block that shares out the positions, for its threads with `go`; the block calls
+// converged.  seen_free of `seen` positions looked at were free.  A request's steps are the positions from
+// the page before its own; together the requests examine max_steps positions each, and those that find no page
+// end after max_steps -- once they have looked at the list kClockWaits times more.
+__device__ __forceinline__ int32_t clock_share(const AllocArgs& a, ClockList* list, bool go, uint32_t seen_free, uint32_t seen,
+                                               int32_t* steps_out) {
+    __shared__ uint32_t s_need[8], s_free[8], s_got[8];
+    __shared__ uint32_t s_pos[256];              // positions of the pages claimed in a window, from 1
+    __shared__ uint32_t s_p0, s_len, s_end, s_room;
+    const uint32_t T = a.v.n_pages;
+    const unsigned long long most = 32u * (blockDim.x - 2u);       // positions at once: a word per thread, wrapped or not
+    uint32_t M = 0;                                                // requests without a page
+    uint32_t rank = block_prefix(go ? 1u : 0u, s_need, &M);        // this one's place among them
+    unsigned long long left = (unsigned long long)M * a.max_steps;
+    unsigned long long passed = 0;                                 // positions since the last page claimed
+    int32_t id = -1, s = go ? (int32_t)a.max_steps : 0;
+    bool want = go;
+    bool none = false;                                             // the last window had no free page
+    long long avail = 0;                                           // thread 0's: the list's count seen last
+    if (threadIdx.x == 0) avail = (long long)__ldcg(&list->avail);
+    uint32_t waits = 0;
+    for (bool first = true; M; first = false) {
+        if (threadIdx.x == 0) {
+            uint32_t p0 = 0, P = 0;
+            if (!left) __nanosleep(kClockPause);
+            const long long now = (long long)__ldcg(&list->avail);
+            if (none || !left) avail = now;
+            if (!first && avail > 0 && clock_take(list, &p0, &P)) {
+                const uint32_t fit = (uint32_t)min(most, (unsigned long long)P);
+                if (fit < P) {
+                    const uint32_t rest = p0 + fit;
+                    clock_fill(list, atomicAdd(&list->tail, 1ull), rest >= T ? rest - T : rest, P - fit);
+                }
+                P = fit;
+            } else if (left) {
+                const unsigned long long mean = (unsigned long long)M * seen / (seen_free ? seen_free : 1u);
+                unsigned long long len = mean + 1ull;
+                if (!first) len = mean + (mean >> 3) + 8ull;
+                else if (avail > kClockMany) len -= min(mean / 2u, (unsigned long long)sqrtf((float)(mean * seen / (seen_free + 1u))));
+                P = (uint32_t)min(min(min(len, most), left), (unsigned long long)T);
+                p0 = (uint32_t)(atomicAdd(a.arm, (unsigned long long)P) % T);
+            }
+            avail = now;
+            s_room = clock_room(avail);
+            s_p0 = p0;
+            s_len = P;
+        }
+        __syncthreads();
+        const uint32_t p0 = s_p0, P = s_len;
+        if (!P && ++waits >= kClockWaits) break;
+        // thread i: word i of the pages p0 .. p0 + P - 1, wrapping past the last page
+        const uint32_t i = threadIdx.x, w0 = p0 >> 5;
+        const uint32_t end_a = min(T, p0 + P);                     // first stretch [p0, end_a)
+        const uint32_t n_a = ((end_a + 31u) >> 5) - w0;
+        const uint32_t end_b = P - (end_a - p0);                   // second stretch [0, end_b)
+        const uint32_t w = i < n_a ? w0 + i : i - n_a;
+        const uint32_t lo = i < n_a ? max(p0, w << 5) : w << 5, hi = i < n_a ? end_a : end_b;
+        uint32_t fr = 0u;
+        if ((w << 5) < hi) fr = ~load_word(a.v.words + w) & bit_range(lo & 31u, min(31u, hi - 1u - (w << 5)));
+        uint32_t total = 0, got_total = 0;
+        const uint32_t excl = block_prefix((uint32_t)__popc(fr), s_free, &total);
+        const uint32_t to_pos = i < n_a ? 1u - p0 : T - p0 + 1u;   // page + to_pos: its position in the window
+        uint32_t end = P;
+        if (excl < M && M - excl <= (uint32_t)__popc(fr)) {        // the last page needed is here
+            end = (w << 5) + nth_set_bit(fr, (int)(M - excl - 1u)) + to_pos;
+            s_end = end;
+        }
+        const bool leave = end < P && s_room;
+        unsigned long long ticket = 0;
+        if (leave) ticket = atomicAdd(&list->tail, 1ull);
+        uint32_t got = low_bits(fr, (int)M - (int)excl);
+        if (got) got &= ~atomicOr(a.v.words + w, got);             // less what another claim took first
+        if (leave) clock_fill(list, ticket, p0 + end >= T ? p0 + end - T : p0 + end, P - end);
+        const uint32_t at0 = block_prefix((uint32_t)__popc(got), s_got, &got_total);
+        const uint32_t used = total >= M ? s_end : P;
+        for (uint32_t m = got, k = at0; m; m &= m - 1u, ++k) s_pos[k] = (w << 5) + (uint32_t)__ffs((int)m) - 1u + to_pos;
+        __syncthreads();
+        if (want && rank < got_total) {
+            const uint32_t at = s_pos[rank];
+            const uint32_t p = p0 + at - 1u;
+            id = (int32_t)(p >= T ? p - T : p);
+            s = (int32_t)min((unsigned long long)a.max_steps, rank ? (unsigned long long)(at - s_pos[rank - 1u]) : passed + at);
+            want = false;
+        }
+        passed = got_total ? used - min(used, s_pos[got_total - 1u]) : passed + used;
+        none = total == 0u;
+        M -= got_total;
+        left = min(left - min(left, (unsigned long long)used), (unsigned long long)M * a.max_steps);
+        rank -= got_total;
+        seen_free += total;
+        seen += P;
+        if (seen > (1u << 24)) {
+            seen >>= 1;
+            seen_free >>= 1;
+        }
+    }
+    *steps_out = s;
+    return id;
+}
+
+__global__ void __launch_bounds__(256, kClockBlocks) k_alloc_clock(AllocArgs a, ClockList* list, uint32_t at_work) {
+    stream_wait();
+    __shared__ uint32_t s_sample[8];
+    Acc acc;
+    if (all_listed(a)) return;
+    const bool listed = a.budget && __ldcg(&a.budget->list_mode);
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < a.n; base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t r = base + threadIdx.x;
+        const bool go = must_walk(a, listed, r);
+        int32_t s = 0, id;
+        // a word drawn at random by each thread: free pages of 1024 positions (warp), of all (block)
+        const uint32_t f = __reduce_add_sync(
+            kFull32, (uint32_t)__popc(~load_word(a.v.words + idx_hi(request_seed(a.seed, (uint32_t)r) & 0x7fffffff, a.v.n_words32))));
+        if ((threadIdx.x & 31u) == 0u) s_sample[threadIdx.x >> 5] = f;
+        __syncthreads();
+        uint32_t seen_free = 0;
+        for (uint32_t i = 0; i < blockDim.x >> 5; ++i) seen_free += s_sample[i];
+        const uint32_t seen = 32u * blockDim.x;
+        // the pages that were free when the launch began: those free now, and those that the blocks before have
+        // taken, but for the ones that may still be at work
+        const uint64_t taken = base > at_work ? base - at_work : 0u;
+        if (a.n > 32u && 3.0f * (float)a.n >= 2.0f * ((float)seen_free / (float)seen * (float)a.v.n_pages + (float)taken))
+            id = clock_share(a, list, go, seen_free, seen, &s);
+        else
+            id = sweep_single_warp(a.v, a.arm, go, f, a.max_steps, a.n <= 32u, &s);
+        if (r < a.n && !(listed && !go)) {                         // else answered by the budget pass
+            a.ids[r] = id;
+            if (a.steps) a.steps[r] = s;
+            acc.ok += id >= 0;
+            acc.fail += id < 0;
+            acc.steps += (unsigned long long)s;
+        }
+        __syncthreads();                                           // s_sample is used again
     }
     flush_acc(acc, a.stats);
 }
@@ -529,7 +727,10 @@ int launch_alloc(pbm_pool* p, const pbm_walk_config* c, const AllocArgs& a, bool
         launch_next(k_alloc_thread<Walk::Crw>, grid, block, 0, s, a);
         break;
     case PBM_SINGLE_CLOCK:
-        launch_next(k_alloc_thread<Walk::SingleClock>, grid, block, 0, s, a);
+        // always in blocks of 256, which share out positions best (a larger one is refused, as the others are)
+        if (serial) launch_next(k_alloc_thread<Walk::SingleClock>, grid, block, 0, s, a);
+        else launch_next(k_alloc_clock, capped_grid(a.n, 256, a.budget ? kListedBlocks : kThreadBlocks), block > 256 ? block : 256, 0, s, a,
+                         p->d_clock_list, (uint32_t)(sm_count() * kClockBlocks * 256));
         break;
     case PBM_DIST_CLOCK:
         launch_next(k_alloc_thread<Walk::DistClock>, grid, block, 0, s, a);

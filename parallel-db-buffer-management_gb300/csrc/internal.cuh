@@ -190,6 +190,18 @@ struct BudgetCaptureSpaces {
     std::vector<char*> chunks;
 };
 
+// Stretches of the single clock's sweep that blocks took and did not need (see k_alloc_clock),
+// first in, first out: position and length in one word, 0 = empty.  Half of the slots are
+// for the blocks that find room at the same moment, 32 an SM at most; a stretch that finds
+// no room is passed until the arm comes round.
+constexpr uint32_t kClockSlots = 16384;
+struct ClockList {
+    alignas(128) unsigned long long head;    // next ticket to take
+    alignas(128) unsigned long long tail;    // next ticket to fill
+    alignas(128) unsigned long long avail;   // filled slots
+    alignas(128) unsigned long long slot[kClockSlots];
+};
+
 constexpr int kDefaultBlock = 256;
 constexpr int kCappedBlocks = 5;   // resident blocks the register-capped batch kernels are built for
 
@@ -209,6 +221,7 @@ struct pbm_pool {
     int32_t* d_cursors;             // clustered walk, per slot
     uint32_t* d_arms;               // distributed clock, per slot
     unsigned long long* d_arm;      // single clock
+    pbm::ClockList* d_clock_list;
     int32_t* d_ring;                // FIFO ring, n_pages entries (lazily built)
     pbm::FifoState* d_fifo;
     bool fifo_valid;

@@ -594,6 +594,7 @@ static int pool_reset_impl(pbm_pool* p, cudaStream_t s) {
     PBM_LAUNCH_CHECK();
     PBM_CUDA_TRY(cudaMemsetAsync(p->d_stats, 0, sizeof(DevStats), s));
     PBM_CUDA_TRY(cudaMemsetAsync(p->d_arm, 0, sizeof(unsigned long long), s));
+    PBM_CUDA_TRY(cudaMemsetAsync(p->d_clock_list, 0, sizeof(ClockList), s));
     p->fifo_valid = false;
     return PBM_OK;
 }
@@ -643,6 +644,7 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
     const size_t o_words = place(p->bitmap_bytes), o_seen = place(p->bitmap_bytes);
     const size_t o_cursors = place(sizeof(int32_t) * p->max_slots), o_arms = place(sizeof(uint32_t) * p->max_slots);
     const size_t o_stats = place(sizeof(DevStats)), o_arm = place(sizeof(unsigned long long));
+    const size_t o_clock = place(sizeof(ClockList));
     const size_t o_fifo = place(sizeof(FifoState)), o_check = place(sizeof(CheckCounters));
     const size_t o_budget = place(budget_space_bytes(p->budget_blocks) * kBudgetSpaces);
     const size_t o_scan = place(sizeof(unsigned long long) * nb_scan);
@@ -655,6 +657,7 @@ int pbm_pool_create(const pbm_pool_config* cfg, pbm_pool** out) {
         p->d_arms = reinterpret_cast<uint32_t*>(all + o_arms);
         p->d_stats = reinterpret_cast<DevStats*>(all + o_stats);
         p->d_arm = reinterpret_cast<unsigned long long*>(all + o_arm);
+        p->d_clock_list = reinterpret_cast<ClockList*>(all + o_clock);
         p->d_fifo = reinterpret_cast<FifoState*>(all + o_fifo);
         p->d_check = reinterpret_cast<CheckCounters*>(all + o_check);
         for (uint32_t i = 0; i < kBudgetSlots; ++i) p->budget_space[i] = budget_space_at(all + o_budget, p->budget_blocks, i);

@@ -517,3 +517,59 @@ def test_captured_budget_launches_outlive_their_pool(cuda, pbm_mod):
         pool.close()
         g.reset()
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("parts,max_steps", [(1, 512), (1, 4096), (3, 4096)])
+@pytest.mark.parametrize("block_size", [32, 256])
+@pytest.mark.parametrize("T,occ", [(3000, 0.0), (65536, 0.5), (1 << 20, 0.5), (1 << 20, 0.9), ((1 << 24) - 5, 0.5),
+                                   (1 << 24, 0.9), (1 << 22, 0.98)])
+def test_clock_sweep_serves_every_free_page(cuda, pbm_mod, orc, T, occ, block_size, parts, max_steps):
+    """Launches that ask for exactly the free pages, in one call or in several, get all of them; the next request
+    finds none; and again, once a third of them has come back."""
+    torch, pbm = cuda, pbm_mod
+    pool = pbm.Pool(T, 64)
+    pool.prefill(occ, 3)
+    free = T - pool.used()
+    if parts > 1 and occ > 0.95:
+        max_steps = 1 << 16        # pages that the first launches passed lie far apart
+    cfg = pbm.walk_config(pbm.SINGLE_CLOCK, max_steps=max_steps, block_size=block_size)
+    ids = torch.empty(free, dtype=torch.int32, device="cuda")
+    steps = torch.empty(free, dtype=torch.int32, device="cuda")
+    cut = np.linspace(0, free, parts + 1).astype(np.int64)
+    for lo, hi in zip(cut[:-1], cut[1:]):
+        pool.alloc(cfg, int(hi - lo), 7, ids[lo:], steps[lo:])
+    assert int((ids < 0).sum()) == 0 and pool.used() == T
+    chk = pool.check(ids, free)
+    assert (chk.n_duplicates, chk.n_not_marked, chk.n_out_of_range) == (0, 0, 0)
+    assert int(steps.min()) >= 1 and int(steps.max()) <= max_steps
+    one = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pool.alloc(cfg, 1, 7, one)
+    assert one.item() == -1
+    k = free // 3
+    pool.free(cfg, k, ids)
+    pool.alloc(pbm.walk_config(pbm.SINGLE_CLOCK, max_steps=1 << 20, block_size=block_size), k, 9, ids)
+    assert int((ids < 0).sum()) == 0 and pool.used() == T
+    assert pool.check(ids, free).n_duplicates == 0
+    pool.close()
+
+
+def test_clock_sweeps_side_by_side_serve_their_requests(cuda, pbm_mod):
+    """Launches in several streams that ask for three quarters of the free pages between them."""
+    torch, pbm = cuda, pbm_mod
+    T, streams = 1 << 20, [torch.cuda.Stream() for _ in range(3)]
+    pool = pbm.Pool(T, 64)
+    cfg = pbm.walk_config(pbm.SINGLE_CLOCK)
+    for k in range(10):
+        pool.reset()
+        pool.prefill(0.7, k)
+        free = T - pool.used()
+        n = 3 * free // 4
+        ids = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        cut = np.linspace(0, n, 4).astype(np.int64)
+        torch.cuda.synchronize()
+        for s, lo, hi in zip(streams, cut[:-1], cut[1:]):
+            pool.alloc(cfg, int(hi - lo), k, ids[lo:], stream=s.cuda_stream)
+        torch.cuda.synchronize()
+        assert int((ids < 0).sum()) == 0 and pool.used() == T - free + n
+        assert pool.check(ids, n).n_duplicates == 0
+    pool.close()
