@@ -164,3 +164,35 @@ def test_overfull_pool_fails_within_the_bound(cuda, pbm_mod, backend, max_steps)
     run(_table(torch, pbm.OP_MFREE, np.array([n])), None, 1, sizes, ptrs, n, 4, pbm.LAUNCH_PERSISTENT)
     assert not ptrs.any() and (pool.used() == 0 if backend == "runs" else pool.qmalloc_counts()[2:] == (0, 0, 0))
     pool.close()
+
+
+@pytest.mark.parametrize("backend", ["runs", "queue"])
+@pytest.mark.parametrize("n", [32, 64, 1000])
+def test_serial_replay_frees_a_slot_once(cuda, pbm_mod, backend, n):
+    """In the replay in request order a slot is empty once it is freed: a second group that frees the same slots
+    frees nothing, and the blocks beside theirs stay."""
+    torch, pbm = cuda, pbm_mod
+    pool = pbm.Pool(1 << 12, 4096, materialize=True)
+    pre = "" if backend == "runs" else "q"
+    getattr(pool, pre + "malloc_init")()
+    sizes = torch.full((2 * n,), 16, dtype=torch.int32, device="cuda")
+    ptrs = torch.zeros(2 * n, dtype=torch.int64, device="cuda")
+    t = np.zeros(4, dtype=[("op", "<i4"), ("count", "<u4"), ("offset", "<u8")])
+    t["op"] = [pbm.OP_MALLOC, pbm.OP_MFREE, pbm.OP_MFREE, pbm.OP_MFREE]
+    t["count"] = [2 * n, n, n, n]
+    table = torch.from_numpy(t.view(np.uint8).copy()).cuda()
+    getattr(pool, pre + "malloc_batch")(table, None, 4, sizes, ptrs, 2 * n, 5, pbm.LAUNCH_SERIAL)
+    s = pool.stats()
+    assert (s.successes, s.failures, s.frees) == (2 * n, 0, n)
+    p = ptrs.cpu().numpy()
+    assert not p[:n].any() and np.unique(p[n:]).size == n and p[n:].all()
+    rest = np.zeros(1, dtype=t.dtype)
+    rest["op"], rest["count"], rest["offset"] = pbm.OP_MFREE, n, n
+    getattr(pool, pre + "malloc_batch")(torch.from_numpy(rest.view(np.uint8).copy()).cuda(), None, 1, sizes, ptrs, 2 * n, 6,
+                                        pbm.LAUNCH_SERIAL)
+    assert pool.stats().frees == 2 * n and not ptrs.any()
+    if backend == "runs":
+        assert pool.used() == 0 and pool.malloc_counts() == (0, 0)
+    else:
+        assert pool.qmalloc_counts()[2:] == (0, 0, 0)
+    pool.close()
