@@ -442,6 +442,9 @@ __global__ void __launch_bounds__(256) k_fifo_free(PoolView v, uint32_t n, const
         const uint64_t r = base + (uint64_t)j * blockDim.x + threadIdx.x;
         id[j] = r < n ? ids[r] : -1;
         if (id[j] >= (int32_t)v.n_pages) id[j] = -1;
+        // the bit, a round trip and two barriers before the page is in its slot: a get of another
+        // stream sets it again as soon as it has the page
+        if (id[j] >= 0) atomicAnd(v.words + ((uint32_t)id[j] >> 5), ~(1u << ((uint32_t)id[j] & 31u)));
         const uint32_t b = __ballot_sync(kFull32, id[j] >= 0);
         cnt += (uint32_t)__popc(b);          // the warp's
     }
@@ -463,7 +466,6 @@ __global__ void __launch_bounds__(256) k_fifo_free(PoolView v, uint32_t n, const
     for (int j = 0; j < ITEMS; ++j) {
         const uint32_t b = __ballot_sync(kFull32, id[j] >= 0);
         if (id[j] >= 0) {
-            atomicAnd(v.words + ((uint32_t)id[j] >> 5), ~(1u << ((uint32_t)id[j] & 31u)));
             const uint64_t pos = (uint64_t)s_slot + rank + (uint32_t)__popc(b & ((1u << lane) - 1u));
             int32_t* slot = ring + (pos >= v.n_pages ? pos % v.n_pages : pos);
             uint32_t k = 0;

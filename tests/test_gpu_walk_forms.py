@@ -573,3 +573,31 @@ def test_clock_sweeps_side_by_side_serve_their_requests(cuda, pbm_mod):
         assert int((ids < 0).sum()) == 0 and pool.used() == T - free + n
         assert pool.check(ids, n).n_duplicates == 0
     pool.close()
+
+
+@pytest.mark.parametrize("n", [100, 40000, 200000])
+def test_free_list_gets_and_puts_in_two_streams(cuda, pbm_mod, n):
+    """Gets of one stream beside puts of another, on a list so short that pages come straight back: in the end the
+    bitmap marks exactly the pages that are held."""
+    torch, pbm = cuda, pbm_mod
+    T = 3 * n
+    pool = pbm.Pool(T, 64)
+    cfg = pbm.walk_config(pbm.LINKED_LIST)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    held = torch.full((2, n), -1, dtype=torch.int32, device="cuda")
+    pool.alloc(cfg, n, 0, held[0])
+    pool.alloc(cfg, n, 0, held[1])
+    torch.cuda.synchronize()
+    for k in range(60):
+        new = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        pool.free(cfg, n, held[k % 2], stream=a.cuda_stream)
+        pool.alloc(cfg, n, k, new, stream=b.cuda_stream)
+        torch.cuda.synchronize()
+        assert (new >= 0).all()
+        held[k % 2] = new
+        ids = np.sort(held.cpu().numpy().ravel())
+        assert np.unique(ids).size == 2 * n
+        bits = np.unpackbits(pool.read_bitmap().view(np.uint8), bitorder="little")[:T]
+        assert np.array_equal(np.nonzero(bits)[0], ids)
+    pool.close()
