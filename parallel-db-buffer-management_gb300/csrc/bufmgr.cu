@@ -973,15 +973,16 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
         PBM_LAUNCH_CHECK();
         return PBM_OK;
     }
-    // Blocks of 64 threads for rounds that would not give every SM two blocks of 256 (a
-    // round of 16,384 fetches is 64 such blocks), and for rounds that copy, whose
-    // staging buffers are then shared out in small blocks.  A larger round
-    // that copies nothing merges its requests over 256 threads, over 128 with private
-    // hands, whose kernel has 78 registers (eight rounds of 131,072 and 262,144 fetches, blocks of
-    // 64 / 128 / 256: 150 / 135 / 127 and 246 / 226 / 219 us with the single hand, 183 / 168 / 184
-    // and 194 / 172 / 188 us with private ones).
+    // Blocks of 64 threads for rounds that copy, whose staging buffers are shared out in small
+    // blocks, and for small rounds, which otherwise leave SMs without one.  A larger round that copies
+    // nothing merges its requests over 256 threads, over 128 with private hands, whose kernel has
+    // 78 registers.  us a round, releases and Zipf(0.99) fetches, replayed from a graph, 64 threads / 256 (128):
+    //   fetches       8,192   16,384   32,768   50,000   80,000   131,072   262,144
+    //   single hand  4.5/4.6  4.7/4.7  5.8/5.2  6.5/5.8  8.7/7.2  14.2/9.5  25.2/19.7
+    //   private      3.9/4.2  4.0/4.2  4.2/4.3  4.9/4.8  7.2/6.2   8.4/7.8  12.7/11.9
+    // so the line lies at half a block of 256 an SM (19,456), with private hands at two blocks of 128 (38,912).
     const bool copy = m->v.backing && m->v.frames;
-    const bool small = copy || work < (uint32_t)sm_count() * 512u;
+    const bool small = copy || work < (uint32_t)sm_count() * (m->v.dist ? 256u : 128u);
     const int block = serial ? 1 : small ? 64 : m->v.dist ? 128 : 256;
     const int grid = serial ? 1 : (int)(((uint64_t)work + (uint32_t)block - 1u) / (uint32_t)block);
     // Three blocks with full staging buffers fit an SM.  A copying round of more blocks than

@@ -167,3 +167,32 @@ def test_backing_store_in_host_memory(cuda, pbm_mod, frame_size, R, policy, by_p
     assert (c.bad_unpins, c.timeouts, c.failures, chk.mismatches, chk.loading, chk.pins) == (0, 0, 0, 0, 0, R)
     assert c.hits + c.misses == 4 * R and c.evictions > 0
     bm.close()
+
+
+@pytest.mark.parametrize("per_sm", [128, 256])
+@pytest.mark.parametrize("extra", [-1, 0, 4000])
+@pytest.mark.parametrize("policy", [0, 1])
+def test_rounds_where_the_blocks_grow(cuda, pbm_mod, per_sm, extra, policy):
+    """Rounds on both sides of the sizes from which blocks are larger, with hot pages and ids that name none: every
+    request holds the frame of its page, and the pins are what the host counts."""
+    torch, pbm = cuda, pbm_mod
+    R = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    n_logical, n_frames = 300000, 150000
+    rng = np.random.default_rng(R)
+    bm = pbm.BufferManager(n_logical, n_frames, policy=policy, n_arms=R if policy else 1)
+    prev = idx = None
+    for r in range(3):
+        pages = np.where(rng.random(R) < 0.3, rng.integers(0, 5, R), rng.integers(0, n_logical, R)).astype(np.int32)
+        pages[rng.random(R) < 0.02] = -1
+        d = torch.from_numpy(pages).cuda()
+        frames, held = (torch.empty(R, dtype=torch.int32, device="cuda") for _ in range(2))
+        bm.round_pages(prev, idx, R if r else 0, d, R, r * R, frames, held)
+        assert np.array_equal(held.cpu().numpy(), np.where(pages >= 0, pages, -1))
+        frame_of, pins, of_frame = bm.read_tables()[0], bm.read_tables()[1], frames.cpu().numpy()
+        ok = pages >= 0
+        assert np.array_equal(frame_of[pages[ok]], of_frame[ok])
+        assert np.array_equal(pins, np.bincount(pages[ok], minlength=n_logical))
+        prev, idx = held, torch.randperm(R, device="cuda").to(torch.int32)
+    c, chk = bm.counters(), bm.check()
+    assert (c.bad_unpins, c.timeouts, c.failures, chk.mismatches, chk.loading) == (0, 0, 0, 0, 0)
+    bm.close()
