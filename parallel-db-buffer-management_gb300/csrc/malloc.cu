@@ -112,10 +112,12 @@ __device__ __forceinline__ void flush_macc(const MAcc& c, DevStats* st) {
 // With a.fuse each block scans the step's group counts into shared memory itself, and
 // the graph form's step comes with the launch's parameters, so a replay is one
 // launch (a prefix kernel before it and a step kernel after it took 7 us of 39).  With page
-// runs and at least that many for every warp, a warp serves 64 requests at a time, two
-// rounds, and two rounds of frees, each a chain of dependent reads, go side by side
-// (524,288 mallocs + frees 54.5 -> 52.2 us); a smaller batch keeps more warps busy with 32, and
-// the replay in request order takes 32: a slot that two of its groups free is empty for the second.
+// runs and at least 96 requests for every warp (467,000 on 152 SMs), a warp serves 64 at
+// a time, two rounds, and two rounds of frees, each a chain of dependent reads, go side by side.  A
+// smaller batch keeps more warps busy with 32; us for mallocs and their frees, 256 groups, 32 / 64 at a time:
+//   requests  3,000  100,000  200,000  300,000    320,000  400,000  524,288    1,000,000  2,000,000
+//             14/18    19/23    25/25  27.6/27.2    30/33    34/36  40.0/38.9      64/64    131/127
+// The replay in request order takes 32: a slot that two of its groups free is empty for the second.
 // The chunks are dealt round robin over the blocks (mallocs and frees, whose chunks cost
 // differently, come in long runs) and a block's warps take its next one from a shared counter.
 template <bool SERIAL, bool Q>
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(256, 4) k_malloc_persistent(MArgs a) {
     const unsigned long long total = pre[a.n_groups];
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long nwarps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-    const unsigned long long ch = !Q && !SERIAL && total >= nwarps * 64ull ? 64ull : 32ull;   // requests per chunk
+    const unsigned long long ch = !Q && !SERIAL && total >= nwarps * 96ull ? 64ull : 32ull;   // requests per chunk
     for (;;) {
         unsigned int k = 0;
         if (lane == 0) k = atomicAdd(&s_next, 1u);
