@@ -246,10 +246,16 @@ int fifo_build(pbm_pool* pool, cudaStream_t s) {
 }
 
 // ---- fail-fast launch budget ----
-// Both passes run at most kBudgetPerSm blocks of kBudgetThreads per SM, what the second
-// one's shared memory lets fit: on 2^24 pages a block's slice is then one word per thread.
-constexpr int kBudgetThreads = 288;
-constexpr int kBudgetPerSm = 6;
+// Both passes run at most kBudgetPerSm blocks of kBudgetThreads per SM: 55 warps, the most
+// whose stages (4 KiB a warp) the second one's shared memory holds.  A thread takes a word
+// at a time, so the time goes up by a step where the pool's words pass a multiple of the
+// threads on the chip (17.1 M pages each), and the more threads, the later.  us for a fail-fast launch of a
+// quarter of the pages at 90% and its frees, 48 warps an SM (6 blocks of 256) / 54 (6 of 288) / 55 (5 of 352):
+//   2^20 pages 13.7 / 13.9 / 14.0    16 M 23.2 / 21.6 / 21.2    2^25 30.7 / 29.2 / 29.1
+//   2^22       15.6 / 16.0 / 15.8    17 M 23.5 / 24.1 / 21.3    2^26 45.3 / 44.9 / 45.7
+//   12 M       19.3 / 20.1 / 19.7    20 M 24.0 / 24.8 / 24.7    2^27 91.4 / 91.0 / 92.1
+constexpr int kBudgetThreads = 352;
+constexpr int kBudgetPerSm = 5;
 
 // Pass 1: the free pages (clear bits; padding bits stay set) of each block's
 // contiguous slice of `per` 64-bit words, into counts[block].

@@ -601,3 +601,22 @@ def test_free_list_gets_and_puts_in_two_streams(cuda, pbm_mod, n):
         bits = np.unpackbits(pool.read_bitmap().view(np.uint8), bitorder="little")[:T]
         assert np.array_equal(np.nonzero(bits)[0], ids)
     pool.close()
+
+
+@pytest.mark.parametrize("T", [17_100_000, 17_200_001, 40_000_003])
+def test_budget_pass_with_several_words_a_thread(cuda, pbm_mod, T):
+    """Pools around and past a word for every thread of the pass: request r gets the r-th free page."""
+    torch, pbm = cuda, pbm_mod
+    pool = pbm.Pool(T, 64)
+    pool.prefill(0.93, 6)
+    words = pool.read_bitmap()
+    free = np.nonzero(np.unpackbits(words.view(np.uint8), bitorder="little")[:T] == 0)[0]
+    cfg = pbm.walk_config(pbm.COLLAB_RW_BM, fail_fast=1)
+    for n in ((len(free) + 1) // 2, len(free) - 1, len(free) + 9):
+        pool.write_bitmap(words)
+        ids = torch.full((n,), -9, dtype=torch.int32, device="cuda")
+        pool.alloc(cfg, n, 3, ids)
+        k = min(n, len(free))
+        assert np.array_equal(ids.cpu().numpy(), np.concatenate([free[:k], np.full(n - k, -1)]))
+        assert pool.used() == T - len(free) + k
+    pool.close()
