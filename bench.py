@@ -10,7 +10,9 @@ its slot of a resident held-page arena (all prefilled pages, shuffled), so
 occupancy stays at 90%.  Ops = 2 x requests (one alloc, one free).
 
 Forms timed on the same requests:
-  value    batched: one persistent kernel per step, replayed from a CUDA graph
+  value    batched: one persistent kernel per step, captured once and replayed
+           (pbm_graph_replay: a one-kernel graph is replayed as a launch of that
+           kernel, which may overlap the end of the kernel before it)
   plain    one kernel launch per caller group (256 launches per step)
   e2e      through the C ABI with host buffers: the step's host descriptor
            table carried in the persistent launch's parameters, the step's new
@@ -57,7 +59,7 @@ GROUP_SEED = 4
 N_GROUPS = 256
 MAX_GROUP = 65536
 SEED0 = 1000
-METRIC = "alloc+free ops/s at 90% occupancy (batched persistent kernel, CUDA-graph replay)"
+METRIC = "alloc+free ops/s at 90% occupancy (batched persistent kernel, graph replays as overlapping launches)"
 UNIT = "ops/s"
 # DRAM bytes per alloc+free pair of the batch kernel: dram__bytes_read.sum +
 # dram__bytes_write.sum of one captured launch (7.82 MB for the 1,420,753-pair
@@ -338,7 +340,7 @@ def workload_config():
                     "with LogU[1,65536] requests (seed 4), swap op on a resident held-page arena",
         "pool_pages": T_PAGES, "page_size": PAGE_SIZE, "occupancy": OCCUPANCY, "prefill_seed": PREFILL_SEED,
         "groups_per_step": N_GROUPS, "walk": "autotuned for the 90% band (see tuned_config); reference arm: word-probe walk",
-        "launch": "persistent kernel in a CUDA graph", "l2": "flushed between timed steps (512 MiB write)",
+        "launch": "persistent kernel captured in a graph, replayed as overlapping launches (pbm_graph_replay)", "l2": "flushed between timed steps (512 MiB write)",
         "parallelism": "single GPU per rank (independent pools)",
     }
 
@@ -983,7 +985,7 @@ def config_malloc(torch, pbm, stream, flush, rounds=16, plain_rounds=4, max_step
         pool.close()
     out["graph_over_plain"] = out["graph"]["value"] / out["plain"]["value"]
     out["backends"] = {"graph, plain": "page runs with live counts per run (pbm_malloc_*)",
-                       "queue_graph": "per-class block queues (pbm_qmalloc_*), CUDA-graph form"}
+                       "queue_graph": "per-class block queues (pbm_qmalloc_*), graph form"}
     return out
 
 
