@@ -975,8 +975,8 @@ int launch_round(pbm_bufmgr* m, bool by_page, const int32_t* d_release_of, const
     }
     // Blocks of 64 threads for rounds that copy, whose staging buffers are shared out in small
     // blocks, and for small rounds, which otherwise leave SMs without one.  A larger round that copies
-    // nothing merges its requests over 256 threads, over 128 with private hands, whose kernel has
-    // 78 registers.  us a round, releases and Zipf(0.99) fetches, replayed from a graph, 64 threads / 256 (128):
+    // nothing merges its requests over 256 threads, over 128 with private hands, whose kernel takes
+    // 72 registers.  us a round, releases and Zipf(0.99) fetches, replayed from a graph, 64 threads / 256 (128):
     //   fetches       8,192   16,384   32,768   50,000   80,000   131,072   262,144
     //   single hand  4.5/4.6  4.7/4.7  5.8/5.2  6.5/5.8  8.7/7.2  14.2/9.5  25.2/19.7
     //   private      3.9/4.2  4.0/4.2  4.2/4.3  4.9/4.8  7.2/6.2   8.4/7.8  12.7/11.9
