@@ -411,8 +411,8 @@ __device__ __forceinline__ void bulk_stores_done() {
 // loads per lane, kept 2 KiB per warp in flight: a round of 16,384 fetches (30%
 // misses) of 4 KiB pages took 41 us, 18 this way (6 of them here, 3.5 TB/s read).  A
 // piece whose load has not arrived after PBM_COPY_POLLS polls keeps its slot for the rest of the
-// kernel (the load may still write to it), and its page, before it is published, is copied
-// through registers.  The whole warp calls converged.
+// kernel (the load may still write to it), and its lane copies it, and its later pieces, through
+// registers before their pages are published.  The whole warp calls converged.
 constexpr uint32_t kCopyPiece = 4096;
 constexpr uint32_t kCopyStage = 32768;   // per warp, at most
 
@@ -437,9 +437,9 @@ struct CopyStage {
 enum class Copy { None, Bulk, Plain };
 
 // The whole pages of the lanes in `todo`, copied by the warp through registers as
-// one flat run of 16-byte pieces, IN_FLIGHT of them per lane at a time.
-template <uint32_t IN_FLIGHT>
+// one flat run of 16-byte pieces, four of them per lane at a time.
 __device__ __forceinline__ void copy_pages_warp(const BmView& b, uint32_t todo, uint32_t page, int32_t h) {
+    constexpr uint32_t IN_FLIGHT = 4;
     const uint32_t n16 = b.frame_size / 16u;
     const uint64_t total = (uint64_t)__popc(todo) * n16;
     for (uint64_t base = 0; base < total; base += 32u * IN_FLIGHT) {
@@ -465,11 +465,17 @@ __device__ __forceinline__ void copy_pages_warp(const BmView& b, uint32_t todo, 
     }
 }
 
+// A late piece, copied by its lane.  Not inlined: the loop in place made rounds of 16,384 fetches with
+// 4 KiB copies 142.0 us instead of 138.9.
+__device__ __noinline__ void copy_late(char* dst, const char* src, uint32_t bytes) {
+    for (uint32_t j = 0; j < bytes; j += 16u) *reinterpret_cast<int4*>(dst + j) = *reinterpret_cast<const int4*>(src + j);
+}
+
 template <Copy COPY>
 __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs, bool loader, uint32_t page, int32_t h,
                                                   uint32_t old_page, uint32_t k, BmAcc& acc) {
     if constexpr (COPY == Copy::Plain) {
-        copy_pages_warp<4>(b, __ballot_sync(0xffffffffu, loader && h >= 0), page, h);
+        copy_pages_warp(b, __ballot_sync(0xffffffffu, loader && h >= 0), page, h);
         __syncwarp();
     } else if constexpr (COPY == Copy::Bulk) {
         const uint32_t lane = threadIdx.x & 31u;
@@ -477,7 +483,6 @@ __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs
         const uint32_t slots = cs.slots, piece = copy_piece(b.frame_size);
         const uint32_t per = (b.frame_size + piece - 1u) / piece;          // pieces per page
         const uint32_t total = (uint32_t)__popc(todo) * per;
-        uint32_t by_hand = 0u;                                             // loaders whose page has a late piece
         for (uint32_t base = 0; base < total; base += slots) {
             const uint32_t c = base + lane;
             const bool mine = lane < slots && c < total;
@@ -485,23 +490,25 @@ __device__ __forceinline__ void finish_loads_warp(const BmView& b, CopyStage& cs
             const int l = (int)nth_set_bit(todo, (int)li);                 // every lane shuffles
             const uint32_t pg = __shfl_sync(0xffffffffu, page, l);
             const int32_t fr = __shfl_sync(0xffffffffu, h, l);
-            if (mine && !cs.late) {
+            if (mine) {
                 const uint32_t off = (c - li * per) * piece;
                 const uint32_t bytes = b.frame_size - off < piece ? b.frame_size - off : piece;
-                bulk_stores_read();                                        // the slot's last piece has left it
-                bulk_load(cs.buf, b.backing + (size_t)pg * b.frame_size + off, bytes, cs.bar);
-                if (mbar_wait(cs.bar, cs.parity, PBM_COPY_POLLS)) {
-                    cs.parity ^= 1u;
-                    bulk_store(b.frames + (size_t)(uint32_t)fr * b.frame_size + off, cs.buf, bytes);
-                } else {
-                    cs.late = true;
+                const char* src = b.backing + (size_t)pg * b.frame_size + off;
+                char* dst = b.frames + (size_t)(uint32_t)fr * b.frame_size + off;
+                if (!cs.late) {
+                    bulk_stores_read();                                    // the slot's last piece has left it
+                    bulk_load(cs.buf, src, bytes, cs.bar);
+                    if (mbar_wait(cs.bar, cs.parity, PBM_COPY_POLLS)) {
+                        cs.parity ^= 1u;
+                        bulk_store(dst, cs.buf, bytes);
+                    } else {
+                        cs.late = true;
+                    }
                 }
+                if (cs.late) copy_late(dst, src, bytes);
             }
-            if (mine && cs.late) by_hand |= 1u << l;
         }
         if (total) bulk_stores_done();
-        by_hand = __reduce_or_sync(0xffffffffu, by_hand);
-        if (by_hand) copy_pages_warp<1>(b, by_hand, page, h);
         __syncwarp();
     }
     if (loader) publish(b, page, h, old_page, k, acc);
